@@ -627,6 +627,10 @@ struct gpuklu_handle {
   // Polls of a dependency flag before a waiting warp gives up
   // (gpuklu_set_spin_limit); applied to both resident plans.
   unsigned spin_limit = gk::kSpinLimit;
+  // Workspace of the AC sweep, kept between calls up to this size (a larger
+  // one is the call's own).
+  static constexpr size_t kAcKeep = (size_t)512 << 20;
+  DBuf<unsigned char> d_ac;
   // End the device Newton loop at the first non-finite iterate
   // (gpuklu_set_stop_on_nonfinite; off: the reference runs on to the cap).
   bool stop_nonfinite = false;
@@ -1356,69 +1360,87 @@ int gpuklu_ac_sweep(gpuklu_handle* h, gpuklu_circuit* c, const double* x_dc, int
     im_code.insert(im_code.end(), im_l[q].begin(), im_l[q].end());
     im_ptr.push_back((i32)im_code.size());
   }
+  // structure of Y by rows and by columns, a bit per cell
+  const int nw = (n + 31) / 32;
+  std::vector<unsigned> masks((size_t)2 * n * nw, 0u);
+  auto mark = [&](int r, int col) {
+    masks[(size_t)r * nw + (col >> 5)] |= 1u << (col & 31);
+    masks[(size_t)(n + col) * nw + (r >> 5)] |= 1u << (r & 31);
+  };
+  mark(0, 0);
+  for (int q = 0; q < ncell; ++q) mark(crow[q], ccol[q]);
   cudaStream_t s = h->stream;
-  DBuf<i32> d_crow, d_ccol, d_re_ptr, d_re_idx, d_im_ptr, d_im_code, d_status;
-  DBuf<double> d_cap, d_rhs, d_freqs, d_re, d_im, dx, dax, drc, drhs;
-  cudaError_t e = cudaSuccess;
-#define UP(buf, vec) \
-  if (e == cudaSuccess) e = buf.upload(vec, s);
-  std::vector<i32> vrow(crow.begin(), crow.end()), vcol(ccol.begin(), ccol.end());
-  std::vector<double> vfreq(freqs, freqs + nf), vx(x_dc, x_dc + std::max<int64_t>(xlen, 0));
-  UP(d_crow, vrow) UP(d_ccol, vcol) UP(d_re_ptr, re_ptr) UP(d_re_idx, re_idx) UP(d_im_ptr, im_ptr)
-  UP(d_im_code, im_code) UP(d_cap, cap) UP(d_rhs, rhs) UP(d_freqs, vfreq)
-#undef UP
-  if (e == cudaSuccess) e = d_re.resize((size_t)nf * n);
-  if (e == cudaSuccess) e = d_im.resize((size_t)nf * n);
-  if (e == cudaSuccess) e = d_status.resize(1);
-  if (e == cudaSuccess) e = dx.resize(std::max<int64_t>(xlen, 1));
-  if (e == cudaSuccess) e = dax.resize(std::max<size_t>(c->ai.size(), 1));
-  if (e == cudaSuccess) e = drc.resize(std::max(c->ncontrib, 1));
-  if (e == cudaSuccess) e = drhs.resize(n);
-  if (e == cudaSuccess && xlen > 0)
-    e = cudaMemcpyAsync(dx.p, vx.data(), xlen * sizeof(double), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_status.p, 0, sizeof(int), s);
+  const gk::AcShape shape = gk::ac_shape(n, (int)nf, sm_count());
+  // every array of the call in one device workspace, the inputs first and
+  // uploaded in one copy
+  struct Part {
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Part> parts;
+  size_t top = 0;
+  auto part = [&](const void* src, size_t bytes) {
+    parts.push_back({src, bytes, top});
+    top = (top + bytes + 255) & ~(size_t)255;
+    return parts.back().at;
+  };
+  const size_t xl = (size_t)std::max<int64_t>(xlen, 0);
+  const size_t o_row = part(crow.data(), 4 * (size_t)ncell), o_col = part(ccol.data(), 4 * (size_t)ncell),
+               o_rep = part(re_ptr.data(), 4 * re_ptr.size()),
+               o_rei = part(re_idx.data(), 4 * re_idx.size()),
+               o_imp = part(im_ptr.data(), 4 * im_ptr.size()),
+               o_imc = part(im_code.data(), 4 * im_code.size()),
+               o_msk = part(masks.data(), 4 * masks.size()), o_cap = part(cap.data(), 8 * cap.size()),
+               o_rhs = part(rhs.data(), 8 * rhs.size()), o_frq = part(freqs, 8 * (size_t)nf),
+               o_x = part(x_dc, 8 * xl);
+  const int zero = 0;
+  const size_t o_st = part(&zero, sizeof(int)), upload = top;
+  const size_t o_ax = part(nullptr, 8 * c->ai.size()), o_rc = part(nullptr, 8 * (size_t)c->ncontrib),
+               o_r = part(nullptr, 8 * (size_t)n), o_re = part(nullptr, 8 * (size_t)nf * n),
+               o_im = part(nullptr, 8 * (size_t)nf * n), o_m = part(nullptr, shape.scratch_bytes),
+               o_mw = part(nullptr, shape.masks_shared ? 0 : 4 * shape.mask_words * shape.blocks);
+  std::vector<unsigned char> blob(upload, 0);
+  for (const Part& q : parts)
+    if (q.src && q.bytes) std::memcpy(blob.data() + q.at, q.src, q.bytes);
+  // the workspace stays with the handle up to kAcKeep bytes
+  DBuf<unsigned char> once;
+  DBuf<unsigned char>& ws = top <= gpuklu_handle::kAcKeep ? h->d_ac : once;
+  cudaError_t e = ws.resize(top);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(ws.p, blob.data(), upload, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return h->cuda_fail(e, "ac upload");
+  auto dbl = [&](size_t at) { return reinterpret_cast<double*>(ws.p + at); };
+  auto i32p = [&](size_t at) { return reinterpret_cast<i32*>(ws.p + at); };
   // G: the DC stamp at the operating point (the AC stamps of R, V, D and M
   // are the DC stamp's matrix entries there, stamp.rs:1525-1747)
-  gk::launch_stamp(c->dc, dx.p, (int)std::min<int64_t>(xlen, nc), 1e-12, 1.0, 0.0, nullptr, -1.0,
-                   dax.p, drc.p, drhs.p, s, 1e-12);
+  gk::launch_stamp(c->dc, dbl(o_x), (int)std::min<int64_t>(xlen, nc), 1e-12, 1.0, 0.0, nullptr,
+                   -1.0, dbl(o_ax), dbl(o_rc), dbl(o_r), s, 1e-12);
   gk::AcArgs a{};
   a.n = n;
   a.ncell = ncell;
-  a.cell_row = d_crow.p;
-  a.cell_col = d_ccol.p;
-  a.re_ptr = d_re_ptr.p;
-  a.re_idx = d_re_idx.p;
-  a.im_ptr = d_im_ptr.p;
-  a.im_code = d_im_code.p;
-  a.cap = d_cap.p;
-  a.ax = dax.p;
-  a.rhs = d_rhs.p;
-  a.freqs = d_freqs.p;
-  a.out_re = d_re.p;
-  a.out_im = d_im.p;
-  a.status = d_status.p;
-  DBuf<double> d_scratch;
-  if (gk::ac_fits_shared(n)) {
-    gk::launch_ac_dense(a, (int)nf, s);
-  } else {
-    // one n x n complex matrix per block in global memory, at most ~2 GB of
-    // them (and no more blocks than frequencies or two per SM)
-    const size_t per = (size_t)16 * n * n;
-    int blocks = (int)std::min<int64_t>(nf, std::max<size_t>(1, ((size_t)2 << 30) / per));
-    blocks = std::min(blocks, 2 * sm_count());
-    e = d_scratch.resize(per / 8 * blocks);
-    if (e != cudaSuccess) return h->cuda_fail(e, "ac scratch");
-    a.scratch = d_scratch.p;
-    gk::launch_ac_dense_global(a, (int)nf, blocks, s);
-  }
+  a.cell_row = i32p(o_row);
+  a.cell_col = i32p(o_col);
+  a.re_ptr = i32p(o_rep);
+  a.re_idx = i32p(o_rei);
+  a.im_ptr = i32p(o_imp);
+  a.im_code = i32p(o_imc);
+  a.cap = dbl(o_cap);
+  a.ax = dbl(o_ax);
+  a.rhs = dbl(o_rhs);
+  a.freqs = dbl(o_frq);
+  a.out_re = dbl(o_re);
+  a.out_im = dbl(o_im);
+  a.status = i32p(o_st);
+  a.scratch = dbl(o_m);
+  a.masks0 = reinterpret_cast<const unsigned*>(ws.p + o_msk);
+  a.masks = reinterpret_cast<unsigned*>(ws.p + o_mw);
+  gk::launch_ac_sparse(a, (int)nf, shape, s);
   int st = 0;
   e = cudaGetLastError();
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out_re, d_re.p, (size_t)nf * n * 8, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(out_re, a.out_re, (size_t)nf * n * 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out_im, d_im.p, (size_t)nf * n * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, d_status.p, sizeof(int), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(out_im, a.out_im, (size_t)nf * n * 8, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, a.status, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return h->cuda_fail(e, "ac sweep");
   if (st) return h->fail(GPUKLU_SINGULAR, "ac sweep: a pivot below 1e-30");

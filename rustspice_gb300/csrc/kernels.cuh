@@ -219,7 +219,9 @@ struct AcArgs {
   const double* freqs;
   double *out_re, *out_im;          // nf x n
   int* status;                      // 1: a pivot below 1e-30
-  double* scratch;                  // global path: per block an n x n complex matrix
+  double* scratch;                  // per block an n x n complex matrix
+  const unsigned* masks0;           // structure of Y: rows' bit masks [n][nw], then columns'
+  unsigned* masks;                  // per block the same two, where shared memory has no room
 };
 
 // --------------------------------------------------------------- launches
@@ -325,11 +327,16 @@ void launch_gather(double* dst, const double* src, const int* idx, int n, cudaSt
 void launch_bbd_combine(const double* z, const double* w2, const double* xT, const BbdArgs& B,
                         double* x, cudaStream_t s);
 
-// One thread block per frequency; shared memory ac_smem_bytes(n, 256).
-size_t ac_smem_bytes(int n, int threads);
-void launch_ac_dense(const AcArgs& a, int nf, cudaStream_t s);
-bool ac_fits_shared(int n);
-void launch_ac_dense_global(const AcArgs& a, int nf, int blocks, cudaStream_t s);
+// AC sweep: `blocks` thread blocks of `warps` warps loop over the frequencies,
+// each with scratch_bytes / blocks of AcArgs::scratch and, unless
+// masks_shared, mask_words of AcArgs::masks.
+struct AcShape {
+  int warps, blocks;
+  bool masks_shared;
+  size_t smem, scratch_bytes, mask_words;
+};
+AcShape ac_shape(int n, int nf, int sms);
+void launch_ac_sparse(const AcArgs& a, int nf, const AcShape& s, cudaStream_t st);
 
 // Transient forward / adjoint over a batch: one warp per instance.
 void launch_atran(const BatchArgs& a, const AtranArgs& t, int grid, cudaStream_t s);
