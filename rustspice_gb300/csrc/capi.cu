@@ -198,24 +198,34 @@ int make_cta_groups(const gk::Plan& p, int sms, std::vector<i32>& grp, std::vect
   return rows;
 }
 
-// The solve as a step program (k_solve_steps): every operation the column
-// sweeps perform, in their order - per BTF block in solve order the
-// coupling terms of its rows, the forward sweep (L columns ascending), the
-// backward sweep (per column descending: the pivot division, then its U
-// entries) - as (destination row, source row, value index, kind), each
-// placed in the first step after the last step that writes its source or
-// its destination and after the last step that reads its destination. Every
-// row then sees its updates in the sweeps' order, so the results are the
-// sweeps' bit for bit. Plans whose solution vector does not fit one block's
-// shared memory get none.
-void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector<i32>& out_ptr) {
-  out_ops.clear();
-  out_ptr.clear();
-  if (p.n == 0 || (size_t)8 * p.n + 16 > (size_t)(227 * 1024)) return;
-  std::vector<int4> ops;
+// The solve as a list of operations (destination row, source row, value
+// index, kind: 0 subtract lu[value] times the source, 2 the same with ax, 1
+// divide by the pivot lu[value]), in the order the column sweeps perform
+// them: per BTF block in solve order the coupling terms of its rows, the
+// forward sweep (L columns ascending), the backward sweep (per column
+// descending: the pivot division, then its U entries). transpose: the solve
+// with A^T - per block in reverse the coupling, U^T ascending (a column's U
+// entries, then the division), L^T descending (each row's L entries subtract
+// its value: a row's terms then come in the order their sources are known;
+// k_tsolve, row by row, takes them in the opposite order).
+void solve_op_list(const gk::Plan& p, std::vector<int4>& ops, bool transpose) {
+  ops.clear();
   for (int bb = 0; bb < p.nblocks; ++bb) {
-    const int b = p.offd_lower ? bb : p.nblocks - 1 - bb;
+    const int b = (transpose ? !p.offd_lower : p.offd_lower) ? bb : p.nblocks - 1 - bb;
     const int b0 = p.block_ptr[b], b1 = p.block_ptr[b + 1];
+    if (transpose) {
+      for (int k = b0; k < b1; ++k) {
+        for (int e = p.offdT_ptr[k]; e < p.offdT_ptr[k + 1]; ++e)
+          ops.push_back(make_int4(k, p.offdT_row[e], p.offdT_raw[e], 2));
+        for (int q = p.col_ptr[k]; q < p.dslot[k]; ++q)
+          ops.push_back(make_int4(k, p.slot_row[q], q, 0));
+        ops.push_back(make_int4(k, -1, p.dslot[k], 1));
+      }
+      for (int k = b1 - 1; k >= b0; --k)
+        for (int e = p.lrow_ptr[k]; e < p.lrow_ptr[k + 1]; ++e)
+          ops.push_back(make_int4(p.lrow_col[e], k, p.lrow_slot[e], 0));
+      continue;
+    }
     for (int i = b0; i < b1; ++i)
       for (int e = p.offd_ptr[i]; e < p.offd_ptr[i + 1]; ++e)
         ops.push_back(make_int4(i, p.offd_col[e], p.offd_raw[e], 2));
@@ -228,7 +238,23 @@ void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector
         ops.push_back(make_int4(p.slot_row[q], j, q, 0));
     }
   }
-  std::vector<int> lw(p.n, 0), lr(p.n, 0), step(ops.size());
+}
+
+// Operations per chunk of the step-program solve: the most that fit twice
+// beside the solution vector of n rows in one block's shared memory, or 0.
+int solve_chunk(int n) {
+  for (int ch = 1024; ch >= 32 && n > 0; ch /= 2)
+    if (gk::solve_steps_bytes(n, ch) <= (size_t)(227 * 1024)) return ch;
+  return 0;
+}
+
+// The first step each operation can run in: after the last step that writes
+// its source or its destination and after the last step that reads its
+// destination. Every row then sees its updates in the list's order, so the
+// results are the sweeps' bit for bit. Returns the number of steps.
+int solve_op_steps(int n, const std::vector<int4>& ops, std::vector<int>& step) {
+  std::vector<int> lw(n, 0), lr(n, 0);
+  step.assign(ops.size(), 0);
   int nsteps = 0;
   for (size_t q = 0; q < ops.size(); ++q) {
     const int4 o = ops[q];
@@ -239,6 +265,19 @@ void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector
     if (o.y >= 0) lr[o.y] = std::max(lr[o.y], st);
     nsteps = std::max(nsteps, st);
   }
+  return nsteps;
+}
+
+// The operations by step (the plan's step program). Plans whose solution
+// vector does not fit one block's shared memory get none.
+void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector<i32>& out_ptr) {
+  out_ops.clear();
+  out_ptr.clear();
+  if (p.n == 0 || (size_t)8 * p.n + 16 > (size_t)(227 * 1024)) return;
+  std::vector<int4> ops;
+  std::vector<int> step;
+  solve_op_list(p, ops, false);
+  const int nsteps = solve_op_steps(p.n, ops, step);
   std::vector<i32> cnt(nsteps + 2, 0);
   for (int st : step) ++cnt[st];
   out_ptr.assign(nsteps + 1, 0);
@@ -248,18 +287,273 @@ void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector
   for (size_t q = 0; q < ops.size(); ++q) out_ops[pos[step[q] - 1]++] = ops[q];
 }
 
+// The step program as k_solve_steps runs it. A step of up to 32 operations
+// is a row of 32 slots that the first warp runs alone, a larger one rows of
+// `width` slots, one per compute thread, padded with operations that do
+// nothing; consecutive rows of a kind are a segment, and segments are cut
+// into chunks of at most `chunk` slots and gk::kSolveSegs segments.
+//
+// A row of the system whose updates outnumber the steps they wait for (the
+// ground and supply rows: thousands of terms, all but a few of them known
+// early) would make as many steps of one operation. The tail of such a run -
+// the updates that come after the step in which its last source is known -
+// becomes one chain operation instead, which a warp runs: 32 products at a
+// time, subtracted one after another in the same order. Chains are taken
+// from `least` updates on, and `least` (none, 6 or 24) is chosen by the
+// estimated time: about 200 cycles a row, 114 more with a division, 40 for a
+// barrier, and 64 a term for a step's longest chain (an FP64 operation waits 64
+// cycles for the one before). On the 120x120 mesh with 1000 inverters 7
+// chains take the solve from 11,252 rows to 6,666.
+struct SolveProgram {
+  std::vector<int4> ops, chunks, chains;
+  std::vector<int2> segs, terms;
+  int chunk = 0, width = 0;
+};
+
+// One row's updates from `first` on, as a chain standing at operation `last`.
+struct SolveChain {
+  int last;            // its last operation: where it stands in the list
+  std::vector<int> q;  // its operations, in order
+};
+
+// The steps with chains of at least `least` updates: st[q] operation q's step
+// (0 inside a chain), chain[q] its chain or -1. Returns the number of steps.
+int chain_steps(int n, const std::vector<int4>& ops, std::vector<int>& step, int nsteps, int least,
+                std::vector<int>& chain, std::vector<SolveChain>& chains) {
+  const size_t no = ops.size();
+  chain.assign(no, -1);
+  chains.clear();
+  // runs: consecutive subtractions into one row, nothing reading the row and
+  // nothing writing a source in between. prev[q]: the operation before q in
+  // q's run; arr[q]: the step after which the run's sources up to q are known
+  std::vector<int> tail(n, -1), len(n, 0), lw(n, 0), prev(no), arr(no);
+  std::vector<int> ends;
+  auto close = [&](int d) {
+    if (tail[d] >= 0 && len[d] >= least) ends.push_back(tail[d]);
+    tail[d] = -1;
+    len[d] = 0;
+  };
+  for (size_t q = 0; q < no; ++q) {
+    const int4 o = ops[q];
+    if (o.y >= 0) close(o.y);  // a read ends the source row's run
+    if (o.w == 1) {
+      close(o.x);
+    } else {
+      const int t = tail[o.x];
+      prev[q] = t;
+      arr[q] = std::max(t >= 0 ? arr[t] : 0, lw[o.y]);
+      ++len[o.x];
+      tail[o.x] = (int)q;
+    }
+    lw[o.x] = step[q];
+  }
+  for (int d = 0; d < n; ++d) close(d);
+  // the tail of a run after the step in which its last source is known
+  for (int e : ends) {
+    SolveChain ch{e, {}};
+    for (int q = e; q >= 0 && step[q] > arr[e]; q = prev[q]) ch.q.push_back(q);
+    if ((int)ch.q.size() < least) continue;
+    std::reverse(ch.q.begin(), ch.q.end());
+    for (int q : ch.q) chain[q] = (int)chains.size();
+    chains.push_back(std::move(ch));
+  }
+  if (chains.empty()) return nsteps;
+  // steps again, a chain standing at its last operation; a source written
+  // between its operation and that place would be read too late: such a chain
+  // (none in the lists solve_op_list makes) voids them all
+  std::vector<int> lr(n, 0), ready(chains.size(), 0), held(n, -1);
+  std::fill(lw.begin(), lw.end(), 0);
+  int ns = 0;
+  for (size_t q = 0; q < no; ++q) {
+    const int4 o = ops[q];
+    const int c = chain[q];
+    if (held[o.x] >= 0 && chains[held[o.x]].last > (int)q) {
+      chain.assign(no, -1);
+      chains.clear();
+      solve_op_steps(n, ops, step);
+      return nsteps;
+    }
+    int s = std::max(lw[o.x], lr[o.x]) + 1;
+    if (o.y >= 0) s = std::max(s, lw[o.y] + 1);
+    if (c >= 0) {
+      ready[c] = std::max(ready[c], s);
+      if (held[o.y] < 0 || chains[held[o.y]].last < chains[c].last) held[o.y] = c;
+      if (chains[c].last != (int)q) {
+        step[q] = 0;
+        continue;
+      }
+      s = ready[c];  // the writers after it wait for the chain's reads
+      for (int i : chains[c].q) lr[ops[i].y] = std::max(lr[ops[i].y], s);
+    } else if (o.y >= 0) {
+      lr[o.y] = std::max(lr[o.y], s);
+    }
+    step[q] = s;
+    lw[o.x] = s;
+    ns = std::max(ns, s);
+  }
+  return ns;
+}
+
+// Estimated cycles of a schedule (the rule above).
+double solve_cycles(const std::vector<int4>& ops, const std::vector<int>& st, int ns,
+                    const std::vector<int>& chain, const std::vector<SolveChain>& chains,
+                    int width) {
+  std::vector<int> cnt(ns + 1, 0), longest(ns + 1, 0);
+  std::vector<char> div(ns + 1, 0);
+  for (size_t q = 0; q < ops.size(); ++q) {
+    if (st[q] == 0) continue;
+    if (chain[q] >= 0) {
+      longest[st[q]] = std::max(longest[st[q]], (int)chains[chain[q]].q.size());
+    } else {
+      ++cnt[st[q]];
+      div[st[q]] |= ops[q].w == 1;
+    }
+  }
+  double cyc = 0.0;
+  for (int t = 1; t <= ns; ++t) {
+    const int rows = cnt[t] <= 32 ? 1 : (cnt[t] + width - 1) / width;
+    cyc += (cnt[t] ? 200.0 * rows + (div[t] ? 114.0 : 0.0) + (cnt[t] > 32 ? 40.0 : 0.0) : 0.0) +
+           (longest[t] ? 400.0 + 64.0 * longest[t] : 0.0);
+  }
+  return cyc;
+}
+
+// The program's slots, segments and chunks for a schedule.
+void lay_out_solve(const std::vector<int4>& ops, const std::vector<int>& st, int ns,
+                   const std::vector<int>& chain, const std::vector<SolveChain>& chains, int chunk,
+                   SolveProgram& out) {
+  const size_t no = ops.size();
+  std::vector<i32> ptr(ns + 2, 0);
+  for (size_t q = 0; q < no; ++q)
+    if (st[q] > 0) ++ptr[st[q]];
+  for (int t = 1; t <= ns + 1; ++t) ptr[t] += ptr[t - 1];
+  std::vector<i32> at(ptr.begin(), ptr.end()), by(ptr[ns]);
+  for (size_t q = 0; q < no; ++q)
+    if (st[q] > 0) by[at[st[q] - 1]++] = (i32)q;
+  out = SolveProgram();
+  out.chunk = chunk;
+  out.width = std::min(gk::kSolveRow, chunk);
+  out.ops.reserve(by.size() + (size_t)32 * ns);
+  int slot0 = 0, seg0 = 0;  // the open chunk's first slot and segment
+  auto close = [&]() {
+    if ((int)out.segs.size() > seg0)
+      out.chunks.push_back(make_int4(slot0, (int)out.ops.size() - slot0, seg0,
+                                     (int)out.segs.size() - seg0));
+    slot0 = (int)out.ops.size();
+    seg0 = (int)out.segs.size();
+  };
+  // a row (or, with first >= 0, `count` chains from there) joins the open
+  // segment of its kind
+  auto add = [&](int kind, int slots, int count, int first) {
+    const bool joins = (int)out.segs.size() > seg0 && first < 0 &&
+                       (out.segs.back().x & 3) == kind;
+    if ((int)out.ops.size() - slot0 + slots > chunk ||
+        (!joins && (int)out.segs.size() - seg0 >= gk::kSolveSegs))
+      close();
+    if ((int)out.segs.size() > seg0 && first < 0 && (out.segs.back().x & 3) == kind)
+      out.segs.back().x += count << 2;
+    else
+      out.segs.push_back(make_int2(kind | count << 2, first));
+  };
+  std::vector<int> chs, plain;
+  for (int t = 1; t <= ns; ++t) {
+    chs.clear();
+    plain.clear();
+    for (int e = ptr[t - 1]; e < ptr[t]; ++e) (chain[by[e]] >= 0 ? chs : plain).push_back(by[e]);
+    if (!chs.empty()) {
+      const int first = (int)out.chains.size();
+      for (int q : chs) {
+        const SolveChain& ch = chains[chain[q]];
+        out.chains.push_back(make_int4(ops[q].x, (int)out.terms.size(), (int)ch.q.size(), 0));
+        for (int i : ch.q)
+          out.terms.push_back(make_int2(ops[i].y, ops[i].w == 2 ? ~ops[i].z : ops[i].z));
+      }
+      add(gk::kSolveSegChain, 0, (int)chs.size(), first);
+    }
+    const int m = (int)plain.size();
+    const int kind = m <= 32 ? gk::kSolveSegSolo : gk::kSolveSegWide;
+    const int row = m <= 32 ? 32 : out.width;
+    for (int e0 = 0; e0 < m; e0 += row) {
+      const int cnt = std::min(row, m - e0);
+      bool div = false;
+      for (int e = e0; e < e0 + cnt; ++e) div |= ops[plain[e]].w == 1;
+      add(kind, row, 1, -1);
+      // the row's flags, in every slot: a division among its operations, the
+      // last row of its step
+      const int fl = (div ? 4 : 0) | (e0 + row >= m ? 8 : 0);
+      for (int e = e0; e < e0 + row; ++e) {
+        int4 o = make_int4(0, 0, 0, 3);
+        if (e < m) {
+          o = ops[plain[e]];
+          if (o.w == 1) o.y = o.x;  // a division's source is its own row
+        }
+        o.w |= fl;
+        out.ops.push_back(o);
+      }
+    }
+  }
+  close();
+}
+
+void make_solve_program(const gk::Plan& p, bool transpose, SolveProgram& out) {
+  out = SolveProgram();
+  const int chunk = solve_chunk(p.n);
+  if (chunk == 0) return;
+  std::vector<int4> ops;
+  std::vector<int> step;
+  solve_op_list(p, ops, transpose);
+  const int nsteps = solve_op_steps(p.n, ops, step);
+  std::vector<int> chain(ops.size(), -1), best_step, best_chain;
+  std::vector<SolveChain> chains, best_chains;
+  int best_ns = nsteps;
+  double best = solve_cycles(ops, step, nsteps, chain, chains, std::min(gk::kSolveRow, chunk));
+  best_step = step;
+  best_chain = chain;
+  for (int least : {6, 24}) {
+    std::vector<int> s = step;
+    const int ns = chain_steps(p.n, ops, s, nsteps, least, chain, chains);
+    if (chains.empty()) break;  // nor any longer ones
+    const double cyc = solve_cycles(ops, s, ns, chain, chains, std::min(gk::kSolveRow, chunk));
+    if (cyc < best) {
+      best = cyc;
+      best_ns = ns;
+      best_step.swap(s);
+      best_chain.swap(chain);
+      best_chains.swap(chains);
+    }
+  }
+  lay_out_solve(ops, best_step, best_ns, best_chain, best_chains, chunk, out);
+}
+
+// Device copy of a SolveProgram.
+struct SolveDev {
+  DBuf<int4> ops, chunks, chains;
+  DBuf<int2> segs, terms;
+  cudaError_t upload(const SolveProgram& sp, cudaStream_t s, gk::SolveSched& d) {
+    cudaError_t e = ops.upload(sp.ops, s);
+    if (e == cudaSuccess) e = chunks.upload(sp.chunks, s);
+    if (e == cudaSuccess) e = segs.upload(sp.segs, s);
+    if (e == cudaSuccess) e = chains.upload(sp.chains, s);
+    if (e == cudaSuccess) e = terms.upload(sp.terms, s);
+    d = gk::SolveSched{(int)sp.chunks.size(), sp.chunk, sp.width, ops.p,
+                       chunks.p, chains.p, segs.p, terms.p};
+    return e;
+  }
+};
+
 // Device copy of a Plan.
 struct PlanDev {
   DBuf<i32> col_ptr, dslot, slot_row, upd_ptr, upd_dst, col_single, amap_ptr, amap_idx,
       offd_ptr, offd_col, offd_raw, offdT_ptr, offdT_row, offdT_raw, lrow_ptr, lrow_col,
       lrow_slot, urow_ptr, urow_col,
       urow_slot, in_row, out_col, pcol_ptr, pcol_raw, pcol_q, pos_block, block_ptr, task,
-      ttask, cs_chunk, cs_op, cs_grp, cs_gchunk, cs_gop, ss_ptr;
-  DBuf<int4> ss_ops;
+      ttask, cs_chunk, cs_op, cs_grp, cs_gchunk, cs_gop;
+  SolveDev ss, sst;  // the solve's step program; the transpose solve's, made when first used
   gk::DPlan dp{}, dpt{};
   int64_t updates = 0;  // multiply-subtract pairs of one refactorization
 
-  cudaError_t upload(const gk::Plan& p, cudaStream_t s) {
+  // solves: the plan's solves run too (not the pivot-free plan's)
+  cudaError_t upload(const gk::Plan& p, cudaStream_t s, bool solves) {
     std::vector<i32> h_in_row(p.n), h_out_col(p.n), bp(p.block_ptr.begin(), p.block_ptr.end());
     for (int r = 0; r < p.n; ++r) h_in_row[p.in_pos[r]] = r;
     for (int c = 0; c < p.n; ++c) h_out_col[p.out_pos[c]] = c;
@@ -287,17 +581,12 @@ struct PlanDev {
     if (e == cudaSuccess) e = cs_grp.upload(hg, s);
     if (e == cudaSuccess) e = cs_gchunk.upload(hgc, s);
     if (e == cudaSuccess) e = cs_gop.upload(hgo, s);
-    std::vector<int4> sso;
-    std::vector<i32> ssp;
+    SolveProgram sp;
     const char* ess = getenv("GPUKLU_SOLVE_STEPS");
-    if (!(ess && ess[0] == '0')) make_solve_steps(p, sso, ssp);
-    if (e == cudaSuccess) e = ss_ops.upload(sso, s);
-    if (e == cudaSuccess) e = ss_ptr.upload(ssp, s);
+    if (solves && !(ess && ess[0] == '0')) make_solve_program(p, false, sp);
     updates = (int64_t)p.upd_dst.size();
     gk::DPlan d{};
-    d.ss_nsteps = ssp.empty() ? 0 : (int)ssp.size() - 1;
-    d.ss_ops = ss_ops.p;
-    d.ss_ptr = ss_ptr.p;
+    if (e == cudaSuccess) e = ss.upload(sp, s, d.ss);
     d.n = p.n;
     d.noffd = p.offd_ptr.empty() ? 0 : p.offd_ptr.back();
     d.cs_nchunk = (int)(hc.size() / 4);
@@ -344,7 +633,15 @@ struct PlanDev {
     dpt = d;
     dpt.task = ttask.p;
     dpt.ntask = (int)tt.size();
+    dpt.ss = gk::SolveSched{};
     return e;
+  }
+
+  // The transpose solve's step program, on its first use.
+  cudaError_t upload_transpose(const gk::Plan& p, cudaStream_t s) {
+    SolveProgram sp;
+    make_solve_program(p, true, sp);
+    return sst.upload(sp, s, dpt.ss);
   }
 };
 
@@ -663,7 +960,7 @@ struct gpuklu_handle {
   }
 
   int upload_plan() {
-    cudaError_t e = pd.upload(plan, stream);
+    cudaError_t e = pd.upload(plan, stream, true);
     apply_spin_limit();
     if (e == cudaSuccess) e = d_lu.resize(std::max(plan.nslots(), 1));
     if (e != cudaSuccess) return cuda_fail(e, "upload plan");
@@ -712,7 +1009,7 @@ struct gpuklu_handle {
     last_ai.assign(ai, ai + ai_len);
     cudaError_t e = cudaSuccess;
     if (!pd_sym_ok) {
-      e = pd_sym.upload(sym_plan, stream);
+      e = pd_sym.upload(sym_plan, stream, false);
       apply_spin_limit();
       if (e != cudaSuccess) return cuda_fail(e, "upload plan");
       pd_sym_ok = true;
@@ -989,8 +1286,13 @@ struct gpuklu_handle {
       if (!sync) return GPUKLU_OK;
       return check_status("dense solve");
     }
-    if (steps_sol && !transpose) {
-      gk::launch_solve_steps(pd.dp, d_rhs.p, d_ax.p, d_lu.p, d_rec.p, d_out.p, stream);
+    if (steps_sol) {
+      if (transpose && pd.dpt.ss.nchunks == 0) {
+        const cudaError_t e = pd.upload_transpose(plan, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "transpose solve program");
+      }
+      gk::launch_solve_steps(transpose ? pd.dpt : pd.dp, transpose, d_rhs.p, d_ax.p, d_lu.p,
+                             d_rec.p, d_out.p, stream);
       if (!sync) return GPUKLU_OK;
       return check_status("solve");
     }

@@ -883,90 +883,220 @@ __global__ void __launch_bounds__(256) k_solve_cta(DPlan P, const double* __rest
   for (int i = tid; i < m; i += blockDim.x) out[P.out_col[r0 + i]] = w[i];
 }
 
-// a / b correctly rounded, from y = 1/b correctly rounded, by Markstein's
-// correction (P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q = a y is
-// within an ulp of a / b, the residual r = a - b q is exact in one fma, and
-// q + r y rounded to nearest is the correctly rounded quotient. Three
-// dependent FP64 operations instead of a division's sequence. Operands or a
-// quotient near the ends of the exponent range (zeros, subnormals,
-// infinities, NaN included) take the division itself; the exponent tests are
-// integer operations.
-__device__ __forceinline__ double div_markstein(double a, double b, double y) {
-  const double q = a * y;
-  const unsigned ea = (unsigned)(__double_as_longlong(a) >> 52) & 0x7ffu;
-  const unsigned eb = (unsigned)(__double_as_longlong(b) >> 52) & 0x7ffu;
-  const unsigned eq = (unsigned)(__double_as_longlong(q) >> 52) & 0x7ffu;
-  if (ea - 64u > 1919u || eb - 64u > 1919u || eq - 64u > 1919u) return a / b;
-  const double r = fma(-b, q, a);
-  return fma(r, y, q);
+// The solve as a step program, one thread block, the solution vector in
+// shared memory. The pivots' reciprocals come first (n divisions in
+// parallel); then four compute warps run the rows - the operations the column
+// sweeps perform, in the reference's order for every row of the system (each
+// update a separately rounded product and difference, the pivot division
+// exact), one per thread - while four loader warps fetch the next chunk's
+// operations and matrix values into the other half of a shared double
+// buffer.
+//
+// Both kinds of operation are one formula: p = v T[s], r = c p + T[d] in one
+// rounding, with v the matrix value and c = -1 for an update (r = T[d] - p).
+// A division a / b is Markstein's correction (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34(1), 1990) from the correctly rounded reciprocal y = 1/b: with s = d,
+// v = y and c = -b, p is within an ulp of a / b, r = a - b p is exact and
+// r y + p is the correctly rounded quotient; only rows with a division spend
+// that third operation. Operands or a quotient near the ends of the exponent
+// range (zeros, subnormals, infinities, NaN included) take the division
+// itself; the tests are integer operations on the exponents of a, b and y
+// (the quotient's is the sum of a's and y's, or one more), so none waits for
+// an FP64 result.
+//
+// A step costs its latency: a shared load, two dependent FP64 operations (64
+// cycles each, and 50 more until anything but an FP64 operation sees the
+// result), a shared store and, when more than one warp is at it, the
+// barrier. Compute warps that fetch from global memory themselves, however
+// far ahead, take 430 to 620 cycles a step (a warp's few scoreboards are
+// shared by the loads in flight and the FP64 results), hence the loader
+// warps; with 128 loader threads the loads set the pace, 256 to 896 take the
+// same time. Measured against one set of 128 threads that loads two steps
+// ahead and no chains, per solve: 32x32 diode mesh 274 -> 119 us, 48x48 589 ->
+// 235 us, 120x120 mesh with 1000 inverters 8.26 -> 1.97 ms; its transpose
+// solve, a grid kernel before, 19.4 -> 1.97 ms.
+constexpr int kSolveLoaders = 256, kLoadBatch = 4;
+constexpr int kSolveStepsThreads = kSolveRow + kSolveLoaders;
+// flags in a slot's destination address (a multiple of 8 otherwise)
+constexpr unsigned kSlotDivRow = 1u, kSlotLast = 2u, kSlotDiv = 4u;
+constexpr unsigned kSlotSlow = 1u;  // in its source address
+
+__device__ __forceinline__ double lds_f64(unsigned a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_f64(unsigned a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ unsigned exponent_of(double a) {
+  return (unsigned)(__double2hiint(a) >> 20) & 0x7ffu;
 }
 
-// The solve as a step program, one thread block: the solution vector in
-// shared memory, the pivots' reciprocals computed first (n divisions in
-// parallel), then step by step the operations the column sweeps perform, in
-// the reference's order for every row (each row's updates separately rounded
-// products and differences, the pivot division exact), the operations of a
-// step spread over the block's threads. A step's operation, its matrix value
-// and (for a division) its reciprocal are loaded two steps ahead: none of
-// them depends on the solution.
-constexpr int kSolveStepsThreads = 128;
-
-struct SolveOp {
-  int4 o;
-  double v, y;
-};
-
 __global__ void __launch_bounds__(kSolveStepsThreads)
-    k_solve_steps(DPlan P, const double* __restrict__ rhs, const double* __restrict__ ax,
-                  const double* __restrict__ lu, double* rec, double* out) {
+    k_solve_steps(SolveSched S, int n, const int* __restrict__ in, const int* __restrict__ outp,
+                  const int* __restrict__ dslot, const double* __restrict__ rhs,
+                  const double* __restrict__ ax, const double* __restrict__ lu, double* rec,
+                  double* out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* const T = reinterpret_cast<double*>(smem_raw);
-  const int tid = threadIdx.x, n = P.n;
+  double* const T = reinterpret_cast<double*>(smem_raw);  // the solution, a spare entry at n
+  double2* const svc = reinterpret_cast<double2*>(T + ((n + 2) & ~1));  // (v, c) of every slot
+  uint2* const sad = reinterpret_cast<uint2*>(svc + 2 * S.chunk);  // destination, source address
+  int2* const sseg = reinterpret_cast<int2*>(sad + 2 * S.chunk);   // segments, an end mark
+  const unsigned T0 = (unsigned)__cvta_generic_to_shared(T);
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int i = tid; i < n; i += blockDim.x) {
-    T[i] = rhs[P.in_row[i]];
-    rec[i] = 1.0 / lu[P.dslot[i]];
+    T[i] = rhs[in[i]];
+    rec[i] = 1.0 / lu[dslot[i]];
   }
+  if (tid == 0) T[n] = 0.0;
   __syncthreads();
-  const int4* const ops = P.ss_ops;
-  const int* const sp = P.ss_ptr;
-  const int ns = P.ss_nsteps;
-  const int nops = sp[ns];
-  auto fetch = [&](int p) {
-    SolveOp f;
-    f.o = make_int4(0, -1, 0, 3);
-    f.v = 0.0;
-    f.y = 0.0;
-    if (p < nops) {
-      f.o = __ldg(ops + p);
-      f.v = f.o.w == 2 ? __ldg(ax + f.o.z) : __ldg(lu + f.o.z);
-      if (f.o.w == 1) f.y = __ldcg(rec + f.o.x);  // written above by this block
+  // chunk c into its half of the buffer, by the threads from tid0 on:
+  // kLoadBatch operations' loads in flight together, then their values'
+  auto load = [&](int c, int tid0) {
+    const int4 C = __ldg(S.chunks + c);
+    const int h = (c & 1) * S.chunk, hs = (c & 1) * (kSolveSegs + 1), nt = blockDim.x - tid0;
+    for (int i = tid - tid0; i <= C.w; i += nt)
+      sseg[hs + i] = i < C.w ? __ldg(S.segs + C.z + i) : make_int2(3, -1);
+    for (int i0 = tid - tid0; i0 < C.y; i0 += kLoadBatch * nt) {
+      int4 o[kLoadBatch];
+      double m[kLoadBatch], y[kLoadBatch];
+#pragma unroll
+      for (int u = 0; u < kLoadBatch; ++u)
+        o[u] = i0 + u * nt < C.y ? __ldg(S.ops + C.x + i0 + u * nt) : make_int4(0, 0, 0, 3);
+#pragma unroll
+      for (int u = 0; u < kLoadBatch; ++u) {
+        const int kind = o[u].w & 3;
+        m[u] = kind != 3 ? __ldg((kind == 2 ? ax : lu) + o[u].z) : 0.0;
+        y[u] = kind == 1 ? __ldcg(rec + o[u].x) : 0.0;  // written above by this block
+      }
+#pragma unroll
+      for (int u = 0; u < kLoadBatch; ++u) {
+        const int i = i0 + u * nt, kind = o[u].w & 3;
+        if (i >= C.y) break;
+        const bool div = kind == 1, none = kind == 3;
+        const bool slow =
+            div && (exponent_of(m[u]) - 64u > 1919u || exponent_of(y[u]) - 64u > 1919u);
+        svc[h + i] = make_double2(div ? y[u] : m[u], div ? -m[u] : (none ? 0.0 : -1.0));
+        sad[h + i] =
+            make_uint2((T0 + 8u * (unsigned)(none ? n : o[u].x)) | (unsigned)(o[u].w >> 2) |
+                           (div ? kSlotDiv : 0u),
+                       (T0 + 8u * (unsigned)(none ? n : o[u].y)) | (slow ? kSlotSlow : 0u));
+      }
     }
-    return f;
   };
-  auto exec = [&](const SolveOp& f) {
-    const int d = f.o.x;
-    if (f.o.w == 1)
-      T[d] = div_markstein(T[d], f.v, f.y);
-    else if (f.o.w != 3)
-      T[d] = __dsub_rn(T[d], __dmul_rn(f.v, T[f.o.y]));
+  // one chain: 32 products, then their differences in order (every lane
+  // computes them); terms fetched two chunks ahead, values one
+  auto run_chain = [&](int4 o) {
+    const int2 nt = make_int2(0, 0);
+    const int2* const tp = S.terms + o.y;
+    auto value = [&](int z) { return __ldg(z < 0 ? ax + ~z : lu + z); };
+    double v = T[o.x];
+    int2 t0 = lane < o.z ? __ldg(tp + lane) : nt;
+    int2 t1 = lane + 32 < o.z ? __ldg(tp + lane + 32) : nt;
+    double c0 = lane < o.z ? value(t0.y) : 0.0;
+    for (int b = 0; b < o.z; b += 32) {
+      const double c1 = b + 32 + lane < o.z ? value(t1.y) : 0.0;
+      const int2 t2 = b + 64 + lane < o.z ? __ldg(tp + b + 64 + lane) : nt;
+      const double p = __dmul_rn(c0, T[t0.x]);
+      const int cnt = min(32, o.z - b);
+      if (cnt == 32) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v = __dsub_rn(v, __shfl_sync(FULL, p, i));
+      } else {
+        for (int i = 0; i < cnt; ++i) v = __dsub_rn(v, __shfl_sync(FULL, p, i));
+      }
+      t0 = t1;
+      t1 = t2;
+      c0 = c1;
+    }
+    if (lane == 0) T[o.x] = v;
   };
-  int s0 = sp[0], s1 = ns >= 1 ? sp[1] : s0, s2 = ns >= 2 ? sp[2] : s1, s3 = ns >= 3 ? sp[3] : s2;
-  SolveOp f0 = fetch(s0 + tid), f1 = fetch(s1 + tid);
-  for (int t = 0; t < ns; ++t) {
-    const SolveOp f2 = fetch(s2 + tid);
-    const int s4 = t + 4 <= ns ? sp[t + 4] : s3;
-    if (s0 + tid < s1) exec(f0);
-    for (int p = s0 + tid + kSolveStepsThreads; p < s1; p += kSolveStepsThreads) exec(fetch(p));
+  // one slot's operation
+  auto exec = [&](uint2 a, double2 vc) {
+    const unsigned da = a.x & ~7u;
+    const double td = lds_f64(da), ts = lds_f64(a.y & ~7u);
+    const double p = vc.x * ts;
+    double r = fma(vc.y, p, td);
+    if (a.x & kSlotDivRow) {
+      const double q = fma(r, vc.x, p);
+      if (a.x & kSlotDiv) {
+        const unsigned ea = exponent_of(td);
+        r = q;
+        if ((a.y & kSlotSlow) || ea - 64u > 1919u || ea + exponent_of(vc.x) - 1088u > 1917u)
+          r = td / -vc.y;
+      }
+    }
+    sts_f64(da, r);
+  };
+  if (S.nchunks > 0) load(0, 0);
+  __syncthreads();
+  for (int c = 0; c < S.nchunks; ++c) {
+    if (tid >= kSolveRow) {
+      if (c + 1 < S.nchunks) load(c + 1, kSolveRow);
+    } else {
+      const int2* seg = sseg + (c & 1) * (kSolveSegs + 1);
+      int base = (c & 1) * S.chunk;
+      int2 next = *seg;
+      while ((next.x & 3) != 3) {
+        const int2 g = next;
+        next = *++seg;
+        const int kind = g.x & 3, cnt = g.x >> 2;
+        if (kind == kSolveSegSolo) {
+          // two register sets, each slot's operands read a row ahead
+          if (tid < 32) {
+            const uint2* pa = sad + base + lane;
+            const double2* pv = svc + base + lane;
+            uint2 a0 = pa[0], a1 = a0;
+            double2 v0 = pv[0], v1 = v0;
+            int q = 0;
+            for (; q + 2 <= cnt; q += 2) {
+              a1 = pa[32];
+              v1 = pv[32];
+              exec(a0, v0);
+              __syncwarp();
+              pa += 64;
+              pv += 64;
+              if (q + 2 < cnt) {
+                a0 = pa[0];
+                v0 = pv[0];
+              }
+              exec(a1, v1);
+              __syncwarp();
+            }
+            if (q < cnt) exec(a0, v0);
+          }
+          base += 32 * cnt;
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        } else if (kind == kSolveSegWide) {
+          const bool on = tid < S.width;
+          const uint2* pa = sad + base + (on ? tid : 0);
+          const double2* pv = svc + base + (on ? tid : 0);
+          uint2 a0 = pa[0], a1 = a0;
+          double2 v0 = pv[0], v1 = v0;
+          for (int q = 0; q < cnt; ++q) {
+            pa += S.width;
+            pv += S.width;
+            if (q + 1 < cnt) {
+              a1 = *pa;
+              v1 = *pv;
+            }
+            if (on) exec(a0, v0);
+            if (a0.x & kSlotLast) asm volatile("bar.sync 1, 128;" ::: "memory");
+            a0 = a1;
+            v0 = v1;
+          }
+          base += S.width * cnt;
+        } else {
+          for (int m = tid >> 5; m < cnt; m += kSolveRow >> 5) run_chain(__ldg(S.chains + g.y + m));
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
+      }
+    }
     __syncthreads();
-    s0 = s1;
-    s1 = s2;
-    s2 = s3;
-    s3 = s4;
-    f0 = f1;
-    f1 = f2;
   }
-  for (int i = tid; i < n; i += blockDim.x) out[P.out_col[i]] = T[i];
+  for (int i = tid; i < n; i += blockDim.x) out[outp[i]] = T[i];
 }
 
 // --------------------------------------------------------------- devices
@@ -1657,15 +1787,18 @@ void launch_solve_cta(const DPlan& P, const double* rhs, const double* ax, const
 }
 
 bool solve_steps_fits(const DPlan& P) {
-  return P.n > 0 && P.ss_nsteps > 0 && (size_t)8 * P.n + 16 <= (size_t)smem_optin();
+  return P.n > 0 && P.ss.nchunks > 0 &&
+         solve_steps_bytes(P.n, P.ss.chunk) <= (size_t)smem_optin();
 }
 
-void launch_solve_steps(const DPlan& P, const double* rhs, const double* ax, const double* lu,
-                        double* rec, double* out, cudaStream_t s) {
-  const size_t bytes = (size_t)8 * P.n + 16;
+void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,
+                        const double* lu, double* rec, double* out, cudaStream_t s) {
+  const size_t bytes = solve_steps_bytes(P.n, P.ss.chunk);
   if (bytes > 48 * 1024)
     cudaFuncSetAttribute(k_solve_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  k_solve_steps<<<1, kSolveStepsThreads, bytes, s>>>(P, rhs, ax, lu, rec, out);
+  k_solve_steps<<<1, kSolveStepsThreads, bytes, s>>>(
+      P.ss, P.n, transpose ? P.out_col : P.in_row, transpose ? P.in_row : P.out_col, P.dslot, rhs,
+      ax, lu, rec, out);
 }
 
 bool solve_groups_fit(const DPlan& P) {

@@ -10,6 +10,28 @@ namespace gk {
 // seconds of waiting at most. A handle may lower it (gpuklu_set_spin_limit).
 constexpr unsigned kSpinLimit = 1u << 22;
 
+// A solve as a step program (k_solve_steps): slots of operations (destination
+// row, source row, value index, kind 0 subtract lu[value] times the source,
+// 1 divide by lu[value], 2 as 0 with ax[value], 3 nothing; | 4 when the row
+// of slots has a division, | 8 in the last row of its step), grouped into
+// segments (kind | count << 2, first chain or -1): rows of 32 slots that one
+// warp runs, rows of `width` slots, or chains (destination row, first term,
+// terms; a term: source row, lu value or ~ax value), and those into chunks
+// (first slot, slots, first segment, segments). 0 chunks: none.
+constexpr int kSolveRow = 128;   // compute threads
+constexpr int kSolveSegs = 64;   // segments of a chunk, at most
+enum { kSolveSegSolo = 0, kSolveSegWide = 1, kSolveSegChain = 2 };
+struct SolveSched {
+  int nchunks, chunk, width;
+  const int4 *ops, *chunks, *chains;
+  const int2 *segs, *terms;
+};
+// Shared memory of k_solve_steps: the solution and a spare entry, then twice
+// a chunk's slots (two doubles, two words) and segments.
+inline size_t solve_steps_bytes(int n, int chunk) {
+  return (size_t)8 * ((n + 2) & ~1) + (size_t)2 * chunk * 24 + (size_t)2 * (kSolveSegs + 1) * 8;
+}
+
 // Device pointers of one Plan (see analysis.h for the meaning of each array).
 struct DPlan {
   int n, nslots, nblocks, ntask;
@@ -29,13 +51,7 @@ struct DPlan {
   // and chunks [grp[4g+2], grp[4g+3]) of cs_gchunk / cs_gop.
   int cs_ngrp, cs_grp_rows;     // groups; rows of the largest
   const int *cs_grp, *cs_gchunk, *cs_gop;
-  // The solve as a step program (k_solve_steps): ss_ptr[ss_nsteps] operations
-  // (destination row, source row or -1, value index, kind: 0 lu value, 2
-  // coupling ax value, 1 division by the pivot lu[value]), ss_nsteps + 1
-  // step pointers; 0 steps: none.
-  int ss_nsteps;
-  const int4* ss_ops;
-  const int* ss_ptr;
+  SolveSched ss;  // the solve (dp) or the transpose solve (dpt) as a step program
   // Polls of a dependency flag before a waiting warp gives up and reports
   // DS_TIMEOUT (kSpinLimit unless the handle sets another).
   unsigned spin_limit;
@@ -257,9 +273,10 @@ void launch_refactor_cta(const DPlan& P, const double* ax, double* lu, int* stat
                          cudaStream_t s, const PivotCheck& pc = PivotCheck());
 bool solve_cta_fits(const DPlan& P);
 bool solve_steps_fits(const DPlan& P);
-// rec: n doubles of scratch (the pivots' reciprocals)
-void launch_solve_steps(const DPlan& P, const double* rhs, const double* ax, const double* lu,
-                        double* rec, double* out, cudaStream_t s);
+// rec: n doubles of scratch (the pivots' reciprocals); transpose: P.ss is
+// the transpose solve's program
+void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,
+                        const double* lu, double* rec, double* out, cudaStream_t s);
 // One block per group of uncoupled BTF blocks (cs_grp); fits when the
 // largest group's rows fit one block's shared memory.
 bool solve_groups_fit(const DPlan& P);
