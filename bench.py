@@ -546,7 +546,8 @@ def run_gpu(a):
     fp64 = float(np.sum(f_inst * itt))
     fp64_tflops = fp64 / (ms_step * 1e-3) / 1e12
     fp64_peak = float(N.lib().gpuklu_fp64_peak_tflops())
-    cap = phases[0]["lane_cap"]
+    # with the continuation kernel every iteration is its own
+    cap = 0 if bt.info()["cont_kernel"] else phases[0]["lane_cap"]
     lane_it = np.minimum(itt, cap) if cap > 0 else np.zeros_like(itt)
     second = "k_batch_cont" if bt.info()["cont_kernel"] else "k_batch_newton"
     kern = {}
@@ -670,11 +671,12 @@ def _converged_only_step(B, conv, cfg, flush, dev, steps, sched=None):
     ms = _timed_runs(bt, cfg, flush, max(3, steps // 2))
     _, itt, rs, _ = bt.results(with_x=False)
     ph = bt.phase_ms()
+    kernels = {"k_batch_cont": ph["warps_ms"]} if bt.info()["cont_kernel"] else \
+        {"k_batch_lanes": ph["lanes_ms"], "k_batch_newton": ph["warps_ms"]}
     bt.close()
     return {"instances": int(B.ninst - len(idx)), "converged_only_ms_per_step": ms,
             "converged_only_iterations": int(itt.sum()),
-            "converged_only_kernel_ms": {"k_batch_lanes": ph["lanes_ms"],
-                                         "continuation": ph["warps_ms"]},
+            "converged_only_kernel_ms": kernels,
             "how": "the same batch with only the converged instances, timed the same way; "
                    "the capped instances cost the difference to ms_per_step"}
 

@@ -312,10 +312,10 @@ gpuklu_batch* gpuklu_batch_create(int64_t ncirc, const int64_t* dev_off,
                                   const double* inst_val, const double* x0,
                                   const int64_t* x0_off, int64_t x0_len);
 void gpuklu_batch_destroy(gpuklu_batch* b);
-/* Runs every instance's Newton loop on the device: a lane-per-instance
- * kernel for the first lane_cap iterations, then the continuation kernel (one
- * warp per instance still iterating; the warp classes when it is off); with
- * lane_cap 0 the continuation kernel starts every instance. */
+/* Runs every instance's Newton loop on the device: one warp per instance, the
+ * programs in up to eight classes by size, all classes concurrent. With that
+ * kernel switched off: a lane-per-instance kernel for the first lane_cap
+ * iterations, then the warp classes for the instances still iterating. */
 int gpuklu_batch_run(gpuklu_batch* b, const gpuklu_newton_config* cfg);
 /* Results: per instance iterations (final run), total iterations, exit
  * reason, and x (n of its circuit values, at x_out + x_off[i]; x_off may be
@@ -350,12 +350,11 @@ void* gpuklu_batch_stream(gpuklu_batch* b);
  * lane phase). */
 int gpuklu_batch_phase_ms(gpuklu_batch* b, double* out);
 /* The batch's schedule; no counterpart in the reference. lane_cap: Newton
- * iterations an instance runs in the lane-per-instance phase before it is
- * parked for the continuation (default 6; ignored when that phase is off;
- * 0 with the continuation kernel: no lane phase, the continuation starts
- * every instance); cont_tiles: shared-program tiles per circuit program in
- * the warp classes' continuation (default 2; the continuation kernel has
- * none). Results agree across schedules to the batch's 1e-10 bar (an
+ * iterations an instance runs with the lane-per-instance kernel's order of
+ * additions (default 6; with the warp-per-instance kernel switched off, in
+ * that kernel before it is parked for the warp classes); cont_tiles: shared-program tiles per circuit program in
+ * the warp classes' continuation (default 2; the warp-per-instance kernel
+ * has none). Results agree across schedules to the batch's 1e-10 bar (an
  * instance's arithmetic differs between the kernels only in rounding). */
 int gpuklu_batch_set_schedule(gpuklu_batch* b, int lane_cap, int cont_tiles);
 /* Autotuner: times one run of the batch per candidate schedule (lane_cap in

@@ -15,6 +15,9 @@
 // of each solve: DC (capacitor open), BE (g = C/dt, rhs += be_sign g v_prev;
 // be_sign -1 is the reference's sign, +1 the physical one), trapezoidal
 // (g = 2C/dt, rhs += g v_prev + i_prev).
+// The factorization and substitutions are the program's row stream
+// (bt::run_stream). Measured, 512 chains of 8-64 stages, 0-2 ns: 166.7 -> 62.1
+// ms against the columns one after another.
 #include <cfloat>
 
 #include "batch_common.cuh"
@@ -82,8 +85,9 @@ __device__ void stamp_step(const BatchArgs& A, const AtranArgs& T, const bt::Pro
                            double* DV, int sl) {
   bt::stamp_devices<LPI>(P, dparams, -1, 0.0, X, X, A.cfg.gmin, 1e-12, true, DV, sl);
   __syncwarp();
-  for (int d = sl; d < P.ndev; d += LPI) {
-    if (P.dev_type[d] != 5) continue;
+  for (int q = P.nev - P.ncap + sl; q < P.nev; q += LPI) {
+    const int4 e = __ldg(P.ev + q);
+    const int d = e.x;
     const double C = __ldg(dparams + 4 * d);
     double g = 0.0, ieq = 0.0;
     if (s.mode == BE) {
@@ -93,8 +97,8 @@ __device__ void stamp_step(const BatchArgs& A, const AtranArgs& T, const bt::Pro
       g = 2.0 * C / s.dt;
       ieq = g * s.capv[d] + s.capi[d];
     }
-    DV[P.dev_dv[d]] = g;
-    DV[P.dev_dv[d] + 1] = ieq;
+    DV[e.w] = g;
+    DV[e.w + 1] = ieq;
   }
   for (int r = w0 + sl; r < w1; r += LPI) DV[P.dev_dv[T.wave_dev[r]]] = wave_value(T, r, s.t);
   __syncwarp();
@@ -105,15 +109,14 @@ __device__ void stamp_step(const BatchArgs& A, const AtranArgs& T, const bt::Pro
 // on convergence X takes the whole solution. Returns 0 when converged.
 __device__ int newton_atran(const BatchArgs& A, const AtranArgs& T, const bt::Prog& P,
                             const double* dparams, int w0, int w1, double* X, int m,
-                            const Step& s, double* TS, double* DV, double* V, int sl,
-                            int& iters) {
+                            const Step& s, double* TS, double* DV, double* V, int2* ring,
+                            int sl, int& iters) {
   const NewtonCfg& cfg = A.cfg;
   double damp = cfg.damping, prev = DBL_MAX;
   for (int it = 0; it < cfg.max_iters; ++it) {
     stamp_step(A, T, P, dparams, w0, w1, X, s, DV, sl);
     bt::assemble<LPI>(P, DV, V, TS, sl);
-    __syncwarp();
-    bt::factor_solve<LPI>(P, V, TS, sl);
+    bt::run_stream<LPI>(P.stream, ring, TS - P.nc, sl, P.nc + P.n + P.nv + 1);
     bool conv = true;
     double ss = 0.0;
     for (int c = sl; c < m; c += LPI) {
@@ -145,7 +148,7 @@ __global__ void k_atran(BatchArgs A, AtranArgs T) {
   const int lane = threadIdx.x & 31, sl = lane;
   unsigned char* const sbase =
       smem_raw + (size_t)(threadIdx.x >> 5) * ((size_t)A.prog_ints * 4 + (size_t)A.region * 8);
-  int* const sprog = reinterpret_cast<int*>(sbase);
+  int2* const ring = reinterpret_cast<int2*>(sbase);
   double* const sreg = reinterpret_cast<double*>(sbase + (size_t)A.prog_ints * 4);
   while (true) {
     int inst = 0;
@@ -153,17 +156,20 @@ __global__ void k_atran(BatchArgs A, AtranArgs T) {
     inst = __shfl_sync(bt::kFull, inst, 0);
     if (inst >= A.ninst) return;
     const GroupHdr G = A.groups[A.inst_group[inst]];
-    bt::Prog P = bt::stage_program(A, G, sprog, lane);
+    const bt::Prog P = bt::global_view(A, G);
     const int nc = P.nc, n = P.n, ndev = P.ndev;
     double* const X = sreg;        // the last accepted point (n)
     double* const XB = X + n;      // backward-Euler solve (n)
     double* const XT = XB + n;     // trapezoidal solve (n)
-    double* const TS = XT + n;     // right-hand side / solution (n)
-    double* const CV = TS + n;     // capacitor voltage at the last point (ndev)
-    double* const CI = CV + ndev;  // trapezoidal history current (ndev)
+    double* const TS = XT + n;     // right-hand side / solution (n), then V and
+    double* const V = TS + n;      // two constants: the row stream's entries
+    double* const CV = V + P.nv + 2;  // capacitor voltage at the last point (ndev)
+    double* const CI = CV + ndev;     // trapezoidal history current (ndev)
     double* const DV = CI + ndev;
-    double* const V = DV + G.ndv;
-    P.map = reinterpret_cast<int*>(V + P.nv);
+    if (sl == 0) {
+      V[P.nv] = 1.0;
+      V[P.nv + 1] = 0.0;
+    }
     const double* dparams = A.dparams + A.inst_p_off[inst];
     const int w0 = T.wave_ptr[inst], w1 = T.wave_ptr[inst + 1];
     const int b0 = T.bp_ptr[inst], b1 = T.bp_ptr[inst + 1];
@@ -176,7 +182,7 @@ __global__ void k_atran(BatchArgs A, AtranArgs T) {
     int iters = 0, status = 0, npts = 0, acc = 0, rej = 0;
     // ---- DC operating point at tstart (engine.rs:412-451)
     Step st{DC, T.tstart, 0.0, CV, CI};
-    if (newton_atran(A, T, P, dparams, w0, w1, X, nc, st, TS, DV, V, sl, iters)) status = 2;
+    if (newton_atran(A, T, P, dparams, w0, w1, X, nc, st, TS, DV, V, ring, sl, iters)) status = 2;
     const double min_dt = fmax(T.tstep * 1e-6, 1e-15);
     const double max_dt = fmin(T.tmax, T.tstop / 10.0);
     double t = T.tstart, dt = fmin(T.tstep, max_dt);
@@ -220,9 +226,9 @@ __global__ void k_atran(BatchArgs A, AtranArgs T) {
       __syncwarp();
       Step sb{BE, tt, dt, CV, CI};
       Step sr{TRAP, tt, dt, CV, CI};
-      bool fail = newton_atran(A, T, P, dparams, w0, w1, XB, n, sb, TS, DV, V, sl, iters) != 0;
+      bool fail = newton_atran(A, T, P, dparams, w0, w1, XB, n, sb, TS, DV, V, ring, sl, iters) != 0;
       if (!fail)
-        fail = newton_atran(A, T, P, dparams, w0, w1, XT, n, sr, TS, DV, V, sl, iters) != 0;
+        fail = newton_atran(A, T, P, dparams, w0, w1, XT, n, sr, TS, DV, V, ring, sl, iters) != 0;
       if (fail) {  // Newton failed: a quarter of the step, at least min_dt
         ++consecutive;
         ++rej;

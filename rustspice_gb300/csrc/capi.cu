@@ -1992,7 +1992,8 @@ struct gpuklu_batch {
   DBuf<i32> d_order, d_dev_type, d_dev_nodes, d_dev_dv, d_amap_ptr, d_amap_code,
       d_rmap_ptr, d_rmap_code, d_col_ptr, d_dslot, d_col_single, d_in_row, d_out_pos,
       d_offd_ptr, d_slot_row, d_upd_ptr, d_upd_dst, d_offd_col, d_block_ptr, d_heavy, d_ov_dev,
-      d_lvl_col, d_lseg_ptr, d_lseg, d_amap4, d_rmap4, d_lng, d_ops, d_step_ptr,
+      d_lvl_col, d_lseg_ptr, d_lseg, d_amap4, d_rmap4, d_lng, d_ops, d_step_ptr, d_recs, d_segs, d_asm4,
+      d_asm_dst, d_ev,
       d_iters,
       d_iters_total, d_reason, d_status;
   DBuf<double> d_dparams, d_ov_val, d_x0, d_xout;
@@ -2045,7 +2046,14 @@ struct gpuklu_batch {
   // continuation kernel: one warp per parked instance from a queue over the
   // groups (cont.cu); off: the warp classes continue them
   bool cont_kernel = false;
-  int cont_grid = 0, cont_wpb = 0, cont_m = 1;
+  // its classes: programs of similar size in one launch each, on its own stream
+  struct ContClass {
+    int m = 1, grid = 0, slice = 0, dvs = 0, dvx = 0, first = 0, count = 0;
+    long long dv_off = 0;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done = nullptr;
+  };
+  std::vector<ContClass> cont;
   DBuf<i32> d_cont_groups;
   DBuf<unsigned> d_cont_cursor;
   DBuf<double> d_dv;
@@ -2075,6 +2083,10 @@ struct gpuklu_batch {
       if (c->stream) cudaStreamDestroy(c->stream);
       if (c->done) cudaEventDestroy(c->done);
     }
+    for (auto& c : cont) {
+      if (c.stream) cudaStreamDestroy(c.stream);
+      if (c.done) cudaEventDestroy(c.done);
+    }
     if (start_ev) cudaEventDestroy(start_ev);
     for (auto& ev : ph_ev)
       if (ev) cudaEventDestroy(ev);
@@ -2096,6 +2108,10 @@ struct Program {
       offd_col, block_ptr, heavy, lvl_col, lseg_ptr, lseg, amap4, rmap4, lng;
   std::vector<i32> ops;       // step program: two ints per operation
   std::vector<i32> step_ptr;  // nsteps + 1 (empty: no step program)
+  // row streams (two words per record and per segment; empty: none)
+  std::vector<i32> stream, sseg, tstream, tsseg;
+  std::vector<i32> asm4, asm_dst;  // assembly records, longest lists first
+  std::vector<i32> ev;        // devices to evaluate (four words each)
   int64_t flops = 0, bytes = 0;
   std::string key() const {
     std::string k;
@@ -2183,18 +2199,14 @@ void device_codes(int type, int dv, bool transient, int m[8], int r[2]) {
 // destination, so a step's operations are independent and each value sees
 // its operations in the original order. Regions beyond 15-bit offsets get no
 // step program.
-void build_steps(const gk::Plan& P, int nc, int ndv, std::vector<i32>& out_ops,
-                 std::vector<i32>& out_steps) {
-  out_ops.clear();
-  out_steps.clear();
+struct StepOp {
+  int d, a, b, c, k;
+};
+
+// The operations of the factorization and both substitutions in their order.
+void factor_ops(const gk::Plan& P, int nc, int ndv, std::vector<StepOp>& ops) {
   const int n = P.n, nslots = P.nslots();
   const long long vbase = (long long)nc + n + ndv;
-  const long long top = vbase + nslots + (long long)P.offd_raw.size();
-  if (top >= 32768 || n == 0) return;
-  struct Op {
-    int d, a, b, c, k;
-  };
-  std::vector<Op> ops;
   auto T_ = [nc](int i) { return nc + i; };
   auto V_ = [vbase](long long v) { return (int)(vbase + v); };
   std::vector<int> pend_a((size_t)nslots, -1), pend_b((size_t)nslots, -1);
@@ -2253,10 +2265,41 @@ void build_steps(const gk::Plan& P, int nc, int ndv, std::vector<i32>& out_ops,
       }
     }
   }
-  std::vector<int> lw((size_t)top, 0), lr((size_t)top, 0), step(ops.size());
+}
+
+// The transpose solve with the factors (bt::run_stream on the same region):
+// on entry T[out_pos[c]] holds the right-hand side of column c, on exit T[i]
+// the solution of row in_row[i]. Blocks in reverse; U^T ascending, each row's
+// terms in order and its pivot's reciprocal fused into the last; L^T
+// descending, every row subtracting its value from the rows its L entries
+// name; then the block's coupling into the earlier blocks.
+void transpose_ops(const gk::Plan& P, int nc, std::vector<StepOp>& ops) {
+  const int n = P.n, nslots = P.nslots(), vbase = nc + n;
+  for (int b = P.nblocks - 1; b >= 0; --b) {
+    const int b0 = P.block_ptr[b], b1 = P.block_ptr[b + 1];
+    for (int k = b0; k < b1; ++k) {
+      const int ds = P.dslot[k];
+      for (int s = P.col_ptr[k]; s < ds; ++s)
+        ops.push_back({nc + k, vbase + s, nc + P.slot_row[s], s + 1 == ds ? vbase + ds : 0,
+                       s + 1 == ds ? 6 : 0});
+      if (P.col_ptr[k] == ds) ops.push_back({nc + k, nc + k, vbase + ds, 0, 2});
+    }
+    for (int k = b1 - 1; k >= b0; --k)
+      for (int e = P.lrow_ptr[k]; e < P.lrow_ptr[k + 1]; ++e)
+        ops.push_back({nc + P.lrow_col[e], vbase + P.lrow_slot[e], nc + k, 0, 0});
+    for (int i = b0; i < b1; ++i)
+      for (int e = P.offd_ptr[i]; e < P.offd_ptr[i + 1]; ++e)
+        ops.push_back({nc + P.offd_col[e], vbase + nslots + e, nc + i, 0, 0});
+  }
+}
+
+// The step of every operation (from 1); returns how many there are.
+int place_ops(const std::vector<StepOp>& ops, size_t top, std::vector<int>& step) {
+  std::vector<int> lw(top, 0), lr(top, 0);
+  step.assign(ops.size(), 0);
   int nsteps = 0;
   for (size_t q = 0; q < ops.size(); ++q) {
-    const Op& o = ops[q];
+    const StepOp& o = ops[q];
     int st = std::max(lw[o.d], lr[o.d]) + 1;
     if (o.k != 1) st = std::max(st, std::max(lw[o.a], lw[o.b]) + 1);
     if (o.k >= 5) st = std::max(st, lw[o.c] + 1);
@@ -2269,6 +2312,33 @@ void build_steps(const gk::Plan& P, int nc, int ndv, std::vector<i32>& out_ops,
     if (o.k >= 5) lr[o.c] = std::max(lr[o.c], st);
     nsteps = std::max(nsteps, st);
   }
+  return nsteps;
+}
+
+// 15-bit offsets: a region with one more entry pair for the row stream's
+// constants.
+bool offsets_fit(const gk::Plan& P, int nc, int ndv) {
+  return P.n > 0 &&
+         (long long)nc + P.n + ndv + P.nslots() + (long long)P.offd_raw.size() < 32768 - 2;
+}
+
+i32 op_word0(const StepOp& o) {
+  return (i32)((unsigned)o.d | ((unsigned)o.a << 15) | (((unsigned)o.k & 3u) << 30));
+}
+i32 op_word1(const StepOp& o) {
+  return (i32)((unsigned)o.b | ((unsigned)o.c << 15) | (((unsigned)o.k >> 2) << 30));
+}
+
+void build_steps(const gk::Plan& P, int nc, int ndv, std::vector<i32>& out_ops,
+                 std::vector<i32>& out_steps) {
+  out_ops.clear();
+  out_steps.clear();
+  const size_t top = (size_t)nc + P.n + ndv + P.nslots() + P.offd_raw.size();
+  if (top >= 32768 || P.n == 0) return;
+  std::vector<StepOp> ops;
+  std::vector<int> step;
+  factor_ops(P, nc, ndv, ops);
+  const int nsteps = place_ops(ops, top, step);
   std::vector<i32> cnt(nsteps + 2, 0);
   for (int st : step) ++cnt[st];
   out_steps.assign(nsteps + 1, 0);
@@ -2276,12 +2346,105 @@ void build_steps(const gk::Plan& P, int nc, int ndv, std::vector<i32>& out_ops,
   std::vector<i32> pos(out_steps.begin(), out_steps.end() - 1);
   out_ops.assign(2 * ops.size(), 0);
   for (size_t q = 0; q < ops.size(); ++q) {  // program order within a step
-    const Op& o = ops[q];
+    const StepOp& o = ops[q];
     const int at = pos[step[q] - 1]++;
-    out_ops[2 * at] = (i32)((unsigned)o.d | ((unsigned)o.a << 15) | (((unsigned)o.k & 3u) << 30));
-    out_ops[2 * at + 1] =
-        (i32)((unsigned)o.b | ((unsigned)o.c << 15) | (((unsigned)o.k >> 2) << 30));
+    out_ops[2 * at] = op_word0(o);
+    out_ops[2 * at + 1] = op_word1(o);
   }
+}
+
+// The operations as a row stream (bt::run_stream): per step its reciprocals,
+// then the others in rows, plain or (any of them with a second product)
+// fused, as wide as the step (8, 16 or 32 records, wider steps in several
+// rows), consecutive rows of a kind and width as one segment. Runs of steps
+// of one operation become one segment: serial where each operation's b is the
+// d of the one before, sum where all have the same d.
+// top: the region's entry behind the values, which holds 1.0 (c of operations
+// without a second product in a fused row); the next one is for idle lanes.
+// recs: two words per record, whole chunks; segs: two words per segment.
+void make_stream(const std::vector<StepOp>& ops, const std::vector<int>& step, int nsteps, int top,
+                 std::vector<i32>& recs, std::vector<i32>& segs) {
+  std::vector<i32> ptr(nsteps + 2, 0), by(ops.size());
+  for (int st : step) ++ptr[st];
+  for (int t = 1; t <= nsteps + 1; ++t) ptr[t] += ptr[t - 1];
+  {
+    std::vector<i32> at(ptr.begin(), ptr.end());
+    for (size_t q = 0; q < ops.size(); ++q) by[at[step[q] - 1]++] = (i32)q;
+  }
+  auto size = [&](int t) { return ptr[t] - ptr[t - 1]; };
+  auto only = [&](int t) -> const StepOp& { return ops[by[ptr[t - 1]]]; };
+  recs.clear();
+  segs.clear();
+  const StepOp idle{top + 1, top + 1, top + 1, top + 1, 0};
+  auto put = [&](StepOp o, bool rcp) {
+    if (!rcp && o.k < 5) o.c = top;
+    recs.push_back(op_word0(o));
+    recs.push_back(op_word1(o));
+  };
+  auto align = [&]() {
+    while (recs.size() % (2 * gk::kStreamAlign)) put(idle, true);
+  };
+  int last = -1;  // the open row segment's key
+  auto row = [&](int kind, const std::vector<int>& v) {
+    const int lw = v.size() <= 8 ? 3 : (v.size() <= 16 ? 4 : 5), W = 1 << lw;
+    const int key = kind | lw << 3;
+    for (size_t p = 0; p < v.size(); p += W) {
+      if (key != last) {
+        align();
+        segs.insert(segs.end(), {key, 0});
+        last = key;
+      }
+      ++segs.back();
+      for (size_t q = p; q < p + W; ++q) put(q < v.size() ? ops[v[q]] : idle, false);
+    }
+  };
+  auto list = [&](int kind, const std::vector<int>& v) {
+    align();
+    segs.insert(segs.end(), {kind, (i32)v.size()});
+    for (int q : v) put(ops[q], kind == gk::kRowRcp);
+    last = -1;
+  };
+  std::vector<int> run, rcp, rest;
+  for (int t = 1; t <= nsteps; ++t) {
+    if (size(t) == 1) {
+      // a run of one-operation steps from here
+      run.assign(1, by[ptr[t - 1]]);
+      int kind = -1;
+      for (int u = t + 1; u <= nsteps && size(u) == 1; ++u) {
+        const StepOp &o = only(u), &l = ops[run.back()];
+        if (o.k == 1 || l.k == 1) break;
+        // serial: nothing an operation reads but b comes from the run
+        bool serial = kind != gk::kRowSum && o.b == l.d && o.k == 6 && l.k == 6 && o.a != o.d &&
+                      o.c != o.d;
+        if (serial)
+          for (int q : run) serial &= o.d != ops[q].d && o.a != ops[q].d && o.c != ops[q].d;
+        // sum: plain updates of one entry, the last with its product
+        const bool sum = kind != gk::kRowSerial && o.d == l.d && (l.k == 0 || l.k == 4) &&
+                         o.k != 2 && o.a != o.d && o.b != o.d && (o.k < 5 || o.c != o.d);
+        if (!serial && !sum) break;
+        kind = serial ? gk::kRowSerial : gk::kRowSum;
+        run.push_back(by[ptr[u - 1]]);
+      }
+      const StepOp& f = ops[run[0]];
+      if (run.size() >= 3 && f.a != f.d && f.b != f.d &&
+          (kind == gk::kRowSum || f.c != f.d)) {
+        list(kind, run);
+        t += (int)run.size() - 1;
+        continue;
+      }
+    }
+    rcp.clear();
+    rest.clear();
+    bool fused = false;
+    for (int e = ptr[t - 1]; e < ptr[t]; ++e) {
+      const int q = by[e];
+      (ops[q].k == 1 ? rcp : rest).push_back(q);
+      fused |= ops[q].k >= 5;
+    }
+    if (!rcp.empty()) list(gk::kRowRcp, rcp);
+    if (!rest.empty()) row(fused ? gk::kRowFused : gk::kRowPlain, rest);
+  }
+  while (recs.size() % (2 * gk::kStreamChunk)) put(idle, true);
 }
 
 Program make_program(const gpuklu_circuit& C, const gk::Plan& P) {
@@ -2427,8 +2590,21 @@ Program make_program(const gpuklu_circuit& C, const gk::Plan& P) {
       std::fill(g.lseg_ptr.begin(), g.lseg_ptr.end(), 0);
     }
   }
-  const char* esp = getenv("GPUKLU_STEP_PROGRAM");
-  if (!C.transient && !(esp && esp[0] == '0')) build_steps(P, C.node_count, 0, g.ops, g.step_ptr);
+  // devices to evaluate: by type (a warp's lanes then take one branch),
+  // capacitors last and only where they are stamped
+  {
+    const int order[] = {6, 4, 3, 0, 1, 2, 5};
+    for (int ty : order)
+      for (int d = 0; d < C.ndev; ++d) {
+        if (C.type[d] != ty || (ty == 5 && !C.transient)) continue;
+        const int* nd = &C.nodes[(size_t)d * 4];
+        const bool three = ty == 4 || ty == 6;
+        g.ev.insert(g.ev.end(), {d, nd[0] | nd[1] << 16, (three ? nd[2] : 0) | ty << 16,
+                                 g.dev_dv[d]});
+        if (ty == 5) ++h.ncap;
+      }
+    h.nev = (int)(g.ev.size() / 4);
+  }
   // FP64 operations of one Newton iteration: device evaluation, assembly
   // additions, refactorization, both substitutions, block coupling, update
   const int64_t nl = P.nnz_l, nu = P.nnz_u - P.n;
@@ -2439,6 +2615,49 @@ Program make_program(const gpuklu_circuit& C, const gk::Plan& P) {
                    6 * (nl + nu) + 6LL * P.n + 4LL * h.node_count);
   h.cost = (int)std::min<int64_t>(g.flops, 0x7fffffff);
   return g;
+}
+
+// The program's assembly records, step program and row streams (once per
+// program, not per circuit).
+void finish_program(const gpuklu_circuit& C, const gk::Plan& P, Program& g) {
+  {
+    const int nv = g.h.nslots + g.h.noffd, n = P.n;
+    std::vector<std::pair<int, int>> by;  // (codes, destination): T at 0, V at n
+    auto codes = [](const std::vector<i32>& m, int i) {
+      int k = 0;
+      while (k < 4 && m[(size_t)4 * i + k] != 4) ++k;
+      return k;
+    };
+    for (int i = 0; i < n; ++i) by.push_back({codes(g.rmap4, i), i});
+    for (int v = 0; v < nv; ++v) by.push_back({codes(g.amap4, v), n + v});
+    std::stable_sort(by.begin(), by.end(), [](const std::pair<int, int>& a,
+                                              const std::pair<int, int>& b) {
+      return a.first > b.first;
+    });
+    for (auto& e : by) {
+      const i32* src = e.second < n ? &g.rmap4[(size_t)4 * e.second]
+                                    : &g.amap4[(size_t)4 * (e.second - n)];
+      g.asm4.insert(g.asm4.end(), src, src + 4);
+      g.asm_dst.push_back(e.second);
+    }
+  }
+  const char* esp = getenv("GPUKLU_STEP_PROGRAM");
+  const bool steps = !(esp && esp[0] == '0');
+  if (!C.transient && steps) build_steps(P, C.node_count, 0, g.ops, g.step_ptr);
+  if ((C.transient || steps) && offsets_fit(P, C.node_count, 0)) {
+    const int top = C.node_count + P.n + g.h.nslots + g.h.noffd;
+    std::vector<StepOp> ops;
+    std::vector<int> step;
+    factor_ops(P, C.node_count, 0, ops);
+    int ns = place_ops(ops, (size_t)top, step);
+    make_stream(ops, step, ns, top, g.stream, g.sseg);
+    if (C.transient) {
+      ops.clear();
+      transpose_ops(P, C.node_count, ops);
+      ns = place_ops(ops, (size_t)top, step);
+      make_stream(ops, step, ns, top, g.tstream, g.tsseg);
+    }
+  }
 }
 
 // Circuit constants (4 per device) with the reference's arithmetic:
@@ -2570,6 +2789,7 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
       }
     if (gid < 0) {
       gid = (int)progs.size();
+      finish_program(*C, H->plan, pr);
       progs.push_back(std::move(pr));
       keys.push_back(std::move(k));
     }
@@ -2580,7 +2800,8 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
   const int ng = (int)progs.size();
   std::vector<i32> dev_type, dev_nodes, dev_dv, amap_ptr, amap_code, rmap_ptr, rmap_code,
       col_ptr, dslot, col_single, in_row, out_pos, offd_ptr, slot_row, upd_ptr, upd_dst,
-      offd_col, block_ptr, heavy, lvl_col, lseg_ptr, lseg, amap4, rmap4, lng, ops, step_ptr;
+      offd_col, block_ptr, heavy, lvl_col, lseg_ptr, lseg, amap4, rmap4, lng, ops, step_ptr,
+      recs, segs, asm4, asm_dst, ev;
   auto cat = [](std::vector<i32>& dst, const std::vector<i32>& src) {
     dst.insert(dst.end(), src.begin(), src.end());
   };
@@ -2611,6 +2832,24 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
     h.nsteps = pr.step_ptr.empty() ? 0 : (int)pr.step_ptr.size() - 1;
     cat(ops, pr.ops);
     cat(step_ptr, pr.step_ptr);
+    auto stream = [&](const std::vector<i32>& r, const std::vector<i32>& sg, int& off, int& nch,
+                      int& soff, int& nsg) {
+      const size_t words = 2 * gk::kStreamChunk;
+      off = (int)(recs.size() / words);
+      nch = (int)(r.size() / words);
+      soff = (int)(segs.size() / 2);
+      nsg = (int)(sg.size() / 2);
+      cat(recs, r);
+      cat(segs, sg);
+      segs.insert(segs.end(), 2, 0);  // the kernel reads one segment ahead
+    };
+    stream(pr.stream, pr.sseg, h.stream_off, h.nchunk, h.sseg_off, h.nsseg);
+    stream(pr.tstream, pr.tsseg, h.tstream_off, h.ntchunk, h.tsseg_off, h.ntsseg);
+    h.asm_off = (int)asm_dst.size();
+    cat(asm4, pr.asm4);
+    cat(asm_dst, pr.asm_dst);
+    h.ev_off = (int)(ev.size() / 4);
+    cat(ev, pr.ev);
     cat(dev_type, pr.dev_type);
     cat(dev_nodes, pr.dev_nodes);
     cat(dev_dv, pr.dev_dv);
@@ -2798,6 +3037,7 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
   UP(d_upd_dst, upd_dst) UP(d_offd_col, offd_col) UP(d_block_ptr, block_ptr)
   UP(d_heavy, heavy) UP(d_lvl_col, lvl_col) UP(d_lseg_ptr, lseg_ptr) UP(d_lseg, lseg)
   UP(d_amap4, amap4) UP(d_rmap4, rmap4) UP(d_lng, lng) UP(d_ops, ops) UP(d_step_ptr, step_ptr)
+  UP(d_recs, recs) UP(d_segs, segs) UP(d_asm4, asm4) UP(d_asm_dst, asm_dst) UP(d_ev, ev)
   UP(d_dparams, dparams) UP(d_p_off, poff) UP(d_ov_dev, ov_dev) UP(d_ov_val, ov_val)
   UP(d_x0_off, x0o) UP(d_x_off, B->x_off)
 #undef UP
@@ -2825,65 +3065,105 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
                                                  h.noffd + 4LL * h.ndev);
     }
     if (B->lanes && !B->ltiles.empty()) {
-      int regs = 0, bps = 0;
-      gk::lanes_kernel_info(B->lane_wpb, &regs, &bps);
-      const long long warps_max = (long long)sm_count() * std::max(bps, 1) * B->lane_wpb;
-      const long long warps = std::min<long long>(warps_max, (long long)B->ltiles.size());
-      B->lane_grid = (int)((warps + B->lane_wpb - 1) / B->lane_wpb);
-      const long long stride = lregion * 32;
-      if (e == cudaSuccess)
-        e = B->d_scratch.resize((size_t)B->lane_grid * B->lane_wpb * (size_t)stride);
-      if (e == cudaSuccess) e = B->d_ltiles.upload(B->ltiles, s);
-      if (e == cudaSuccess) e = B->d_lcounter.resize(1);
-      if (e == cudaSuccess) e = B->d_cont_list.resize(std::max<int64_t>(ninst, 1));
-      for (auto* b : {&B->d_cont_it, &B->d_cont_total, &B->d_cont_gstep})
-        if (e == cudaSuccess) e = b->resize(std::max<int64_t>(ninst, 1));
-      for (auto* b : {&B->d_cont_damp, &B->d_cont_prev})
-        if (e == cudaSuccess) e = b->resize(std::max<int64_t>(ninst, 1));
-      if (e == cudaSuccess) e = B->d_cont_count.resize(std::max(ngr, 1));
       if (e == cudaSuccess) e = B->d_gnext2.resize(std::max(ngr, 1));
-      B->args.warp_stride = stride;
-      // continuation kernel: a warp's shared slice holds X, T and the LU
-      // values of the largest program, its global slice the device records;
-      // as many warps per block as the slices fit (at most 16)
+      // Continuation kernel: a block (one warp) holds, per instance, T and the
+      // LU values in shared memory, sized for the largest program of its
+      // class, and the row stream's ring; the device records, the iterate and
+      // its differences in a slice of global memory. A class takes the
+      // programs down to 0.8 of its largest; the eighth takes the rest.
       const char* eck = getenv("GPUKLU_CONT_KERNEL");
-      int slice = 0, dvs = 0, ncs = 0;
-      bool steps_all = true;
-      for (int g : gorder) {
-        const gk::GroupHdr& h = B->groups[g];
-        slice = std::max(slice, h.n + h.nslots + h.noffd);
-        dvs = std::max(dvs, h.ndv);
-        ncs = std::max(ncs, h.node_count);
-        if (h.inst_count > 0 && h.nsteps == 0) steps_all = false;
-      }
-      slice = (slice + 1) & ~1;
-      const int dvx = (dvs + 3) & ~3;  // the iterate after the records
-      dvs = dvx + ((ncs + 3) & ~3);
-      // instances per warp: one; GPUKLU_CONT_M=2 puts two of a program in a
-      // warp (16 lanes each, a step's FP64 instruction serving both), which
-      // measured slower: the phase waits for its longest instances, and
-      // their iterations take longer with half the lanes
+      // Instances per warp: one. GPUKLU_CONT_M=2 puts two of a program in a
+      // warp (16 lanes each, a row's FP64 instruction serving both; the same
+      // results bit for bit): 976 instances take 10.3 ms against 7.6 ms, 249,856
+      // 70.3 ms against 69.2 ms, because an instance that runs to the
+      // iteration cap keeps its warp long after the other half has run out.
       const char* ecm = getenv("GPUKLU_CONT_M");
       const int cm = ecm && ecm[0] == '2' ? 2 : 1;
-      int wpb = std::min(16, (int)((size_t)(227 * 1024) / ((size_t)cm * slice * 8)));
-      if (const char* ecw = getenv("GPUKLU_CONT_WARPS")) wpb = std::max(1, std::min(wpb, atoi(ecw)));
-      if (!(eck && eck[0] == '0') && steps_all && wpb >= 1) {
-        int r3 = 0, b3 = 0;
-        gk::cont_kernel_info(cm, wpb, slice, &r3, &b3);
-        if (b3 > 0) {
-          B->cont_kernel = true;
-          B->cont_m = cm;
-          B->cont_wpb = wpb;
-          B->cont_grid = sm_count() * b3;
-          B->args.slice = slice;
-          B->args.dv_stride = dvs;
-          B->args.dv_x = dvx;
-          std::vector<i32> cg(gorder.begin(), gorder.end());
-          if (e == cudaSuccess) e = B->d_cont_groups.upload(cg, s);
-          if (e == cudaSuccess) e = B->d_cont_cursor.resize(1);
-          if (e == cudaSuccess)
-            e = B->d_dv.resize((size_t)B->cont_grid * wpb * cm * (size_t)dvs);
+      const char* ecw = getenv("GPUKLU_CONT_WARPS");  // resident warps per SM and class
+      int prio_low = 0, prio_high = 0;
+      if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess)
+        prio_low = prio_high = 0;
+      auto need = [&](int g) {
+        const gk::GroupHdr& h = B->groups[g];
+        return (h.n + h.nslots + h.noffd + 2 + 1) & ~1;
+      };
+      std::vector<int> by;
+      bool ok = !(eck && eck[0] == '0');
+      for (int g : gorder)
+        if (B->groups[g].inst_count > 0) {
+          by.push_back(g);
+          if (B->groups[g].nchunk == 0) ok = false;
         }
+      std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return need(x) > need(y); });
+      std::vector<i32> cg;
+      long long dv = 0;
+      for (size_t q = 0; ok && q < by.size();) {
+        gpuklu_batch::ContClass k;
+        k.slice = need(by[q]);
+        k.first = (int)cg.size();
+        const bool rest = B->cont.size() == 7;
+        int64_t inst = 0;
+        std::vector<int> in;
+        for (; q < by.size() && (rest || need(by[q]) * 5 >= k.slice * 4); ++q) {
+          const gk::GroupHdr& h = B->groups[by[q]];
+          k.dvx = std::max(k.dvx, (h.ndv + 3) & ~3);
+          k.dvs = std::max(k.dvs, h.node_count);
+          inst += h.inst_count;
+          in.push_back(by[q]);
+        }
+        k.dvs = (k.dvx + 2 * k.dvs + 3) & ~3;
+        std::stable_sort(in.begin(), in.end(), [&](int x, int y) {
+          return B->groups[x].cost > B->groups[y].cost;
+        });
+        cg.insert(cg.end(), in.begin(), in.end());
+        k.count = (int)in.size();
+        int regs = 0, per_sm = 0;
+        for (k.m = cm; k.m >= 1; --k.m) {
+          gk::cont_kernel_info(k.m, k.slice, &regs, &per_sm);
+          if (per_sm > 0) break;
+        }
+        if (per_sm <= 0) {
+          ok = false;
+          break;
+        }
+        if (ecw) per_sm = std::max(1, std::min(per_sm, atoi(ecw)));
+        k.grid = (int)std::min<int64_t>((int64_t)sm_count() * per_sm, (inst + k.m - 1) / k.m);
+        k.dv_off = dv;
+        dv += (long long)k.grid * k.m * k.dvs;
+        // All classes become ready at once; the priorities make the device
+        // start the largest programs first, so that an iteration-capped
+        // instance of a long chain is not what the call ends on.
+        if (cudaStreamCreateWithPriority(
+                &k.stream, cudaStreamNonBlocking,
+                std::min(prio_high + (int)B->cont.size(), prio_low)) != cudaSuccess ||
+            cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming) != cudaSuccess)
+          return nullptr;
+        B->cont.push_back(k);
+      }
+      if (ok) {
+        B->cont_kernel = true;
+        if (e == cudaSuccess) e = B->d_cont_groups.upload(cg, s);
+        if (e == cudaSuccess) e = B->d_cont_cursor.resize(B->cont.size());
+        if (e == cudaSuccess) e = B->d_dv.resize((size_t)dv);
+      }
+      if (!B->cont_kernel) {  // the lane kernel, then the warp classes
+        int regs = 0, bps = 0;
+        gk::lanes_kernel_info(B->lane_wpb, &regs, &bps);
+        const long long warps_max = (long long)sm_count() * std::max(bps, 1) * B->lane_wpb;
+        const long long nwarps = std::min<long long>(warps_max, (long long)B->ltiles.size());
+        B->lane_grid = (int)((nwarps + B->lane_wpb - 1) / B->lane_wpb);
+        const long long stride = lregion * 32;
+        if (e == cudaSuccess)
+          e = B->d_scratch.resize((size_t)B->lane_grid * B->lane_wpb * (size_t)stride);
+        if (e == cudaSuccess) e = B->d_ltiles.upload(B->ltiles, s);
+        if (e == cudaSuccess) e = B->d_lcounter.resize(1);
+        if (e == cudaSuccess) e = B->d_cont_list.resize(std::max<int64_t>(ninst, 1));
+        for (auto* b : {&B->d_cont_it, &B->d_cont_total, &B->d_cont_gstep})
+          if (e == cudaSuccess) e = b->resize(std::max<int64_t>(ninst, 1));
+        for (auto* b : {&B->d_cont_damp, &B->d_cont_prev})
+          if (e == cudaSuccess) e = b->resize(std::max<int64_t>(ninst, 1));
+        if (e == cudaSuccess) e = B->d_cont_count.resize(std::max(ngr, 1));
+        B->args.warp_stride = stride;
       }
     } else {
       B->lanes = false;
@@ -2938,6 +3218,11 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
   a.lng = B->d_lng.p;
   a.ops = reinterpret_cast<const int2*>(B->d_ops.p);
   a.step_ptr = B->d_step_ptr.p;
+  a.recs = reinterpret_cast<const int2*>(B->d_recs.p);
+  a.segs = reinterpret_cast<const int2*>(B->d_segs.p);
+  a.asm4 = B->d_asm4.p;
+  a.asm_dst = B->d_asm_dst.p;
+  a.ev = reinterpret_cast<const int4*>(B->d_ev.p);
   a.inst_p_off = B->d_p_off.p;
   a.dparams = B->d_dparams.p;
   a.inst_ov_dev = B->d_ov_dev.p;
@@ -2965,15 +3250,6 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
     a.cont_gstep = B->d_cont_gstep.p;
     a.cont_damp = B->d_cont_damp.p;
     a.cont_prev = B->d_cont_prev.p;
-    if (B->cont_kernel) {
-      a.cont_groups = B->d_cont_groups.p;
-      a.cont_ngroups = (int)B->d_cont_groups.n;
-      a.cont_cursor = B->d_cont_cursor.p;
-      a.dv_scratch = B->d_dv.p;
-      a.dv_stride = B->args.dv_stride;
-      a.dv_x = B->args.dv_x;
-      a.slice = B->args.slice;
-    }
   }
   B->args = a;
   for (auto& C : B->classes) {
@@ -3038,9 +3314,9 @@ gpuklu_batch* gpuklu_tran_create(int64_t ncirc, const int64_t* dev_off,
   int region = 0, prog = 0;
   for (int64_t i = 0; i < ninst; ++i) {
     const gk::GroupHdr& h = B->groups[B->inst_group_h[i]];
-    region = std::max(region, 2 * h.node_count + 2 * h.n + h.ndv + h.nslots + h.noffd + h.ndev +
-                                  (h.n + 1) / 2 + 1);
-    prog = std::max(prog, (4 * h.n + h.nslots + (h.nseg > 0 ? h.nslots + h.nupd : 0) + 3) & ~3);
+    region = std::max(region, 2 * h.node_count + 2 * h.n + h.ndv + h.nslots + h.noffd + 2 + h.ndev);
+    prog = gk::kStreamRing / 4;  // the row stream's ring
+    if (h.nchunk == 0) region = 1 << 20;  // no row stream: beyond any block's shared memory too
     ck_off[i] = ck;
     ck += nck * h.node_count;
     seg_off[i] = sg;
@@ -3142,9 +3418,9 @@ gpuklu_batch* gpuklu_atran_create(int64_t ncirc, const int64_t* dev_off,
   B->at_pwlptr.assign(1, 0);
   for (int64_t i = 0; i < ninst; ++i) {
     const gk::GroupHdr& h = B->groups[B->inst_group_h[i]];
-    region = std::max(region, 4 * h.n + 2 * h.ndev + h.ndv + h.nslots + h.noffd +
-                                  (h.n + 1) / 2 + 1);
-    prog = std::max(prog, (4 * h.n + h.nslots + (h.nseg > 0 ? h.nslots + h.nupd : 0) + 3) & ~3);
+    region = std::max(region, 4 * h.n + 2 * h.ndev + h.ndv + h.nslots + h.noffd + 2);
+    prog = gk::kStreamRing / 4;  // the row stream's ring
+    if (h.nchunk == 0) region = 1 << 20;  // no row stream: beyond any block's shared memory too
     probe_h[i] = (i32)probe[i];
     for (int64_t d = dev_off[i]; d < dev_off[i + 1]; ++d) {
       if (!wkind || wkind[d] == 0) continue;
@@ -3398,32 +3674,42 @@ int gpuklu_batch_run(gpuklu_batch* b, const gpuklu_newton_config* cfg) {
   if (!b || !cfg) return GPUKLU_INVALID_MATRIX;
   const gk::NewtonCfg c = to_newton_cfg(*cfg);
   cudaStream_t s = b->stream;
+  cudaEventRecord(b->ph_ev[0], s);
+  if (b->lanes && b->cont_kernel) {  // every class at once, the largest programs first
+    cudaMemsetAsync(b->d_gnext2.p, 0, b->d_gnext2.n * sizeof(unsigned), s);
+    cudaMemsetAsync(b->d_cont_cursor.p, 0, b->d_cont_cursor.n * sizeof(unsigned), s);
+    cudaEventRecord(b->ph_ev[1], s);
+    for (const auto& k : b->cont) {
+      cudaStreamWaitEvent(k.stream, b->ph_ev[1], 0);
+      gk::BatchArgs ca = b->args;
+      ca.cfg = c;
+      ca.cont_groups = b->d_cont_groups.p + k.first;
+      ca.cont_ngroups = k.count;
+      ca.cont_cursor = b->d_cont_cursor.p + (&k - b->cont.data());
+      ca.dv_scratch = b->d_dv.p + k.dv_off;
+      ca.dv_stride = k.dvs;
+      ca.dv_x = k.dvx;
+      ca.slice = k.slice;
+      gk::launch_batch_cont(ca, k.m, k.grid, k.stream);
+      cudaEventRecord(k.done, k.stream);
+      cudaStreamWaitEvent(s, k.done, 0);
+    }
+    cudaEventRecord(b->ph_ev[2], s);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return b->fail(cuda_msg(e, "batch launch"));
+    return GPUKLU_OK;
+  }
   cudaMemsetAsync(b->d_gnext.p, 0, b->d_gnext.n * sizeof(unsigned), s);
   for (auto& C : b->classes) cudaMemsetAsync(C->d_counter.p, 0, sizeof(unsigned), s);
   if (b->lanes) {  // phase 1: lane per instance, then the warp classes take the parked ones
     cudaMemsetAsync(b->d_lcounter.p, 0, sizeof(unsigned), s);
     cudaMemsetAsync(b->d_cont_count.p, 0, b->d_cont_count.n * sizeof(unsigned), s);
     cudaMemsetAsync(b->d_gnext2.p, 0, b->d_gnext2.n * sizeof(unsigned), s);
-  }
-  cudaEventRecord(b->ph_ev[0], s);
-  const bool fresh = b->lanes && b->cont_kernel && b->lane_cap == 0;
-  if (b->lanes && !fresh) {
     gk::BatchArgs la = b->args;
     la.cfg = c;
     gk::launch_batch_lanes(la, b->lane_grid, b->lane_wpb, s);
   }
   cudaEventRecord(b->ph_ev[1], s);
-  if (b->lanes && b->cont_kernel) {  // phase 2: one warp per parked instance (or all)
-    cudaMemsetAsync(b->d_cont_cursor.p, 0, sizeof(unsigned), s);
-    gk::BatchArgs ca = b->args;
-    ca.cfg = c;
-    ca.cont_fresh = fresh ? 1 : 0;
-    gk::launch_batch_cont(ca, b->cont_m, b->cont_grid, b->cont_wpb, s);
-    cudaEventRecord(b->ph_ev[2], s);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return b->fail(cuda_msg(e, "batch launch"));
-    return GPUKLU_OK;
-  }
   cudaEventRecord(b->start_ev, s);
   for (auto& C : b->classes) {  // largest programs first, all classes concurrent
     cudaStreamWaitEvent(C->stream, b->start_ev, 0);
@@ -3603,7 +3889,7 @@ int gpuklu_batch_info(const gpuklu_batch* b, int64_t* out) {
   if (!b) return GPUKLU_INVALID_MATRIX;
   for (int q = 0; q < 8; ++q) out[q] = 0;
   out[2] = (int64_t)b->groups.size();
-  out[6] = b->lanes && b->cont_kernel ? (b->lane_cap == 0 ? 1 : 2)
+  out[6] = b->lanes && b->cont_kernel ? (int64_t)b->cont.size()
                                        : (int64_t)b->classes.size() + (b->lanes ? 1 : 0);
   out[7] = b->lanes && b->cont_kernel ? 1 : 0;  // the continuation kernel runs
   for (auto& C : b->classes) {  // the largest class (first) describes the launch

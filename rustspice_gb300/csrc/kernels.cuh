@@ -110,6 +110,25 @@ struct GroupHdr {
   // nsteps 0: none): nops operations at ops_off, nsteps + 1 step pointers
   // at step_off; the operations of one step are independent of each other
   int ops_off, nops, step_off, nsteps;
+  // row streams (bt::run_stream), in chunks of kStreamChunk records and
+  // segments: factorization and substitutions, and (transient) the transpose
+  // solve; no chunks: none
+  int stream_off, nchunk, sseg_off, nsseg, tstream_off, ntchunk, tsseg_off, ntsseg;
+  int asm_off;  // n + nslots + noffd assembly records and their destinations
+  // devices to evaluate, sorted by type, capacitors (the last ncap) last:
+  // (device, node 0 | node 1 << 16, node 2 | type << 16, record offset)
+  int ev_off, nev, ncap;
+};
+
+// A row stream: records of operations in chunks, and segments: kind | log2 of
+// the row width << 3, and a count (rows of plain and fused segments, else
+// operations); a segment starts at a multiple of kStreamAlign records.
+constexpr int kStreamChunk = 128, kStreamAlign = 32;
+constexpr int kStreamRing = 4 * kStreamChunk * 8;  // bytes of a warp's ring
+enum { kRowPlain = 0, kRowFused = 1, kRowRcp = 2, kRowSerial = 3, kRowSum = 4 };
+struct RowStream {
+  const int2 *recs, *segs;
+  int nchunk, nseg;
 };
 
 // Contribution codes of the batched stamp: (index << 3) | kind with kind
@@ -134,6 +153,9 @@ struct BatchArgs {
   const int *lvl_col, *lseg_ptr, *lseg;  // level-scheduled factor (see GroupHdr)
   const int *amap4, *rmap4, *lng;        // padded contribution codes (see GroupHdr)
   const int2* ops;                       // step programs (see GroupHdr)
+  const int2 *recs, *segs;               // row streams
+  const int *asm4, *asm_dst;             // assembly records
+  const int4* ev;                        // devices to evaluate
   const int* step_ptr;
   const long long* inst_p_off;  // offset of the instance's circuit constants (4 per device)
   const double* dparams;
@@ -180,11 +202,10 @@ struct BatchArgs {
   const int* cont_groups;      // the groups, most expensive first
   int cont_ngroups;
   unsigned* cont_cursor;       // first entry of cont_groups that may have parked instances
-  double* dv_scratch;          // per instance slot: device records, then the iterate
-  long long dv_stride;         //   at dv_x (dv_stride doubles per slot)
+  double* dv_scratch;          // per instance slot: device records, then the iterate and
+  long long dv_stride;         //   its differences at dv_x (dv_stride doubles per slot)
   long long dv_x;
-  int slice;                   // shared doubles per instance slot: T and the LU values
-  int cont_fresh;              // 1: no lane phase ran, the continuation starts every instance
+  int slice;                   // shared doubles per instance slot: T, the LU values, two constants
 };
 
 // Batched adaptive transient (atran.cu): per instance its time-dependent
@@ -308,9 +329,11 @@ void launch_batch_newton(const BatchArgs& a, int m, int grid, int warps_per_bloc
                          cudaStream_t s, bool shared = false);
 // Registers per thread and resident blocks per SM of the batched kernel.
 // Lane-per-instance batched Newton (phase 1 of gpuklu_batch_run).
-void launch_batch_cont(const BatchArgs& a, int m, int grid, int warps_per_block,
-                       cudaStream_t s);
-void cont_kernel_info(int m, int warps_per_block, int slice, int* regs, int* blocks_per_sm);
+// Continuation kernel: one warp per block, m instances per warp; kContWarps
+// blocks fit an SM's registers.
+constexpr int kContWarps = 12;
+void launch_batch_cont(const BatchArgs& a, int m, int grid, cudaStream_t s);
+void cont_kernel_info(int m, int slice, int* regs, int* blocks_per_sm);
 void launch_batch_lanes(const BatchArgs& a, int grid, int warps_per_block, cudaStream_t s);
 void lanes_kernel_info(int warps_per_block, int* regs, int* blocks_per_sm);
 

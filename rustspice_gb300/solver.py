@@ -405,8 +405,9 @@ class Batch:
 
     def phase_ms(self) -> dict:
         """Device time of the last run by kernel (CUDA events; waits for the
-        run): the lane-per-instance kernel, the warp kernels after it, and
-        the lane kernel's iteration cap."""
+        run): the lane-per-instance kernel (only the run's resets when
+        ``info()["cont_kernel"]``), the warp kernels, and the iterations with
+        the lane kernel's order of additions."""
         out = np.zeros(3)
         st = N.lib().gpuklu_batch_phase_ms(self._h, N.ptr(out))
         if st != N.OK:
