@@ -588,6 +588,7 @@ struct PlanDev {
     gk::DPlan d{};
     if (e == cudaSuccess) e = ss.upload(sp, s, d.ss);
     d.n = p.n;
+    for (int k = 0; k < p.n; ++k) d.max_col = std::max<int>(d.max_col, p.col_ptr[k + 1] - p.col_ptr[k]);
     d.noffd = p.offd_ptr.empty() ? 0 : p.offd_ptr.back();
     d.cs_nchunk = (int)(hc.size() / 4);
     d.cs_chunk = cs_chunk.p;
@@ -882,20 +883,23 @@ struct gpuklu_handle {
   cudaStream_t stream = nullptr;
   DBuf<double> d_ax, d_lu, d_z, d_x, d_out, d_rhs, d_work, d_rc, d_rhs_c, d_xnew, d_newx,
       d_scratch2;
-  DBuf<unsigned> d_flags, d_zflag, d_xflag, d_counter;
+  DBuf<unsigned> d_zflag, d_xflag, d_counter;
+  DBuf<double> d_big;  // columns too long for shared memory while they are updated
   DBuf<int> d_rperm, d_rinv, d_status;
   DBuf<gk::NewtonState> d_nstate;
-  unsigned epoch = 0, sepoch = 0;
+  unsigned sepoch = 0;
   int64_t factor_count = 0, refactor_count = 0;
   bool cta_ref = false, cta_sol = false;  // one-block refactor / solve for this plan
   bool cta_grp = false;  // the one-block solve over groups of uncoupled BTF blocks
   bool steps_sol = false;  // the solve as a step program (k_solve_steps)
   DBuf<double> d_rec;      // its scratch: the pivots' reciprocals
-  // Plans with up to this many multiply-subtract pairs refactor in one block.
-  // FP64 issue on one SM (a warp instruction per 16 cycles) bounds that
-  // kernel: the 32x32 diode mesh (273k pairs) already refactors faster over
-  // the whole grid, despite the grid kernel's dependency hops through L2.
-  static constexpr int64_t kOneBlockUpdates = 1 << 16;
+  // Plans with up to this many multiply-subtract pairs refactor in one block:
+  // its hops through shared memory are shorter than the grid kernel's through
+  // L2, its one SM's FP64 and instruction issue are the limit beyond. Measured,
+  // one block against grid, us: meshes of 16 nodes (176 pairs) 11.3 / 12.4, 36
+  // (676) 17.9 / 23.4, 64 (1778) 29.7 / 27.5, 144 (8470) 72.6 / 42.3; chains of
+  // 32 stages (287) 31.4 / 40.3, 64 (575) 76.0 / 66.5, 256 (2303) 346 / 255.
+  static constexpr int64_t kOneBlockUpdates = 512;
   // The first factorization's pivot pass on the refactorization kernels:
   // buffers, the pass limit before the sequential kernel takes over, and the
   // passes the last first factorization ran (0: the sequential kernel).
@@ -962,7 +966,8 @@ struct gpuklu_handle {
   int upload_plan() {
     cudaError_t e = pd.upload(plan, stream, true);
     apply_spin_limit();
-    if (e == cudaSuccess) e = d_lu.resize(std::max(plan.nslots(), 1));
+    if (e == cudaSuccess) e = d_lu.resize((size_t)plan.nslots() + gk::kLuPad);
+    if (e == cudaSuccess && gk::refactor_needs_big(pd.dp)) e = d_big.resize(plan.nslots());
     if (e != cudaSuccess) return cuda_fail(e, "upload plan");
     // one-block refactor and solve for small factorizations (GPUKLU_ONE_BLOCK=0: off)
     const char* ob = getenv("GPUKLU_ONE_BLOCK");
@@ -1014,12 +1019,13 @@ struct gpuklu_handle {
       if (e != cudaSuccess) return cuda_fail(e, "upload plan");
       pd_sym_ok = true;
     }
-    e = d_lu.resize(std::max(sym_plan.nslots(), 1));
+    e = d_lu.resize((size_t)sym_plan.nslots() + gk::kLuPad);
+    if (e == cudaSuccess && gk::refactor_needs_big(pd_sym.dp)) e = d_big.resize(sym_plan.nslots());
     size_t nn = (size_t)std::max<int64_t>(n, 1);
     if (e == cudaSuccess) e = d_ax.resize(std::max<int64_t>(ai_len, 1));
     for (auto* b : {&d_z, &d_x, &d_out, &d_rhs, &d_work, &d_xnew, &d_newx})
       if (e == cudaSuccess) e = b->resize(nn);
-    for (auto* b : {&d_flags, &d_zflag, &d_xflag})
+    for (auto* b : {&d_zflag, &d_xflag})
       if (e == cudaSuccess) e = b->resize(nn);
     if (e == cudaSuccess) e = d_counter.resize(1);
     if (e == cudaSuccess) e = d_rperm.resize(nn);
@@ -1028,13 +1034,12 @@ struct gpuklu_handle {
     if (e == cudaSuccess) e = d_rc.resize(2);
     if (e == cudaSuccess) e = d_nstate.resize(1);
     if (e == cudaSuccess) {
-      cudaMemsetAsync(d_flags.p, 0, nn * sizeof(unsigned), stream);
       cudaMemsetAsync(d_zflag.p, 0, nn * sizeof(unsigned), stream);
       cudaMemsetAsync(d_xflag.p, 0, nn * sizeof(unsigned), stream);
       e = cudaMemsetAsync(d_status.p, 0, sizeof(int), stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "analyze buffers");
-    epoch = sepoch = 0;
+    sepoch = 0;
     grid_cols = std::max(1, std::min<int>((int)((n + 3) / 4), sm_count() * 16));
     state = ANALYZED;
     return GPUKLU_OK;
@@ -1052,23 +1057,13 @@ struct gpuklu_handle {
     return GPUKLU_OK;
   }
 
-  unsigned next_epoch(unsigned& ep, DBuf<unsigned>& f) {
-    if (++ep == 0) {  // wrapped: clear the flags
-      cudaMemsetAsync(f.p, 0, f.n * sizeof(unsigned), stream);
-      ep = 1;
-    }
-    return ep;
-  }
-
   // Factor with the values already in d_ax.
   void refactor_launch() {
     if (cta_ref) {
       gk::launch_refactor_cta(pd.dp, d_ax.p, d_lu.p, d_status.p, stream);
       return;
     }
-    unsigned ep = next_epoch(epoch, d_flags);
-    gk::launch_refactor(pd.dp, d_ax.p, d_lu.p, d_flags.p, ep, d_counter.p, d_status.p,
-                        grid_cols, stream);
+    gk::launch_refactor(pd.dp, d_ax.p, d_lu.p, d_big.p, d_status.p, grid_cols, stream);
   }
 
   // The first factorization's pivot pass run as refactorizations of the
@@ -1121,9 +1116,7 @@ struct gpuklu_handle {
       if (one_block) {
         gk::launch_refactor_cta(dp, d_ax.p, d_lu.p, d_status.p, stream, pc);
       } else {
-        unsigned ep = next_epoch(epoch, d_flags);
-        gk::launch_refactor(dp, d_ax.p, d_lu.p, d_flags.p, ep, d_counter.p, d_status.p,
-                            grid_cols, stream, pc);
+        gk::launch_refactor(dp, d_ax.p, d_lu.p, d_big.p, d_status.p, grid_cols, stream, pc);
       }
       e = cudaMemcpyAsync(want.data(), d_want.p, nn * sizeof(int), cudaMemcpyDeviceToHost,
                           stream);

@@ -12,11 +12,11 @@
 //                    does not settle.
 //  * refactor      - left-looking refactorization with frozen pivots. Warps
 //                    take columns in increasing order from an atomic counter
-//                    and wait on per-column completion flags of exactly the
-//                    columns they depend on (the U pattern), so independent
-//                    columns run concurrently without level barriers; a
-//                    warp's column sits in shared memory while it is updated.
-//                    k_refactor_cta is the same in one block, for small plans.
+//                    and wait for exactly the columns they depend on (the U
+//                    pattern), so independent columns run concurrently
+//                    without level barriers; a warp's column sits in shared
+//                    memory while it is updated. k_refactor_cta is the same
+//                    in one block, for small plans.
 //  * solve         - the forward (L) and backward (U) substitutions and the
 //                    BTF block coupling. k_solve_cta sweeps the columns in one
 //                    block (solution vector in shared memory); k_solve runs
@@ -338,13 +338,279 @@ __global__ void k_first_factor_s(DPlan P, const double* __restrict__ ax, double*
 }
 
 // --------------------------------------------------------------- refactor
-// A warp's column lives in shared memory while it is updated (columns of up
-// to kColBuf slots; longer ones stay in memory). The U entries are taken in
-// chunks of 32: one acquire per entry, all lanes at once, finds the columns
-// already final; those need no further wait, and the L column of the next
-// entry (its first 32 values and destinations) is loaded while the current
-// one is applied. The operations and their order are the reference's.
-constexpr int kColBuf = 768;
+// The updates of a column: for its U entries s in order, of columns j, the
+// slots upd_dst of the column lose u * l(q) for every L slot q of column j.
+// The values and the destinations reach the warp through a ring of
+// asynchronous copies, cut into pieces of up to 64 slots that start on an even
+// slot (16 bytes); a piece's header {s, first slot, rows lo, hi and offset of
+// the destinations, column} lies before them. The entries' ranges are read 32
+// at a time, one per lane, two groups ahead. The operations and their order
+// are the reference's.
+constexpr int kPiece = 64;
+constexpr int kDstBytes = 288;  // 64 destinations behind up to 3 others
+constexpr int kGridRing = 8;    // pieces in flight per column
+constexpr int kGridStage = 16 + kDstBytes + 8 * kPiece;
+constexpr int kCtaRing = 4;
+constexpr int kCtaStage = 16 + kDstBytes;  // the values are in shared memory
+constexpr int kColCap = 4096;   // slots of a column kept in shared memory
+
+// The grid kernel has no completion flags: every value of lu is preset to
+// kUnset (all bits one, a NaN; a computed value with these bits is stored as
+// another NaN) and a reader that finds it polls the value itself. One trip
+// through L2 per dependency instead of three (fence, flag, value).
+__device__ __forceinline__ bool unset(double v) { return __double_as_longlong(v) == -1ll; }
+__device__ __forceinline__ double ld_relaxed(const double* p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_set(double* p, double v) {
+  if (unset(v)) v = __longlong_as_double(0x7fffffffffffffffll);
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire_cta(const unsigned* p) {
+  unsigned v;
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_cta(unsigned* p, unsigned v) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// 16 bytes to shared memory, the first n of them from memory, the rest zero.
+__device__ __forceinline__ void cp_async16(void* d, const void* g, int n) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(d);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(g), "r"(n) : "memory");
+}
+
+// The pieces of a column's updates in order, handed out one at a time (by all
+// lanes alike): entries [s0, ds), those without L slots left out.
+struct Pieces {
+  const DPlan& P;
+  int ds, sc, part;
+  int j0, j1, j2, qa, qb, up, nqa, nqb, nup;  // this lane's entry of the group and of the next
+  unsigned mask;                              // entries of the group not yet handed out
+  __device__ __forceinline__ int row_of(int s) const { return s < ds ? P.slot_row[s] : -1; }
+  __device__ __forceinline__ void range_of(int s, int j, int& a, int& b, int& u) const {
+    a = b = u = 0;
+    if (j >= 0) {
+      a = P.dslot[j] + 1;
+      b = P.col_ptr[j + 1];
+      u = P.upd_ptr[s];
+    }
+  }
+  __device__ __forceinline__ Pieces(const DPlan& P_, int s0, int ds_)
+      : P(P_), ds(ds_), sc(s0), part(0) {
+    const int lane = threadIdx.x & 31;
+    j0 = row_of(s0 + lane);
+    j1 = row_of(s0 + 32 + lane);
+    j2 = row_of(s0 + 64 + lane);
+    range_of(s0 + lane, j0, qa, qb, up);
+    range_of(s0 + 32 + lane, j1, nqa, nqb, nup);
+    mask = __ballot_sync(FULL, qb > qa);
+    skip_empty();
+  }
+  __device__ __forceinline__ void skip_empty() {
+    const int lane = threadIdx.x & 31;
+    while (mask == 0 && sc + 32 < ds) {
+      sc += 32;
+      j0 = j1;
+      qa = nqa;
+      qb = nqb;
+      up = nup;
+      j1 = j2;
+      range_of(sc + 32 + lane, j1, nqa, nqb, nup);
+      j2 = row_of(sc + 64 + lane);
+      mask = __ballot_sync(FULL, qb > qa);
+    }
+  }
+  __device__ __forceinline__ bool more() const { return mask != 0; }
+  // Starts the copies of the next piece into stage st (the values only when
+  // there is a lu in memory) and returns its header.
+  __device__ __forceinline__ int4 next(unsigned char* st, const double* lu) {
+    const int lane = threadIdx.x & 31;
+    const int i = __ffs(mask) - 1;
+    const int a = __shfl_sync(FULL, qa, i), b = __shfl_sync(FULL, qb, i);
+    const int u = __shfl_sync(FULL, up, i), j = __shfl_sync(FULL, j0, i);
+    const int base = (a & ~1) + kPiece * part;
+    const int lo = max(a - base, 0), hi = min(b - base, kPiece);
+    const int d0 = u + base + lo - a, da = d0 & ~3, dend = u + base + hi - a;
+    if (da + 4 * lane < dend)
+      cp_async16(st + 16 + 16 * lane, P.upd_dst + da + 4 * lane,
+                 min(16, 4 * (dend - da) - 16 * lane));
+    if (lu != nullptr && 2 * lane < hi)  // lu is padded by a value
+      cp_async16(st + 16 + kDstBytes + 16 * lane, lu + base + 2 * lane, 16);
+    const int4 h = make_int4(sc + i, base, lo | hi << 8 | ((d0 & 3) - lo + 128) << 16, j);
+    if (base + kPiece >= b) {
+      mask &= mask - 1;
+      part = 0;
+    } else {
+      ++part;
+    }
+    return h;
+  }
+};
+
+// One piece as a warp holds it: a0, a1 this lane's rows, their destinations
+// and values.
+struct Piece {
+  int4 h;
+  int e0, e1;
+  bool a0, a1, two;
+  double v0, v1;
+  __device__ __forceinline__ void read(const unsigned char* st, bool values) {
+    const int lane = threadIdx.x & 31;
+    h = *reinterpret_cast<const int4*>(st);
+    const int lo = h.z & 255, hi = (h.z >> 8) & 255;
+    const int* const dst = reinterpret_cast<const int*>(st + 16) + (((h.z >> 16) & 255) - 128);
+    a0 = lane >= lo && lane < hi;  // lo is 0 or 1
+    a1 = lane + 32 < hi;
+    two = hi > 32;
+    e0 = a0 ? dst[lane] : 0;
+    e1 = a1 ? dst[lane + 32] : 0;
+    if (values) {
+      const double* const val = reinterpret_cast<const double*>(st + 16 + kDstBytes);
+      v0 = a0 ? val[lane] : 0.0;
+      v1 = a1 ? val[lane + 32] : 0.0;
+    }
+  }
+};
+
+// The updates of the column in slots [s0, ds) of a factor in shared memory
+// (indexed by slot), completion flags in `done`, by one warp that copies its
+// own pieces. Returns false when a wait gave up.
+__device__ __forceinline__ bool block_updates(const DPlan& P, int s0, int ds, double* lu,
+                                              const unsigned* done, unsigned char* ring,
+                                              int* status) {
+  const int lane = threadIdx.x & 31;
+  Pieces todo(P, s0, ds);
+  int live = 0, head = 0, tail = 0;
+  auto issue = [&]() {
+    if (todo.more()) {
+      unsigned char* const st = ring + tail * kCtaStage;
+      const int4 h = todo.next(st, nullptr);
+      if (lane == 0) *reinterpret_cast<int4*>(st) = h;
+      todo.skip_empty();
+      tail = tail + 1 == kCtaRing ? 0 : tail + 1;
+      ++live;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < kCtaRing; ++i) issue();
+  Piece nx;
+  auto read = [&]() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kCtaRing - 1) : "memory");  // the oldest has landed
+    __syncwarp();
+    nx.read(ring + head * kCtaStage, false);
+  };
+  bool ok = true;
+  if (live > 0) read();
+  while (live > 0) {
+    const Piece p = nx;
+    const double u = lu[p.h.x];
+    double c0 = 0.0, c1 = 0.0;
+    if (p.a0) c0 = lu[p.e0];
+    if (p.two && p.a1) c1 = lu[p.e1];
+    __syncwarp();  // the piece is read by all lanes: the next one takes its stage
+    head = head + 1 == kCtaRing ? 0 : head + 1;
+    --live;
+    issue();
+    if (live > 0) read();
+    unsigned spins = 0;
+    while (!__all_sync(FULL, ld_acquire_cta(&done[p.h.w]) != 0u)) {
+      ++spins;
+      bool stop = spins > P.spin_limit;
+      if (stop && lane == 0) atomicCAS(status, DS_OK, DS_TIMEOUT);
+      if ((spins & 1023u) == 0 && *(volatile int*)status != DS_OK) stop = true;
+      if (__any_sync(FULL, stop)) {
+        ok = false;
+        break;
+      }
+      if (spins > 256) __nanosleep(20);  // shared-memory polls first
+    }
+    if (!ok) break;
+    if (bt::nonzero(u)) {  // the same in every lane
+      if (p.a0) lu[p.e0] = sub(c0, mul(lu[p.h.y + lane], u));
+      if (p.two && p.a1) lu[p.e1] = sub(c1, mul(lu[p.h.y + lane + 32], u));
+    }
+    __syncwarp();
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+  return ok;
+}
+
+// The L values of a column: C[q] / diag for q in (ds, s1), correctly rounded,
+// handed to put(q, value). Division by an invariant integer (Granlund and
+// Montgomery, PLDI 1994) on the significands: FP64 takes about ten operations
+// of 64 cycles a division (620 cycles for 32 rows, one after another), the
+// integer unit two products once the reciprocal stands.
+//   w   2^116 / mb less at most 32, mb the divisor's significand in
+//       [2^52, 2^53): a 24-bit reciprocal and two Newton steps in fixed point
+//   q   floor(2^57 ma / mb), first as the high word of (ma << 5) w, then with
+//       the remainder's correction; rounded to 53 bits, ties to even
+// Zeros keep their sign; operands far from 1 and the non-finite are divided.
+__device__ __forceinline__ unsigned long long significand(double v) {
+  return ((unsigned long long)__double_as_longlong(v) & 0xfffffffffffffull) | (1ull << 52);
+}
+__device__ __forceinline__ int exponent(double v) {
+  return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu);
+}
+__device__ __forceinline__ unsigned long long fixed_reciprocal(unsigned long long mb) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;"
+      : "=f"(r)
+      : "f"(__uint_as_float(0x3f800000u | (unsigned)(mb >> 29 & 0x7fffffu))));
+  const unsigned long long x0 = __float2uint_rz(r * 4294967296.0f);  // saturates below 1
+  const long long e1 = (long long)(0x8000000000000000ull - __umul64hi(mb << 11, x0 << 32));
+  const unsigned long long x1 =
+      (x0 << 32) + (unsigned long long)(((long long)x0 * (e1 >> 12)) >> 19);
+  const long long e2 = (long long)(0x8000000000000000ull - __umul64hi(mb << 11, x1));
+  return x1 + (unsigned long long)(((long long)(x1 >> 32) * e2) >> 31) - 16;
+}
+__device__ __forceinline__ double fixed_divide(double a, double b, unsigned long long mb,
+                                               unsigned long long w) {
+  const unsigned long long ma = significand(a);
+  int e = exponent(a) - exponent(b);
+  unsigned long long q = __umul64hi(ma << 5, w);
+  unsigned long long r = (ma << 57) - q * mb;
+  if (r >= mb) {
+    q += 1;
+    r -= mb;
+  }
+  if (q < (1ull << 57)) {
+    q <<= 1;
+    e -= 1;
+  }
+  const unsigned long long t = q | (r != 0 ? 1ull : 0ull);
+  const unsigned long long m = (t + 15 + (t >> 5 & 1)) >> 5;
+  const unsigned long long sign =
+      (unsigned long long)(__double_as_longlong(a) ^ __double_as_longlong(b)) & (1ull << 63);
+  return __longlong_as_double(
+      (long long)(sign | (((unsigned long long)(e + 1022) << 52) + m)));
+}
+template <class Get, class Put>
+__device__ __forceinline__ void scale_column(int ds, int s1, double diag, Get get, Put put) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long mb = significand(diag), w = fixed_reciprocal(mb);
+  const bool inside = (unsigned)(exponent(diag) - (1023 - 400)) <= 800u;
+  for (int q = ds + 1 + lane; q - lane < s1; q += 32) {
+    const double a = q < s1 ? get(q) : 1.0;
+    const bool zero = !bt::nonzero(a);
+    const bool fast = inside && (zero || (unsigned)(exponent(a) - (1023 - 500)) <= 1000u);
+    double v;
+    if (__all_sync(FULL, fast)) {
+      v = fixed_divide(a, diag, mb, w);
+      if (zero)
+        v = __longlong_as_double((__double_as_longlong(a) ^ __double_as_longlong(diag)) &
+                                 (long long)(1ull << 63));
+    } else {
+      v = a / diag;
+    }
+    if (q < s1) put(q, v);
+  }
+}
 
 // Pivot-pass mode of the refactorization (PivotCheck): the first
 // factorization's threshold rule on column k's finished values - the first L
@@ -387,21 +653,210 @@ __device__ __forceinline__ void pivot_check(const PivotCheck& pc, int k, int ds,
   __syncwarp();
 }
 
-__global__ void k_refactor(DPlan P, const double* __restrict__ ax, double* lu,
-                           unsigned* flags, unsigned epoch, unsigned* counter,
-                           int* status, PivotCheck pc) {
-  extern __shared__ double scol[];
+// The grid kernel: a pair of warps per column. The loader takes the columns in
+// order and copies their pieces; the computing warp holds the column in shared
+// memory (in `big` when it is longer than colcap) and does nothing but the
+// arithmetic, so a piece costs it about 30 instructions and the latency of a
+// multiply, a subtract and two trips to shared memory. Stage protocol: `full`
+// counts the loader's 32 copy completions and its header, `empty` the computing
+// warp; a stage marked last is released when its column is stored, and only
+// then the loader takes another column, so the lowest unfinished column is
+// always at work. The column counter lies behind the values, so one fill
+// presets both: it starts at the largest unsigned. A wait that gives up ends the
+// pair (`dead`) and sets the status, which ends the others.
+//
+// What bounds it: the chain of dependent columns, about 1 us a column (the last
+// update 350 cycles, the reciprocal and the first 32 quotients 820, store to
+// load through L2 900), and for the hub columns 800 cycles a piece. Measured
+// against one warp per column, flags, one entry's loads ahead and FP64
+// compares and divisions: 32 x 32 mesh (n 1026, 25 k slots) 353 -> 178 us,
+// 48 x 48 740 -> 353 us, 120 x 120 with 1000 inverters (n 15,403, 670 k slots)
+// 4.2 -> 1.6 ms.
+constexpr int kStart = -1, kEnd = -2, kNone = -3;  // header.z of a stage that is no piece
+constexpr int kLast = 1 << 24;  // in a piece's header.z
+constexpr int kPairs = 4;       // per block
+
+__device__ __forceinline__ void bar_init(unsigned b, int n) {
+  asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(b), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned b) {
+  asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(b) : "memory");
+}
+__device__ __forceinline__ void bar_arrive_copies(unsigned b) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(b) : "memory");
+}
+// Waits for the end of a barrier's phase; false when the pair has given up.
+__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile int* dead) {
+  for (unsigned spins = 0;; ++spins) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(b), "r"(parity)
+        : "memory");
+    if (__all_sync(FULL, done)) return true;
+    if (__any_sync(FULL, *dead != 0 || spins > 8 * kSpinLimit)) return false;
+    if (spins > 256) __nanosleep(100);
+  }
+}
+
+struct Stages {
+  unsigned char* ring;
+  unsigned bars;  // full[kGridRing], then empty[kGridRing]
+  int st = 0;
+  unsigned ph = 0;
+  __device__ __forceinline__ unsigned char* at() const { return ring + st * kGridStage; }
+  __device__ __forceinline__ unsigned full() const { return bars + 8 * st; }
+  __device__ __forceinline__ unsigned empty() const { return bars + 8 * (kGridRing + st); }
+  __device__ __forceinline__ void advance() {
+    if (++st == kGridRing) {
+      st = 0;
+      ph ^= 1u;
+    }
+  }
+};
+
+__device__ __forceinline__ void load_columns(const DPlan& P, const double* lu, unsigned* counter,
+                                             Stages S, volatile int* dead) {
   const int lane = threadIdx.x & 31;
-  double* const cbuf = scol + (threadIdx.x >> 5) * kColBuf;
-  const int n = P.n;
+  auto publish = [&](int4 h) {  // after the stage's copies
+    if (lane == 0) *reinterpret_cast<int4*>(S.at()) = h;
+    bar_arrive_copies(S.full());
+    if (lane == 0) bar_arrive(S.full());
+  };
   while (true) {
     int k = 0;
-    if (lane == 0) k = (int)atomicAdd(counter, 1u);
+    if (lane == 0) k = (int)(atomicAdd(counter, 1u) + 1u);
     k = __shfl_sync(FULL, k, 0);
-    if (k >= n) return;
+    if (!bar_wait(S.empty(), S.ph ^ 1u, dead)) return;
+    if (k >= P.n) {
+      publish(make_int4(0, 0, kEnd, 0));
+      return;
+    }
     const int s0 = P.col_ptr[k], ds = P.dslot[k], s1 = P.col_ptr[k + 1];
-    const bool staged = s1 - s0 <= kColBuf;
-    double* const C = staged ? cbuf - s0 : lu;  // the column, indexed by slot
+    const int single = P.col_single[k];
+    if (lane == 0) *reinterpret_cast<int4*>(S.at() + 16) = make_int4(s1, single, 0, 0);
+    publish(make_int4(s0, ds, kStart, k));
+    S.advance();
+    Pieces todo(P, s0, ds);
+    bool more = todo.more();
+    do {
+      if (!bar_wait(S.empty(), S.ph ^ 1u, dead)) return;
+      int4 h = make_int4(0, 0, kNone, 0);
+      if (more) {
+        h = todo.next(S.at(), lu);
+        todo.skip_empty();
+        more = todo.more();
+        if (!more) h.z |= kLast;
+      }
+      publish(h);
+      if (!more && !bar_wait(S.empty(), S.ph, dead)) return;
+      S.advance();
+    } while (more);
+  }
+}
+
+// The computing warp's updates of one column; S stands at its first piece.
+// Leaves S at the column's last stage, not yet released.
+template <bool kStaged>
+__device__ __forceinline__ bool grid_updates(const DPlan& P, double* C, const double* lu,
+                                             Stages& S, int* status, volatile int* dead) {
+  const int lane = threadIdx.x & 31;
+  auto at = [&](int s) { return kStaged ? C[s] : ld_cg(&C[s]); };
+  Piece nx;
+  auto read = [&]() {
+    if (!bar_wait(S.full(), S.ph, dead)) return false;
+    nx.read(S.at(), true);
+    __syncwarp();
+    if ((nx.h.z & kLast) == 0) {
+      if (lane == 0) bar_arrive(S.empty());
+      S.advance();
+    }
+    return true;
+  };
+  if (!read()) return false;
+  if (nx.h.z < 0) return true;  // no updates
+  while (true) {
+    // all that does not depend on the values comes before the wait for them
+    const Piece p = nx;
+    const bool last = (p.h.z & kLast) != 0;
+    double x0 = p.v0, x1 = p.v1;
+    const double u = at(p.h.x);
+    double c0 = 0.0, c1 = 0.0;
+    if (p.a0) c0 = at(p.e0);
+    if (p.two && p.a1) c1 = at(p.e1);
+    if (!last && !read()) return false;
+    bool w0 = p.a0 && unset(x0), w1 = p.a1 && unset(x1);
+    unsigned spins = 0;
+    while (__any_sync(FULL, w0 || w1)) {
+      if (w0) {
+        x0 = ld_relaxed(lu + p.h.y + lane);
+        w0 = unset(x0);
+      }
+      if (w1) {
+        x1 = ld_relaxed(lu + p.h.y + lane + 32);
+        w1 = unset(x1);
+      }
+      ++spins;
+      bool stop = spins > P.spin_limit && (w0 || w1);
+      if (stop) atomicCAS(status, DS_OK, DS_TIMEOUT);
+      if ((spins & 63u) == 0 && *(volatile int*)status != DS_OK) stop = true;
+      if (__any_sync(FULL, stop)) return false;
+      if (spins > 64) __nanosleep(64);  // a poll is a trip through L2
+    }
+    if (bt::nonzero(u)) {  // the same in every lane
+      const double m0 = mul(x0, u);
+      if (p.a0) C[p.e0] = sub(c0, m0);
+      if (p.two) {
+        const double m1 = mul(x1, u);
+        if (p.a1) C[p.e1] = sub(c1, m1);
+      }
+    }
+    __syncwarp();
+    if (last) return true;
+  }
+}
+
+__global__ void __launch_bounds__(64 * kPairs) k_refactor(DPlan P, const double* __restrict__ ax,
+                                                          double* lu, double* big, int colcap,
+                                                          int* status, PivotCheck pc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long bars[kPairs][2 * kGridRing];
+  __shared__ int dead_flag[kPairs];
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % kPairs;
+  const bool loader = (threadIdx.x >> 5) >= kPairs;
+  volatile int* const dead = &dead_flag[w];
+  double* const cbuf =
+      reinterpret_cast<double*>(smem_raw + kPairs * kGridRing * kGridStage) + w * colcap;
+  Stages S;
+  S.ring = smem_raw + w * (kGridRing * kGridStage);
+  S.bars = (unsigned)__cvta_generic_to_shared(&bars[w][0]);
+  if (!loader && lane == 0) {
+    for (int i = 0; i < kGridRing; ++i) {
+      bar_init(S.bars + 8 * i, 33);
+      bar_init(S.bars + 8 * (kGridRing + i), 1);
+    }
+    *dead = 0;
+  }
+  __syncthreads();
+  if (loader) {
+    load_columns(P, lu, reinterpret_cast<unsigned*>(lu + P.nslots + 2), S, dead);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  while (true) {
+    if (!bar_wait(S.full(), S.ph, dead)) return;
+    const int4 h = *reinterpret_cast<const int4*>(S.at());
+    if (h.z == kEnd) return;
+    const int4 h1 = *reinterpret_cast<const int4*>(S.at() + 16);
+    const int s0 = h.x, ds = h.y, k = h.w, s1 = h1.x;
+    const bool staged = s1 - s0 <= colcap, single = h1.y != 0;
+    double* const C = staged ? cbuf - s0 : big;  // the column, indexed by slot
+    __syncwarp();
+    if (lane == 0) bar_arrive(S.empty());
+    S.advance();
     // A(:,k) into the column's slots; duplicates summed in CSC order
     for (int s = s0 + lane; s < s1; s += 32) {
       double v = 0.0;
@@ -409,81 +864,27 @@ __global__ void k_refactor(DPlan P, const double* __restrict__ ax, double* lu,
       C[s] = v;
     }
     __syncwarp();
-    for (int sc = s0; sc < ds; sc += 32) {
-      const int cnt = min(32, ds - sc);
-      int jl = 0;
-      bool rdy = true;
-      if (lane < cnt) {
-        jl = P.slot_row[sc + lane];
-        rdy = ld_acquire(&flags[jl]) == epoch;
+    if (!(staged ? grid_updates<true>(P, cbuf - s0, lu, S, status, dead)
+                 : grid_updates<false>(P, big, lu, S, status, dead))) {
+      if (lane == 0) {
+        *dead = 1;
+        atomicCAS(status, DS_OK, DS_TIMEOUT);
       }
-      const unsigned ready = __ballot_sync(FULL, rdy);
-      __syncwarp();  // orders every lane's later loads after the acquires
-      int j = 0, qa = 0, qb = 0, d0 = 0;
-      const int* dst = nullptr;
-      double v0 = 0.0;
-      auto fetch = [&](int i) {
-        j = __shfl_sync(FULL, jl, i);
-        qa = P.dslot[j] + 1;
-        qb = P.col_ptr[j + 1];
-        dst = P.upd_dst + P.upd_ptr[sc + i] - qa;
-        v0 = 0.0;
-        d0 = 0;
-        const int q = qa + lane;
-        if (q < qb && ((ready >> i) & 1u)) {
-          v0 = ld_cg(&lu[q]);
-          d0 = dst[q];
-        }
-      };
-      fetch(0);
-      for (int i = 0; i < cnt; ++i) {
-        const int s = sc + i, cqa = qa, cqb = qb;
-        const int* const cdst = dst;
-        int cd0 = d0;
-        double cv0 = v0;
-        const int cj = j;
-        if (i + 1 < cnt) fetch(i + 1);  // independent of this entry's update
-        if (!((ready >> i) & 1u)) {
-          int ok = 1;
-          if (lane == 0) ok = wait_flag(&flags[cj], epoch, status, P.spin_limit);
-          if (!__shfl_sync(FULL, ok, 0)) return;
-          __syncwarp();
-          const int q = cqa + lane;
-          if (q < cqb) {
-            cv0 = ld_cg(&lu[q]);
-            cd0 = cdst[q];
-          }
-        }
-        const double u = staged ? C[s] : ld_cg(&lu[s]);
-        if (u != 0.0) {
-          int q = cqa + lane;
-          if (q < cqb) {
-            const double c = staged ? C[cd0] : ld_cg(&lu[cd0]);
-            C[cd0] = c - cv0 * u;
-          }
-          for (q += 32; q < cqb; q += 32) {
-            const int d = cdst[q];
-            const double c = staged ? C[d] : ld_cg(&lu[d]);
-            C[d] = c - ld_cg(&lu[q]) * u;
-          }
-        }
-        __syncwarp();
-      }
+      return;
     }
     if (pc.want != nullptr)
       pivot_check(
-          pc, k, ds, s1, P.col_single[k] != 0,
-          [&](int q) { return staged ? C[q] : ld_cg(&lu[q]); },
+          pc, k, ds, s1, single, [&](int q) { return staged ? C[q] : ld_cg(&C[q]); },
           [&](int q, double v) { C[q] = v; });
-    const double diag = perturb(staged ? C[ds] : ld_cg(&lu[ds]), P.col_single[k] != 0);
-    for (int q = ds + 1 + lane; q < s1; q += 32)
-      lu[q] = (staged ? C[q] : ld_cg(&lu[q])) / diag;
-    if (staged)
-      for (int q = s0 + lane; q < ds; q += 32) lu[q] = C[q];
+    const double diag = bt::perturb_bits(staged ? C[ds] : ld_cg(&C[ds]), single);
+    scale_column(
+        ds, s1, diag, [&](int q) { return staged ? C[q] : ld_cg(&C[q]); },
+        [&](int q, double v) { st_set(&lu[q], v); });
+    for (int q = s0 + lane; q < ds; q += 32) lu[q] = staged ? C[q] : ld_cg(&C[q]);
     if (lane == 0) lu[ds] = diag;
     __syncwarp();
-    __threadfence();
-    if (lane == 0) st_release(&flags[k], epoch);
+    if (lane == 0) bar_arrive(S.empty());
+    S.advance();
   }
 }
 
@@ -618,115 +1019,51 @@ __global__ void k_tsolve(DPlan P, const double* __restrict__ g, const double* __
 // the solve run in one thread block, where a hop is a shared-memory flag (or
 // a warp barrier) instead of a round trip through L2.
 
-__device__ __forceinline__ unsigned ld_acquire_cta(const unsigned* p) {
-  unsigned v;
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_cta(unsigned* p, unsigned v) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-
 // k_refactor in one block, with the factor itself in shared memory: the
-// column code is k_refactor's (same operations, same order); the completion
-// flags also live in shared memory, so a warp waiting for a column sees it
-// finish within a few hundred cycles. The static metadata of the U entries is
-// fetched in a pipeline - the row two entries ahead, the L range and update
-// list one entry ahead, the first update destinations before the wait - so a
-// step costs shared-memory latency only. All warps of the block are resident
-// and a warp only waits for columns handed out before its own, so the warp
-// holding the lowest unfinished column always proceeds. Shared: lu[nslots]
-// f64, done[n] u32.
+// column code is k_refactor's (same operations, same order); completion flags
+// live in shared memory, so a warp waiting for a column sees it finish within
+// a few hundred cycles. All warps of the block are resident and a warp only
+// waits for columns handed out before its own, so the warp holding the lowest
+// unfinished column always proceeds. Shared: lu[nslots] f64, the warps' rings,
+// done[n] u32.
 __global__ void __launch_bounds__(1024) k_refactor_cta(DPlan P, const double* __restrict__ ax,
                                                        double* lu_out, int* status,
                                                        PivotCheck pc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* const lu = reinterpret_cast<double*>(smem_raw);
-  unsigned* const sdone = reinterpret_cast<unsigned*>(lu + P.nslots);
+  unsigned char* const rings = smem_raw + (((size_t)8 * P.nslots + 15) & ~(size_t)15);
+  unsigned* const sdone = reinterpret_cast<unsigned*>(rings + (blockDim.x >> 5) * (kCtaRing * kCtaStage));
+  unsigned char* const ring = rings + (threadIdx.x >> 5) * (kCtaRing * kCtaStage);
   __shared__ unsigned snext;
   const int lane = threadIdx.x & 31;
   const int n = P.n;
   for (int i = threadIdx.x; i < n; i += blockDim.x) sdone[i] = 0u;
   if (threadIdx.x == 0) snext = 0u;
   __syncthreads();
-  bool failed = false;
-  while (!failed) {
+  while (true) {
     int k = 0;
     if (lane == 0) k = (int)atomicAdd(&snext, 1u);
     k = __shfl_sync(FULL, k, 0);
     if (k >= n) break;
     const int s0 = P.col_ptr[k], ds = P.dslot[k], s1 = P.col_ptr[k + 1];
+    const bool single = P.col_single[k] != 0;
     for (int s = s0 + lane; s < s1; s += 32) {
       double v = 0.0;
       for (int t = P.amap_ptr[s]; t < P.amap_ptr[s + 1]; ++t) v += ax[P.amap_idx[t]];
       lu[s] = v;
     }
-    int j0 = s0 < ds ? P.slot_row[s0] : 0;
-    int j1 = s0 + 1 < ds ? P.slot_row[s0 + 1] : 0;
-    int qa = 0, qb = 0, up = 0;
-    if (s0 < ds) {
-      qa = P.dslot[j0] + 1;
-      qb = P.col_ptr[j0 + 1];
-      up = P.upd_ptr[s0];
-    }
     __syncwarp();
-    for (int s = s0; s < ds; ++s) {
-      int nqa = 0, nqb = 0, nup = 0, j2 = 0;
-      if (s + 1 < ds) {
-        nqa = P.dslot[j1] + 1;
-        nqb = P.col_ptr[j1 + 1];
-        nup = P.upd_ptr[s + 1];
-      }
-      if (s + 2 < ds) j2 = P.slot_row[s + 2];
-      const int q = qa + lane;
-      const int d0 = q < qb ? P.upd_dst[up + lane] : 0;
-      int ok = 1;
-      if (lane == 0) {
-        unsigned spins = 0;
-        while (ld_acquire_cta(&sdone[j0]) == 0u) {
-          if (++spins > P.spin_limit) {
-            atomicCAS(status, DS_OK, DS_TIMEOUT);
-            ok = 0;
-            break;
-          }
-          if ((spins & 63u) == 0 && *(volatile int*)status != DS_OK) {
-            ok = 0;
-            break;
-          }
-          if (spins > 256) __nanosleep(20);  // shared-memory polls first
-        }
-      }
-      if (!__shfl_sync(FULL, ok, 0)) {
-        failed = true;
-        break;
-      }
-      const double u = lu[s];
-      if (u != 0.0) {
-        if (q < qb) lu[d0] = lu[d0] - lu[q] * u;
-        for (int qq = q + 32; qq < qb; qq += 32) {
-          const int d = P.upd_dst[up + qq - qa];
-          lu[d] = lu[d] - lu[qq] * u;
-        }
-      }
-      __syncwarp();
-      j0 = j1;
-      j1 = j2;
-      qa = nqa;
-      qb = nqb;
-      up = nup;
-    }
-    if (failed) break;
+    if (!block_updates(P, s0, ds, lu, sdone, ring, status)) break;
     if (pc.want != nullptr)
       pivot_check(
-          pc, k, ds, s1, P.col_single[k] != 0, [&](int q) { return lu[q]; },
+          pc, k, ds, s1, single, [&](int q) { return lu[q]; },
           [&](int q, double v) { lu[q] = v; });
-    const double diag = perturb(lu[ds], P.col_single[k] != 0);
-    for (int q = ds + 1 + lane; q < s1; q += 32) lu[q] = lu[q] / diag;
+    const double diag = bt::perturb_bits(lu[ds], single);
+    scale_column(
+        ds, s1, diag, [&](int q) { return lu[q]; }, [&](int q, double v) { lu[q] = v; });
+    __syncwarp();
     if (lane == 0) lu[ds] = diag;
     __syncwarp();
-    __threadfence_block();
     if (lane == 0) st_release_cta(&sdone[k], 1u);
   }
   __syncthreads();
@@ -1735,17 +2072,20 @@ void launch_first_factor(const DPlan& P, int maxblk, const double* ax, double* l
   k_first_factor<<<1, 32, 0, s>>>(P, ax, lu, work, rperm, rinv, tol, status);
 }
 
-void launch_refactor(const DPlan& P, const double* ax, double* lu, unsigned* flags,
-                     unsigned epoch, unsigned* counter, int* status, int grid,
-                     cudaStream_t s, const PivotCheck& pc) {
-  cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  k_refactor<<<grid, 128, 4 * kColBuf * sizeof(double), s>>>(P, ax, lu, flags, epoch, counter,
-                                                             status, pc);
+void launch_refactor(const DPlan& P, const double* ax, double* lu, double* big, int* status,
+                     int grid, cudaStream_t s, const PivotCheck& pc) {
+  cudaMemsetAsync(lu, 0xff, ((size_t)P.nslots + kLuPad) * sizeof(double), s);
+  const int colcap = std::min((P.max_col + 1) & ~1, kColCap);
+  const int bytes = kPairs * (kGridRing * kGridStage + 8 * colcap);
+  cudaFuncSetAttribute(k_refactor, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_refactor<<<grid, 64 * kPairs, bytes, s>>>(P, ax, lu, big, colcap, status, pc);
 }
+bool refactor_needs_big(const DPlan& P) { return P.max_col > kColCap; }
 
 namespace {
 size_t refactor_cta_bytes(const DPlan& P) {
-  return (size_t)8 * P.nslots + (size_t)4 * P.n + 16;
+  return (((size_t)8 * P.nslots + 15) & ~(size_t)15) + (size_t)32 * kCtaRing * kCtaStage +
+         (size_t)4 * P.n + 16;
 }
 int smem_optin() {
   int dev = 0, optin = 0;

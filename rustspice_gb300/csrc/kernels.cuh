@@ -35,6 +35,7 @@ inline size_t solve_steps_bytes(int n, int chunk) {
 // Device pointers of one Plan (see analysis.h for the meaning of each array).
 struct DPlan {
   int n, nslots, nblocks, ntask;
+  int max_col;  // slots of the longest column
   const int *col_ptr, *dslot, *slot_row, *upd_ptr, *upd_dst, *col_single;
   const int *amap_ptr, *amap_idx;
   const int *offd_ptr, *offd_col, *offd_raw;
@@ -281,9 +282,12 @@ struct PivotCheck {
   int* want = nullptr;
   double tol = 0.0;
 };
-void launch_refactor(const DPlan& P, const double* ax, double* lu, unsigned* flags,
-                     unsigned epoch, unsigned* counter, int* status, int grid,
-                     cudaStream_t s, const PivotCheck& pc = PivotCheck());
+// lu: nslots + kLuPad doubles, preset by the call (the padding holds the column
+// counter); big: nslots doubles where refactor_needs_big, else unused.
+constexpr int kLuPad = 4;
+bool refactor_needs_big(const DPlan& P);
+void launch_refactor(const DPlan& P, const double* ax, double* lu, double* big, int* status,
+                     int grid, cudaStream_t s, const PivotCheck& pc = PivotCheck());
 // Slots per chunk of the one-block solve's schedule.
 constexpr int kSolveChunk = 2048;
 // One-block variants for small factorizations; *_cta_fits says whether the
