@@ -3,12 +3,12 @@
 //
 // The diagonal blocks form one block-diagonal matrix M that the regular
 // factor kernels handle (its BTF finds the blocks). Around them:
-//  * ysolve  - Y_k = B_k^-1 R_k for the border columns that touch block k:
-//              one warp per tile of 32 columns, lanes over the columns, rows
-//              of L then U in order (the row-oriented views of the plan);
-//              tiles live in L2-resident [block size][32] arrays.
-//  * schur   - S = B_T - sum_k C_k Y_k, one warp per border column, one lane
-//              summing in a fixed order (deterministic).
+//  * reach   - S = B_T - sum_k C_k B_k^-1 R_k through the two sparse halves
+//              W = L^-1 P R and Z = U^-T Q^T C^T: one warp per border column
+//              (row) of a block, over the elimination path of its entries only;
+//              the column's warp then takes the products with the block's Z.
+//  * schur   - S = B_T - sum_k Z_k^T W_k, a thread block per border column, the
+//              blocks in order (deterministic).
 //  * dense LU of S without pivoting, rows and columns in the AMD order of
 //              S's structural pattern (the reference factors S with its
 //              no-pivot, AMD-ordered SparseLU), in 32-wide panels: panel
@@ -25,96 +25,249 @@ __device__ __forceinline__ double perturb_tiny(double d) {  // sparse_lu.rs no-p
   return d;
 }
 
-__global__ void k_bbd_ysolve(DPlan P, const double* __restrict__ lu,
-                             const double* __restrict__ ax, BbdArgs B, double* ybuf) {
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (t >= B.ntiles) return;
-  const int b0 = B.tile_pos0[t], sz = B.tile_size[t];
-  double* const Y = ybuf + B.tile_off[t];
-  for (int i = 0; i < sz; ++i) Y[(long long)i * 32 + lane] = 0.0;
-  __syncwarp();
-  if (lane == 0)  // R entries in CSC order (duplicates add in that order)
-    for (int e = B.init_ptr[t]; e < B.init_ptr[t + 1]; ++e) Y[B.init_code[e]] += ax[B.init_raw[e]];
-  __syncwarp();
-  // One row's dot product over its entries [e0, e1): the indices of eight
-  // entries load together, then their factor values and Y values, so a row
-  // costs two memory round trips per eight entries; the next row's range is
-  // read one row ahead.
-  auto row_dot = [&](const int* slot, const int* col, int e0, int e1, double v) {
-    double w = 0.0;
-    for (int e = e0; e < e1; e += 8) {
-      int sl[8], cl[8];
+// L and U by rows in the sweeps' order and the pivots' reciprocals.
+__global__ void k_bbd_rows(DPlan P, const double* __restrict__ lu, BbdArgs B) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < B.l.nnz) B.l.val[i] = lu[B.l.slot[i]];
+  if (i < B.u.nnz) B.u.val[i] = lu[B.u.slot[i]];
+  if (i < P.n) B.rec[i] = 1.0 / lu[P.dslot[i]];
+}
+
+constexpr int kSweepThreads = 512;
+
+// One block's triangular sweep on v, level by level: a warp per row where the
+// level has no more rows than warps, eight lanes per row else. The levels, rows
+// and ranges are copied to shared memory first; the next level's entries (four a
+// lane) are read while this one's are at work.
+__device__ __forceinline__ void sweep_block(const BbdSweep& S, int blk, int sz, const double* rec,
+                                            double* v) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int kAhead = 4;
+  int* const lv = reinterpret_cast<int*>(v + sz);  // at most sz + 1 bounds
+  int* const ptr = lv + sz + 1;
+  int* const row = ptr + sz + 1;
+  const int tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
+  const int l0 = S.lvl_ptr[blk], nl = S.lvl_ptr[blk + 1] - l0 - 1;
+  const int first = S.lv[l0], rows = S.lv[l0 + nl] - first;
+  __syncthreads();  // the sweep before has read its lists
+  for (int i = tid; i <= nl; i += blockDim.x) lv[i] = S.lv[l0 + i] - first;
+  for (int i = tid; i <= rows; i += blockDim.x) ptr[i] = S.ptr[first + i];
+  for (int i = tid; i < rows; i += blockDim.x) row[i] = S.row[first + i];
+  __syncthreads();
+  int w, i, e, end, c[kAhead];
+  double l[kAhead];
+  auto fetch = [&](int at, int b) {  // row `at` of the level that ends at row b
+    i = at < b ? at : -1;
+    e = end = 0;
+    if (i >= 0) {
+      e = ptr[i] + (lane & (w - 1));
+      end = ptr[i + 1];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (e + u < e1) {
-          sl[u] = slot[e + u];
-          cl[u] = col[e + u];
+      for (int q = 0; q < kAhead; ++q)
+        if (e + q * w < end) {
+          c[q] = S.col[e + q * w];
+          l[q] = S.val[e + q * w];
         }
-      double lv[8], yv[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (e + u < e1) {
-          lv[u] = lu[sl[u]];
-          yv[u] = Y[(long long)(cl[u] - b0) * 32 + lane];
-        }
-#pragma unroll
-      for (int u = 0; u < 8; u += 2) {
-        if (e + u < e1) v = fma(-lv[u], yv[u], v);
-        if (e + u + 1 < e1) w = fma(-lv[u + 1], yv[u + 1], w);
-      }
     }
-    return v + w;
   };
-  {  // L, unit diagonal
-    int e0 = P.lrow_ptr[b0], e1 = P.lrow_ptr[b0 + 1];
-    for (int i = 0; i < sz; ++i) {
-      const int ce0 = e0, ce1 = e1;
-      if (i + 1 < sz) {
-        e0 = e1;
-        e1 = P.lrow_ptr[b0 + i + 2];
+  auto level = [&](int q, int& a, int& b) {
+    a = q < nl ? lv[q] : 0;
+    b = q < nl ? lv[q + 1] : 0;
+    w = b - a <= nw ? 32 : 8;
+  };
+  int a, b;
+  level(0, a, b);
+  fetch(a + tid / w, b);
+  for (int q = 0; q < nl; ++q) {
+    for (bool more = true; more;) {
+      const int ci = i, cw = w, ce = e, cend = end;
+      int cc[kAhead];
+      double cl[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        cc[u] = c[u];
+        cl[u] = l[u];
       }
-      Y[(long long)i * 32 + lane] =
-          row_dot(P.lrow_slot, P.lrow_col, ce0, ce1, Y[(long long)i * 32 + lane]);
-    }
-  }
-  {  // U
-    int e0 = P.urow_ptr[b0 + sz - 1], e1 = P.urow_ptr[b0 + sz];
-    double dg = lu[P.dslot[b0 + sz - 1]];
-    for (int i = sz - 1; i >= 0; --i) {
-      const int ce0 = e0, ce1 = e1;
-      const double cdg = dg;
-      if (i > 0) {
-        e1 = e0;
-        e0 = P.urow_ptr[b0 + i - 1];
-        dg = lu[P.dslot[b0 + i - 1]];
+      const int at = a + tid / w + (nw * 32) / w;  // this level's next rows, or the next level
+      more = at - tid / w < b;
+      if (more) {
+        a += (nw * 32) / w;
+        fetch(at, b);
+      } else {
+        level(q + 1, a, b);
+        fetch(a + tid / w, b);
       }
-      Y[(long long)i * 32 + lane] =
-          row_dot(P.urow_slot, P.urow_col, ce0, ce1, Y[(long long)i * 32 + lane]) / cdg;
+      if (!__any_sync(FULL, ci >= 0)) continue;  // no FP64 from idle warps
+      double acc = 0.0;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (ce + u * cw < cend) acc = fma(cl[u], v[cc[u]], acc);
+      for (int x = ce + kAhead * cw; x < cend; x += cw) acc = fma(S.val[x], v[S.col[x]], acc);
+      if (cw == 32) {
+        acc += __shfl_xor_sync(FULL, acc, 16);
+        acc += __shfl_xor_sync(FULL, acc, 8);
+      }
+      acc += __shfl_xor_sync(FULL, acc, 4);
+      acc += __shfl_xor_sync(FULL, acc, 2);
+      acc += __shfl_xor_sync(FULL, acc, 1);
+      if (ci >= 0 && (lane & (cw - 1)) == 0) {
+        const int r = row[ci];
+        const double x = v[r] - acc;
+        v[r] = rec != nullptr ? x * rec[r] : x;
+      }
     }
+    __syncthreads();
   }
 }
 
-// S column j (column-major, leading dimension bs): B_T entries, then
-// -C_k Y_k for every tile column that holds border column j.
-__global__ void k_bbd_schur(const double* __restrict__ ax, BbdArgs B,
-                            const double* __restrict__ ybuf, double* S) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (j >= B.bs) return;
-  double* const col = S + (long long)j * B.bs;
-  for (int r = lane; r < B.bs; r += 32) col[r] = 0.0;
-  __syncwarp();
-  if (lane == 0) {
-    for (int e = B.bt_ptr[j]; e < B.bt_ptr[j + 1]; ++e) col[B.bt_row[e]] += ax[B.bt_raw[e]];
-    for (int q = B.yref_ptr[j]; q < B.yref_ptr[j + 1]; ++q) {
-      const int code = B.yref[q];  // (tile << 5) | lane
-      const int t = code >> 5, l = code & 31;
-      const double* Y = ybuf + B.tile_off[t];
-      const int blk = B.tile_blk[t];
-      for (int e = B.c_ptr[blk]; e < B.c_ptr[blk + 1]; ++e)
-        col[B.c_row[e]] = fma(-ax[B.c_raw[e]], Y[(long long)B.c_pos[e] * 32 + l], col[B.c_row[e]]);
+// A thread block per block of M: forward and backward substitution by levels.
+// Bounded by the levels' latency (about 150 levels of 50 x 50 meshes each way:
+// the entries' products, the sum across the warp and a barrier). Measured, 64
+// meshes of 30-50 a side: 0.61 ms against 1.43 ms for a warp per block that
+// takes the columns one after another.
+__global__ void __launch_bounds__(kSweepThreads) k_bbd_solve(DPlan P, BbdArgs B,
+                                                    const double* __restrict__ rhs, double* out) {
+  extern __shared__ double v[];
+  const int blk = blockIdx.x, p0 = P.block_ptr[blk], sz = P.block_ptr[blk + 1] - p0;
+  for (int i = threadIdx.x; i < sz; i += blockDim.x) v[i] = rhs[P.in_row[p0 + i]];
+  sweep_block(B.l, blk, sz, nullptr, v);
+  sweep_block(B.u, blk, sz, B.rec + p0, v);
+  for (int i = threadIdx.x; i < sz; i += blockDim.x) out[P.out_col[p0 + i]] = v[i];
+}
+
+// kRows: Z, by rows of U; else W, by columns of L, and its products with Z.
+// The block's vector v sits in shared memory (kShared) or in scratch. Measured,
+// 64 meshes of 30-50 a side and 1025 border nodes (5.9 k columns and rows, 130
+// steps each): 0.72 ms against 14.7 ms for Y = B^-1 R on dense tiles of 32
+// columns and C Y by one lane per column.
+template <bool kRows, bool kShared>
+__global__ void k_bbd_reach(DPlan P, const double* __restrict__ lu,
+                            const double* __restrict__ ax, BbdArgs B, int stride, int t0, int t1) {
+  extern __shared__ double vmem[];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  const int gw = blockIdx.x * wpb + w;
+  double* const v = kShared ? vmem + (size_t)w * stride : B.scratch + (size_t)gw * stride;
+  const BbdTasks& T = kRows ? B.z : B.w;
+  const double* const val = kRows ? B.u.val : lu;
+  const int* const row = kRows ? B.u.col : P.slot_row;
+  for (int q = t0 + gw; q < t1; q += gridDim.x * wpb) {
+    const int t = T.order[q];
+    const int blk = T.blk[t], p0 = P.block_ptr[blk], sz = P.block_ptr[blk + 1] - p0;
+    const int rb = kRows ? 0 : p0;  // U's columns count from the block's first
+    for (int i = lane; i <= sz; i += 32) v[i] = 0.0;  // v[sz] pads the products
+    __syncwarp();
+    if (lane == 0)  // in CSC order (duplicates add in that order)
+      for (int e = T.init_ptr[t]; e < T.init_ptr[t + 1]; ++e) v[T.init_pos[e]] += ax[T.init_raw[e]];
+    __syncwarp();
+    const int* const reach = T.reach + T.ptr[t];
+    const int len = (int)(T.ptr[t + 1] - T.ptr[t]);
+    double* const out = kRows ? B.zval + B.zout[t] : nullptr;
+    for (int c0 = 0; c0 < len; c0 += 32) {  // the ranges of 32 steps, one per lane
+      int c = 0, qa = 0, qb = 0;
+      double rc = 1.0;
+      if (c0 + lane < len) {
+        c = reach[c0 + lane];
+        const int i = kRows ? B.u.at[c] : 0;
+        qa = kRows ? B.u.ptr[i] : P.dslot[c] + 1;
+        qb = kRows ? B.u.ptr[i + 1] : P.col_ptr[c + 1];
+        if (kRows) rc = B.rec[c];
+      }
+      const int cnt = min(32, len - c0);
+      int na, nb, n0, n1;  // the next step's range, first 64 rows and values
+      double m0, m1;
+      auto fetch = [&](int i) {
+        na = __shfl_sync(FULL, qa, i);
+        nb = __shfl_sync(FULL, qb, i);
+        n0 = n1 = 0;
+        m0 = m1 = 0.0;
+        if (na + lane < nb) {
+          n0 = row[na + lane] - rb;
+          m0 = val[na + lane];
+        }
+        if (na + 32 + lane < nb) {
+          n1 = row[na + 32 + lane] - rb;
+          m1 = val[na + 32 + lane];
+        }
+      };
+      fetch(0);
+      for (int i = 0; i < cnt; ++i) {
+        const int a = na, b = nb, i0 = n0, i1 = n1;
+        const double l0 = m0, l1 = m1;
+        if (i + 1 < cnt) fetch(i + 1);
+        double x = v[__shfl_sync(FULL, c, i) - p0];
+        if (kRows) x *= __shfl_sync(FULL, rc, i);
+        if (kRows && lane == 0) out[(long long)(c0 + i) * 32] = x;
+        if (a + lane < b) v[i0] = fma(-l0, x, v[i0]);
+        if (a + 32 + lane < b) v[i1] = fma(-l1, x, v[i1]);
+        for (int q = a + 64 + lane; q < b; q += 32) {
+          const int r = row[q] - rb;
+          v[r] = fma(-val[q], x, v[r]);
+        }
+        __syncwarp();
+      }
     }
+    if (kRows) continue;
+    const int nrow = B.row_ptr[blk + 1] - B.row_ptr[blk];
+    double* const prod = B.gbuf + (B.goff[t] - B.goff[t0]);
+    const int g0 = B.grp_ptr[blk], g1 = B.grp_ptr[blk + 1];
+    for (int g = g0; g < g1; ++g) {
+      const int* const zi = B.zpos + B.grp_base[g] + lane;
+      const double* const zv = B.zval + B.grp_base[g] + lane;
+      const int glen = B.grp_len[g];  // a multiple of 8
+      double s0 = 0.0, s1 = 0.0;
+      for (int k = 0; k < glen; k += 8) {
+        int ix[8];
+        double zz[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          ix[u] = zi[(k + u) * 32];
+          zz[u] = zv[(k + u) * 32];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          s0 = fma(zz[u], v[ix[u]], s0);
+          s1 = fma(zz[u + 1], v[ix[u + 1]], s1);
+        }
+      }
+      const int r = (g - g0) * 32 + lane;
+      if (r < nrow) prod[r] = s0 + s1;
+    }
+    __syncwarp();
+  }
+}
+
+// S column j (column-major, leading dimension bs): B_T entries, then minus the
+// products of every block that touches border column j. Warp w sums its blocks
+// (every warps-th) in a column of its own, the columns are added in order.
+__global__ void k_bbd_schur(const double* __restrict__ ax, BbdArgs B, int j0, double* S) {
+  extern __shared__ double scol[];
+  const int j = j0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  const int w = tid >> 5, nw = blockDim.x >> 5;
+  double* const col = scol + (size_t)w * B.bs;
+  for (int r = tid; r < nw * B.bs; r += blockDim.x) scol[r] = 0.0;
+  __syncthreads();
+  // B_T, the entries of a row by one warp (the ground's diagonal has thousands)
+  for (int q = B.bt_ptr[j] + w; q < B.bt_ptr[j + 1]; q += nw) {
+    double v = 0.0;
+    for (int e = B.bt_ent[q] + lane; e < B.bt_ent[q + 1]; e += 32) v += ax[B.bt_raw[e]];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) col[B.bt_row[q]] = v;
+  }
+  __syncwarp();
+  const long long g0 = B.goff[B.wref_ptr[j0]];
+  for (int t = B.wref_ptr[j] + w; t < B.wref_ptr[j + 1]; t += nw) {
+    const int blk = B.w.blk[t], r0 = B.row_ptr[blk];
+    const int nrow = B.row_ptr[blk + 1] - r0;
+    const double* const g = B.gbuf + (B.goff[t] - g0);
+    for (int r = lane; r < nrow; r += 32) col[B.row[r0 + r]] -= g[r];
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int r = tid; r < B.bs; r += blockDim.x) {
+    double v = scol[r];
+    for (int q = 1; q < nw; ++q) v += scol[(size_t)q * B.bs + r];
+    S[(long long)j * B.bs + r] = v;
   }
 }
 
@@ -227,33 +380,91 @@ __global__ void k_dlu_update(double* S, int bs, int k0, int nb) {
     }
 }
 
-// x <- S^-1 x with the unit-lower / upper factors, one block.
-__global__ void k_dlu_solve(const double* __restrict__ S, int bs, double* x) {
-  for (int c = 0; c < bs; ++c) {
+// x <- S^-1 x with the unit-lower / upper factors, one block, in panels of 32
+// columns. While the other warps subtract a finished panel from the rows beyond,
+// the first warp subtracts it from the next panel's 32 rows (one per lane) and
+// solves that panel's triangle, its values shuffled. Bounded by FP64 issue on one
+// SM (a million multiply-adds for 1025 rows: 250 us); 0.47 ms against 1.4 ms
+// with two barriers per column.
+constexpr int kDluThreads = 512;
+__global__ void __launch_bounds__(kDluThreads) k_dlu_solve(const double* __restrict__ S, int bs,
+                                                           double* x) {
+  extern __shared__ double xs[];  // x[bs]
+  constexpr unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int r = tid; r < bs; r += blockDim.x) xs[r] = x[r];
+  __syncthreads();
+  const int np = (bs + 31) / 32;
+  // row r less panel p's columns
+  auto update = [&](int r, int p) {
+    const int k0 = 32 * p, nb = min(32, bs - k0);
+    const double* const col = S + (long long)k0 * bs + r;
+    double v = xs[r];
+    if (nb == 32) {
+#pragma unroll 16
+      for (int c = 0; c < 32; ++c) v = fma(-col[(long long)c * bs], xs[k0 + c], v);
+    } else {
+      for (int c = 0; c < nb; ++c) v = fma(-col[(long long)c * bs], xs[k0 + c], v);
+    }
+    return v;
+  };
+  for (int p = -1; p < np - 1; ++p) {  // panel p is final
+    const int n0 = 32 * (p + 1);
+    if (tid < 32) {
+      const int r = n0 + lane;
+      double l[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        l[c] = c < lane && r < bs ? S[(long long)(n0 + c) * bs + r] : 0.0;
+      double v = r >= bs ? 0.0 : p >= 0 ? update(r, p) : xs[r];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const double t = fma(-l[c], __shfl_sync(FULL, v, c), v);
+        if (lane > c) v = t;
+      }
+      if (r < bs) xs[r] = v;
+    } else if (p >= 0) {
+      for (int r = n0 + tid; r < bs; r += blockDim.x - 32) xs[r] = update(r, p);
+    }
     __syncthreads();
-    const double xc = x[c];
-    __syncthreads();
-    for (int r = c + 1 + threadIdx.x; r < bs; r += blockDim.x)
-      x[r] = fma(-S[(long long)c * bs + r], xc, x[r]);
   }
-  for (int c = bs - 1; c >= 0; --c) {
+  for (int p = np; p > 0; --p) {
+    const int n0 = 32 * (p - 1);
+    if (tid < 32) {
+      const int r = n0 + lane;
+      double u[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        u[c] = lane < c && n0 + c < bs ? S[(long long)(n0 + c) * bs + r] : 0.0;
+      const double rc = r < bs ? 1.0 / S[(long long)r * bs + r] : 0.0;
+      double v = r >= bs ? 0.0 : p < np ? update(r, p) : xs[r];
+#pragma unroll
+      for (int c = 31; c >= 0; --c) {
+        if (lane == c) v *= rc;
+        const double t = fma(-u[c], __shfl_sync(FULL, v, c), v);
+        if (lane < c) v = t;
+      }
+      if (r < bs) xs[r] = v;
+    } else if (p < np) {
+      for (int r = tid - 32; r < n0; r += blockDim.x - 32) xs[r] = update(r, p);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) x[c] = x[c] / S[(long long)c * bs + c];
-    __syncthreads();
-    const double xc = x[c];
-    for (int r = threadIdx.x; r < c; r += blockDim.x) x[r] = fma(-S[(long long)c * bs + r], xc, x[r]);
   }
+  for (int r = tid; r < bs; r += blockDim.x) x[r] = xs[r];
 }
 
-// bb[j] = rhs[border row j] - sum_c C[j][c] z[c]  (row lists in CSC order)
+// bb[j] = rhs[border row j] - sum_c C[j][c] z[c], a warp per border row (the
+// ground row has thousands of entries).
 __global__ void k_bbd_border_rhs(const double* __restrict__ ax, const double* __restrict__ rhs,
                                  const double* __restrict__ z, BbdArgs B, double* bb) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (j >= B.bs) return;
-  double v = rhs[B.bperm[j]];
-  for (int e = B.crow_ptr[j]; e < B.crow_ptr[j + 1]; ++e)
-    v = fma(-ax[B.crow_raw[e]], z[B.crow_col[e]], v);
-  bb[j] = v;
+  double v = 0.0;
+  for (int e = B.crow_ptr[j] + lane; e < B.crow_ptr[j + 1]; e += 32)
+    v = fma(ax[B.crow_raw[e]], z[B.crow_col[e]], v);
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  if (lane == 0) bb[j] = rhs[B.bperm[j]] - v;
 }
 
 // w[m] = sum_j R[m][j] xT[j] over the rows of M
@@ -286,14 +497,62 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
 
-void launch_bbd_ysolve(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B,
-                       double* ybuf, cudaStream_t s) {
-  if (B.ntiles > 0) k_bbd_ysolve<<<cdiv(B.ntiles, 4), 128, 0, s>>>(P, lu, ax, B, ybuf);
+namespace {
+// Warps per block of the reach kernels with their vectors in shared memory: two
+// (five blocks of 50 x 50 meshes share an SM), one, or none.
+int reach_warps(int max_block) {
+  const size_t one = (size_t)8 * ((max_block + 2) & ~1);
+  return 2 * one <= (size_t)(226 * 1024) ? 2 : one <= (size_t)(226 * 1024) ? 1 : 0;
+}
+template <bool kRows>
+void launch_reach(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B, int t0,
+                  int t1, cudaStream_t s) {
+  if (t1 <= t0) return;
+  const int stride = (B.max_block + 2) & ~1, wpb = reach_warps(B.max_block);
+  if (wpb > 0) {
+    const int bytes = wpb * stride * 8;
+    cudaFuncSetAttribute(k_bbd_reach<kRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         bytes);
+    k_bbd_reach<kRows, true>
+        <<<cdiv(t1 - t0, wpb), 32 * wpb, bytes, s>>>(P, lu, ax, B, stride, t0, t1);
+  } else {
+    k_bbd_reach<kRows, false>
+        <<<bbd_scratch_warps() / 4, 128, 0, s>>>(P, lu, ax, B, stride, t0, t1);
+  }
+}
+}  // namespace
+
+bool bbd_shared_fits(int max_block) { return reach_warps(max_block) > 0; }
+namespace {
+size_t bbd_solve_bytes(int max_block) { return (size_t)20 * max_block + 16; }
+}  // namespace
+bool bbd_solve_fits(int max_block) { return bbd_solve_bytes(max_block) <= (size_t)(226 * 1024); }
+int bbd_scratch_warps() { return 1024; }
+
+void launch_bbd_z(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B,
+                  cudaStream_t s) {
+  int m = P.n;
+  if (B.l.nnz > m) m = B.l.nnz;
+  if (B.u.nnz > m) m = B.u.nnz;
+  if (m > 0) k_bbd_rows<<<cdiv(m, 256), 256, 0, s>>>(P, lu, B);
+  launch_reach<true>(P, lu, ax, B, 0, B.z.n, s);
 }
 
-void launch_bbd_schur(const double* ax, const BbdArgs& B, const double* ybuf, double* S,
+void launch_bbd_solve(const DPlan& P, const BbdArgs& B, const double* rhs, double* out,
                       cudaStream_t s) {
-  k_bbd_schur<<<cdiv(B.bs, 4), 128, 0, s>>>(ax, B, ybuf, S);
+  const int bytes = (int)bbd_solve_bytes(B.max_block);
+  cudaFuncSetAttribute(k_bbd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_bbd_solve<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, rhs, out);
+}
+
+void launch_bbd_schur(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B, int j0,
+                      int j1, int t0, int t1, double* S, cudaStream_t s) {
+  launch_reach<false>(P, lu, ax, B, t0, t1, s);
+  int nw = 8;  // warps, a column of S each
+  while (nw > 1 && nw * B.bs * 8 > 100 * 1024) nw >>= 1;
+  const int bytes = nw * B.bs * 8;
+  cudaFuncSetAttribute(k_bbd_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_bbd_schur<<<j1 - j0, 32 * nw, bytes, s>>>(ax, B, j0, S);
 }
 
 void launch_dense_lu(double* S, int bs, cudaStream_t s) {
@@ -311,12 +570,13 @@ void launch_dense_lu(double* S, int bs, cudaStream_t s) {
 }
 
 void launch_dense_lu_solve(const double* S, int bs, double* x, cudaStream_t s) {
-  k_dlu_solve<<<1, 1024, 0, s>>>(S, bs, x);
+  cudaFuncSetAttribute(k_dlu_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, bs * 8);
+  k_dlu_solve<<<1, kDluThreads, bs * 8, s>>>(S, bs, x);
 }
 
 void launch_bbd_border_rhs(const double* ax, const double* rhs, const double* z,
                            const BbdArgs& B, double* bb, cudaStream_t s) {
-  k_bbd_border_rhs<<<cdiv(B.bs, 128), 128, 0, s>>>(ax, rhs, z, B, bb);
+  k_bbd_border_rhs<<<cdiv(B.bs, 4), 128, 0, s>>>(ax, rhs, z, B, bb);
 }
 
 void launch_bbd_rmatvec(const double* ax, const double* xT, const BbdArgs& B, double* w,

@@ -525,6 +525,24 @@ void make_solve_program(const gk::Plan& p, bool transpose, SolveProgram& out) {
   lay_out_solve(ops, best_step, best_ns, best_chain, best_chains, chunk, out);
 }
 
+// The columns as the grid refactorization hands them out: by the number of
+// columns that wait for one another behind it, the longest chain first (a
+// column comes after every column it depends on).
+std::vector<i32> column_order(const gk::Plan& p) {
+  std::vector<int> tail(p.n, 0);
+  int most = 0;
+  for (int k = p.n - 1; k >= 0; --k) {
+    for (int q = p.col_ptr[k]; q < p.dslot[k]; ++q)
+      tail[p.slot_row[q]] = std::max(tail[p.slot_row[q]], tail[k] + 1);
+    most = std::max(most, tail[k]);
+  }
+  std::vector<i32> at(most + 2, 0), out(p.n);
+  for (int t : tail) ++at[most - t + 1];
+  for (int t = 0; t <= most; ++t) at[t + 1] += at[t];
+  for (int k = 0; k < p.n; ++k) out[at[most - tail[k]]++] = k;
+  return out;
+}
+
 // Device copy of a SolveProgram.
 struct SolveDev {
   DBuf<int4> ops, chunks, chains;
@@ -543,7 +561,7 @@ struct SolveDev {
 
 // Device copy of a Plan.
 struct PlanDev {
-  DBuf<i32> col_ptr, dslot, slot_row, upd_ptr, upd_dst, col_single, amap_ptr, amap_idx,
+  DBuf<i32> order, col_ptr, dslot, slot_row, upd_ptr, upd_dst, col_single, amap_ptr, amap_idx,
       offd_ptr, offd_col, offd_raw, offdT_ptr, offdT_row, offdT_raw, lrow_ptr, lrow_col,
       lrow_slot, urow_ptr, urow_col,
       urow_slot, in_row, out_col, pcol_ptr, pcol_raw, pcol_q, pos_block, block_ptr, task,
@@ -585,9 +603,11 @@ struct PlanDev {
     const char* ess = getenv("GPUKLU_SOLVE_STEPS");
     if (solves && !(ess && ess[0] == '0')) make_solve_program(p, false, sp);
     updates = (int64_t)p.upd_dst.size();
+    if (e == cudaSuccess) e = order.upload(column_order(p), s);
     gk::DPlan d{};
     if (e == cudaSuccess) e = ss.upload(sp, s, d.ss);
     d.n = p.n;
+    d.order = order.p;
     for (int k = 0; k < p.n; ++k) d.max_col = std::max<int>(d.max_col, p.col_ptr[k + 1] - p.col_ptr[k]);
     d.noffd = p.offd_ptr.empty() ? 0 : p.offd_ptr.back();
     d.cs_nchunk = (int)(hc.size() / 4);
@@ -3926,11 +3946,24 @@ struct gpuklu_bbd {
   bool tiles_ready = false;
   int ntiles = 0;
   std::vector<i32> perm32;
-  DBuf<i32> d_m_raw, d_perm, d_tile_pos0, d_tile_size, d_tile_blk, d_init_ptr, d_init_code,
-      d_init_raw, d_bt_ptr, d_bt_row, d_bt_raw, d_yref_ptr, d_yref, d_c_ptr, d_c_row, d_c_pos,
-      d_c_raw, d_crow_ptr, d_crow_col, d_crow_raw, d_rrow_ptr, d_rrow_col, d_rrow_raw, d_bperm;
-  DBuf<long long> d_tile_off;
-  DBuf<double> d_ax, d_rhs, d_rhs_c, d_x, d_newx, d_y, d_S, d_xT, d_z;
+  DBuf<i32> d_m_raw, d_perm, d_bt_ptr, d_bt_row, d_bt_ent, d_bt_raw, d_crow_ptr, d_crow_col, d_crow_raw,
+      d_rrow_ptr, d_rrow_col, d_rrow_raw, d_bperm, d_grp_ptr, d_grp_len, d_zpos, d_row_ptr, d_row,
+      d_wref_ptr;
+  DBuf<long long> d_grp_base, d_zout, d_goff;
+  struct TaskDev {
+    DBuf<i32> blk, reach, init_ptr, init_pos, init_raw, order;
+    DBuf<long long> ptr;
+  } d_wt, d_zt;
+  struct SweepDev {
+    DBuf<i32> lvl_ptr, lv, row, ptr, col, slot, at;
+    DBuf<double> val;
+  } d_lsw, d_usw;
+  DBuf<double> d_ax, d_rhs, d_rhs_c, d_x, d_newx, d_S, d_xT, d_z;
+  DBuf<double> d_zval, d_gbuf, d_rec, d_scratch;
+  // border columns [cut[i].first, cut[i + 1].first) share gbuf, cut[i].second
+  // their first W task
+  std::vector<std::pair<int, int>> cuts;
+  static constexpr long long kProducts = 1ll << 26;  // doubles of gbuf (one column may exceed it)
   DBuf<gk::NewtonState> d_nstate;
   DBuf<int> d_status;
   DBuf<unsigned> d_bar;  // grid barrier of the cooperative Schur LU
@@ -3963,8 +3996,9 @@ struct gpuklu_bbd {
       for (int q = P.block_ptr[b]; q < P.block_ptr[b + 1]; ++q) pblk[q] = b;
     // R entries by plan block: border column j, M row m, raw q (CSC order)
     std::vector<std::vector<int>> jcols(nb);
-    std::vector<std::vector<std::pair<int, int>>> rent(nb);  // (pos offset, raw) per (j)
-    std::vector<std::vector<int>> rent_j(nb);
+    std::vector<std::vector<std::pair<int, int>>> rent(nb);  // (pos offset, raw), by column
+    std::vector<std::vector<int>> rent_ptr(nb);              // first entry of each of jcols
+    std::vector<std::vector<std::pair<int, int>>> jblk(bs);  // (block, index in its jcols)
     std::vector<std::vector<i32>> rrow(nm);  // per M row: (j, raw) pairs flattened
     std::vector<i32> bt_ptr(bs + 1, 0), bt_row, bt_raw;
     for (int j = 0; j < bs; ++j) {
@@ -3978,45 +4012,24 @@ struct gpuklu_bbd {
           bt_raw.push_back((i32)q);
         } else {
           const int pos = in_pos[nr], b = pblk[pos];
-          if (jcols[b].empty() || jcols[b].back() != j) jcols[b].push_back(j);
+          if (jcols[b].empty() || jcols[b].back() != j) {
+            jblk[j].push_back({b, (int)jcols[b].size()});
+            jcols[b].push_back(j);
+            rent_ptr[b].push_back((int)rent[b].size());
+          }
           rent[b].push_back({pos - P.block_ptr[b], (int)q});
-          rent_j[b].push_back((int)jcols[b].size() - 1);
           rrow[nr].push_back(j);
           rrow[nr].push_back((i32)q);
         }
       }
+      std::sort(jblk[j].begin(), jblk[j].end());
       bt_ptr[j + 1] = (i32)bt_row.size();
     }
-    // tiles of 32 border columns per plan block
-    std::vector<i32> tile_pos0, tile_size, tile_blk, init_ptr(1, 0), init_code, init_raw;
-    std::vector<long long> tile_off;
-    std::vector<std::vector<i32>> yref(bs);
-    long long off = 0;
+    ntiles = 0;
     for (int b = 0; b < nb; ++b) {
-      const int ncol = (int)jcols[b].size();
-      const int sz = P.block_ptr[b + 1] - P.block_ptr[b];
-      const int first_tile = (int)tile_pos0.size();
-      for (int t0 = 0; t0 < ncol; t0 += 32) {
-        tile_pos0.push_back(P.block_ptr[b]);
-        tile_size.push_back(sz);
-        tile_blk.push_back(b);
-        tile_off.push_back(off);
-        off += (long long)sz * 32;
-        const int t = (int)tile_pos0.size() - 1;
-        for (int l = 0; l < 32 && t0 + l < ncol; ++l) yref[jcols[b][t0 + l]].push_back((t << 5) | l);
-      }
-      (void)first_tile;
-      for (int t0 = 0; t0 < ncol; t0 += 32) {  // each tile's R entries, CSC order
-        for (size_t e = 0; e < rent[b].size(); ++e) {
-          const int k = rent_j[b][e];
-          if (k < t0 || k >= t0 + 32) continue;
-          init_code.push_back(rent[b][e].first * 32 + (k - t0));
-          init_raw.push_back(rent[b][e].second);
-        }
-        init_ptr.push_back((i32)init_code.size());
-      }
+      rent_ptr[b].push_back((int)rent[b].size());
+      ntiles += ((int)jcols[b].size() + 31) / 32;
     }
-    ntiles = (int)tile_pos0.size();
     // C entries: block columns c with border rows, per plan block and per border row
     std::vector<std::vector<i32>> cb(nb);    // per plan block: (row, pos, raw) triples
     std::vector<std::vector<i32>> crow(bs);  // per border row: (c, raw)
@@ -4062,8 +4075,8 @@ struct gpuklu_bbd {
             mark[bt_row[e]] = j;
             rows.push_back(bt_row[e]);
           }
-        for (i32 code : yref[j]) {
-          const int b = tile_blk[code >> 5];
+        for (const auto& bl : jblk[j]) {
+          const int b = bl.first;
           for (int r : crows[b])
             if (mark[r] != j) {
               mark[r] = j;
@@ -4077,14 +4090,18 @@ struct gpuklu_bbd {
       gk::amd_order(bs, sap.data(), sai.data(), spos, sinv);
     }
     for (auto& r : bt_row) r = spos[r];
-    std::vector<i32> yref_ptr(bs + 1, 0), yref_flat, bt_ptr_s(bs + 1, 0), bt_row_s, bt_raw_s;
-    for (int s2 = 0; s2 < bs; ++s2) {  // S columns in elimination order
+    std::vector<i32> bt_ptr_s(bs + 1, 0), bt_row_s, bt_raw_s, bt_ent(1, 0);
+    for (int s2 = 0; s2 < bs; ++s2) {  // S columns in elimination order, by row
       const int j = sinv[s2];
-      yref_flat.insert(yref_flat.end(), yref[j].begin(), yref[j].end());
-      yref_ptr[s2 + 1] = (i32)yref_flat.size();
-      for (int e = bt_ptr[j]; e < bt_ptr[j + 1]; ++e) {
-        bt_row_s.push_back(bt_row[e]);
-        bt_raw_s.push_back(bt_raw[e]);
+      std::vector<std::pair<int, int>> en;
+      for (int e = bt_ptr[j]; e < bt_ptr[j + 1]; ++e) en.push_back({bt_row[e], bt_raw[e]});
+      std::stable_sort(en.begin(), en.end(),
+                       [](const auto& x, const auto& y) { return x.first < y.first; });
+      for (size_t e = 0; e < en.size(); ++e) {
+        bt_raw_s.push_back(en[e].second);
+        if (e + 1 < en.size() && en[e + 1].first == en[e].first) continue;
+        bt_row_s.push_back(en[e].first);
+        bt_ent.push_back((i32)bt_raw_s.size());
       }
       bt_ptr_s[s2 + 1] = (i32)bt_row_s.size();
     }
@@ -4093,15 +4110,198 @@ struct gpuklu_bbd {
     bt_raw.swap(bt_raw_s);
     std::vector<i32> bperm(bs);
     for (int s2 = 0; s2 < bs; ++s2) bperm[s2] = d.perm[d.border_start + sinv[s2]];
-    std::vector<i32> c_ptr(nb + 1, 0), c_row, c_pos, c_raw;
-    for (int b = 0; b < nb; ++b) {
-      for (size_t e = 0; e < cb[b].size(); e += 3) {
-        c_row.push_back(spos[cb[b][e]]);
-        c_pos.push_back(cb[b][e + 1]);
-        c_raw.push_back(cb[b][e + 2]);
+
+    // The positions a triangular solve reaches from its right-hand side's. Where
+    // every position's list is the list of its first member, that member apart
+    // (symmetric fill), they are the chains of first members; else the closure.
+    std::vector<int> first_l(nm, -1), first_u(nm, -1);
+    std::vector<char> chain_l(nb, 1), chain_u(nb, 1);
+    auto lcol = [&](int k) {
+      return std::make_pair(P.slot_row.data() + P.dslot[k] + 1, P.slot_row.data() + P.col_ptr[k + 1]);
+    };
+    auto urow = [&](int k) {
+      return std::make_pair(P.urow_col.data() + P.urow_ptr[k], P.urow_col.data() + P.urow_ptr[k + 1]);
+    };
+    auto chains = [&](auto list, std::vector<int>& first, std::vector<char>& ok) {
+      for (int k = 0; k < nm; ++k) {
+        const auto a = list(k);
+        if (a.first == a.second) continue;
+        first[k] = *a.first;
+        const auto f = list(first[k]);
+        if (!std::is_sorted(a.first, a.second) ||
+            !std::includes(f.first, f.second, a.first + 1, a.second))
+          ok[pblk[k]] = 0;
       }
-      c_ptr[b + 1] = (i32)c_row.size();
+    };
+    chains(lcol, first_l, chain_l);
+    chains(urow, first_u, chain_u);
+    std::vector<int> mark(nm, -1);
+    int stamp = 0;
+    auto reach_of = [&](const std::vector<std::pair<int, int>>& init, int b, auto list,
+                        const std::vector<int>& first, bool chain, std::vector<i32>& out) {
+      const int p0 = P.block_ptr[b], p1 = P.block_ptr[b + 1];
+      const size_t at = out.size();
+      ++stamp;
+      if (chain) {
+        for (const auto& en : init)
+          for (int k = p0 + en.first; k >= 0 && mark[k] != stamp; k = first[k]) {
+            mark[k] = stamp;
+            out.push_back(k);
+          }
+        if (init.size() > 1) std::sort(out.begin() + at, out.end());
+        return;
+      }
+      int lo = p1;
+      for (const auto& en : init) {
+        mark[p0 + en.first] = stamp;
+        lo = std::min(lo, p0 + en.first);
+      }
+      for (int k = lo; k < p1; ++k) {
+        if (mark[k] != stamp) continue;
+        out.push_back(k);
+        const auto a = list(k);
+        for (const int* r = a.first; r != a.second; ++r) mark[*r] = stamp;
+      }
+    };
+    struct Tasks {
+      std::vector<i32> blk, reach, init_ptr{0}, init_pos, init_raw;
+      std::vector<long long> ptr{0};
+      void add(int b, const std::vector<std::pair<int, int>>& init) {
+        blk.push_back(b);
+        for (const auto& en : init) {
+          init_pos.push_back(en.first);
+          init_raw.push_back(en.second);
+        }
+        init_ptr.push_back((i32)init_pos.size());
+        ptr.push_back((long long)reach.size());
+      }
+    } wt, zt;
+    // Z tasks: a block's border rows, the longest first, in groups of 32
+    std::vector<i32> grp_ptr(nb + 1, 0), grp_len, zpos, row_ptr(nb + 1, 0), row;
+    std::vector<long long> grp_base, zout;
+    std::vector<int> local(bs, -1);
+    for (int b = 0; b < nb; ++b) {
+      const int p0 = P.block_ptr[b], sz = P.block_ptr[b + 1] - p0;
+      std::vector<int> rows;
+      std::vector<std::vector<std::pair<int, int>>> init;
+      for (size_t e = 0; e < cb[b].size(); e += 3) {
+        int& l = local[cb[b][e]];
+        if (l < 0) {
+          l = (int)rows.size();
+          rows.push_back(cb[b][e]);
+          init.emplace_back();
+        }
+        init[l].push_back({cb[b][e + 1], cb[b][e + 2]});
+      }
+      std::vector<std::vector<i32>> reach(rows.size());
+      for (size_t l = 0; l < rows.size(); ++l) {
+        local[rows[l]] = -1;
+        reach_of(init[l], b, urow, first_u, chain_u[b], reach[l]);
+      }
+      std::vector<int> by(rows.size());
+      for (size_t l = 0; l < rows.size(); ++l) by[l] = (int)l;
+      std::stable_sort(by.begin(), by.end(),
+                       [&](int x, int y) { return reach[x].size() > reach[y].size(); });
+      for (size_t g = 0; g < by.size(); g += 32) {
+        const size_t end = std::min(by.size(), g + 32);
+        const int len = ((int)reach[by[g]].size() + 7) & ~7;
+        const long long base = (long long)zpos.size();
+        grp_base.push_back(base);
+        grp_len.push_back(len);
+        zpos.resize(base + (long long)len * 32, sz);
+        for (size_t i = g; i < end; ++i) {
+          const auto& rc = reach[by[i]];
+          for (size_t q = 0; q < rc.size(); ++q) zpos[base + (long long)q * 32 + (i - g)] = rc[q] - p0;
+          zout.push_back(base + (long long)(i - g));
+          zt.reach.insert(zt.reach.end(), rc.begin(), rc.end());
+          zt.add(b, init[by[i]]);
+          row.push_back(spos[rows[by[i]]]);
+        }
+      }
+      grp_ptr[b + 1] = (i32)grp_len.size();
+      row_ptr[b + 1] = (i32)row.size();
     }
+    // W tasks: the border columns in elimination order, their blocks ascending
+    std::vector<i32> wref_ptr(bs + 1, 0);
+    std::vector<long long> goff(1, 0);
+    cuts.assign(1, {0, 0});
+    for (int s2 = 0; s2 < bs; ++s2) {
+      for (const auto& bl : jblk[sinv[s2]]) {
+        const int b = bl.first;
+        const std::vector<std::pair<int, int>> init(rent[b].begin() + rent_ptr[b][bl.second],
+                                                    rent[b].begin() + rent_ptr[b][bl.second + 1]);
+        reach_of(init, b, lcol, first_l, chain_l[b], wt.reach);
+        wt.add(b, init);
+        goff.push_back(goff.back() + row_ptr[b + 1] - row_ptr[b]);
+      }
+      wref_ptr[s2 + 1] = (i32)wt.blk.size();
+      if (goff.back() - goff[cuts.back().second] > kProducts && s2 > cuts.back().first) {
+        cuts.push_back({s2, wref_ptr[s2]});
+      }
+    }
+    cuts.push_back({bs, (int)wt.blk.size()});
+    long long products = 1;
+    for (size_t i = 0; i + 1 < cuts.size(); ++i)
+      products = std::max(products, goff[cuts[i + 1].second] - goff[cuts[i].second]);
+    int max_block = 0;
+    for (int b = 0; b < nb; ++b)
+      max_block = std::max(max_block, P.block_ptr[b + 1] - P.block_ptr[b]);
+    // the tasks of a batch as they start, the longest first
+    auto by_length = [](const Tasks& t, int a, int b, std::vector<i32>& order) {
+      for (int i = a; i < b; ++i) order.push_back(i);
+      std::stable_sort(order.end() - (b - a), order.end(), [&](int x, int y) {
+        return t.ptr[x + 1] - t.ptr[x] > t.ptr[y + 1] - t.ptr[y];
+      });
+    };
+    std::vector<i32> worder, zorder;
+    for (size_t i = 0; i + 1 < cuts.size(); ++i)
+      by_length(wt, cuts[i].second, cuts[i + 1].second, worder);
+    by_length(zt, 0, (int)zt.blk.size(), zorder);
+    // the factors by rows, each block's rows by level
+    struct Sweep {
+      std::vector<i32> lvl_ptr{0}, lv, row, ptr, col, slot, at;
+    } lsw, usw;
+    auto make_sweep = [&](const auto& rptr, const auto& rcol, const auto& rslot, bool upper,
+                          Sweep& S) {
+      std::vector<int> lev(nm, 0), cnt;
+      std::vector<i32> by;
+      if (upper) S.at.resize(nm);
+      for (int b = 0; b < nb; ++b) {
+        const int p0 = P.block_ptr[b], p1 = P.block_ptr[b + 1];
+        int most = 0;
+        for (int q = p0; q < p1; ++q) {
+          const int i = upper ? p0 + p1 - 1 - q : q;
+          int l = upper ? 1 : 0;  // L rows without entries have nothing to do
+          for (int e = rptr[i]; e < rptr[i + 1]; ++e) l = std::max(l, lev[rcol[e]] + 1);
+          lev[i] = l;
+          most = std::max(most, l);
+        }
+        cnt.assign(most + 2, 0);
+        for (int i = p0; i < p1; ++i) ++cnt[lev[i] + 1];
+        for (int l = 0; l <= most; ++l) cnt[l + 1] += cnt[l];
+        by.resize(p1 - p0);
+        std::vector<int> at(cnt.begin(), cnt.end());
+        for (int i = p0; i < p1; ++i) by[at[lev[i]]++] = i;
+        for (int l = 1; l <= most; ++l) {
+          S.lv.push_back((i32)S.row.size());
+          for (int q = cnt[l]; q < cnt[l + 1]; ++q) {
+            const int i = by[q];
+            if (upper) S.at[i] = (i32)S.row.size();
+            S.row.push_back(i - p0);
+            S.ptr.push_back((i32)S.col.size());
+            for (int e = rptr[i]; e < rptr[i + 1]; ++e) {
+              S.col.push_back(rcol[e] - p0);
+              S.slot.push_back(rslot[e]);
+            }
+          }
+        }
+        S.lv.push_back((i32)S.row.size());
+        S.lvl_ptr.push_back((i32)S.lv.size());
+      }
+      S.ptr.push_back((i32)S.col.size());
+    };
+    make_sweep(P.lrow_ptr, P.lrow_col, P.lrow_slot, false, lsw);
+    make_sweep(P.urow_ptr, P.urow_col, P.urow_slot, true, usw);
     std::vector<i32> crow_ptr(bs + 1, 0), crow_col, crow_raw;
     for (int s2 = 0; s2 < bs; ++s2) {  // border rows in S order
       const int r = sinv[s2];
@@ -4123,46 +4323,74 @@ struct gpuklu_bbd {
     cudaError_t e = cudaSuccess;
 #define UP(buf, vec) \
   if (e == cudaSuccess) e = buf.upload(vec, s);
-    UP(d_tile_pos0, tile_pos0) UP(d_tile_size, tile_size) UP(d_tile_blk, tile_blk)
-    UP(d_tile_off, tile_off) UP(d_init_ptr, init_ptr) UP(d_init_code, init_code)
-    UP(d_init_raw, init_raw) UP(d_bt_ptr, bt_ptr) UP(d_bt_row, bt_row) UP(d_bt_raw, bt_raw)
-    UP(d_yref_ptr, yref_ptr) UP(d_yref, yref_flat) UP(d_c_ptr, c_ptr) UP(d_c_row, c_row)
-    UP(d_c_pos, c_pos) UP(d_c_raw, c_raw) UP(d_crow_ptr, crow_ptr) UP(d_crow_col, crow_col)
-    UP(d_crow_raw, crow_raw) UP(d_rrow_ptr, rrow_ptr) UP(d_rrow_col, rrow_col)
-    UP(d_rrow_raw, rrow_raw) UP(d_bperm, bperm)
+    UP(d_bt_ptr, bt_ptr) UP(d_bt_row, bt_row) UP(d_bt_ent, bt_ent) UP(d_bt_raw, bt_raw)
+    UP(d_crow_ptr, crow_ptr) UP(d_crow_col, crow_col) UP(d_crow_raw, crow_raw)
+    UP(d_rrow_ptr, rrow_ptr) UP(d_rrow_col, rrow_col) UP(d_rrow_raw, rrow_raw) UP(d_bperm, bperm)
+    UP(d_grp_ptr, grp_ptr) UP(d_grp_len, grp_len) UP(d_grp_base, grp_base) UP(d_zout, zout)
+    UP(d_zpos, zpos) UP(d_row_ptr, row_ptr) UP(d_row, row) UP(d_goff, goff)
+    UP(d_wref_ptr, wref_ptr)
+    UP(d_wt.blk, wt.blk) UP(d_wt.ptr, wt.ptr) UP(d_wt.reach, wt.reach)
+    UP(d_wt.init_ptr, wt.init_ptr) UP(d_wt.init_pos, wt.init_pos) UP(d_wt.init_raw, wt.init_raw)
+    UP(d_zt.blk, zt.blk) UP(d_zt.ptr, zt.ptr) UP(d_zt.reach, zt.reach)
+    UP(d_zt.init_ptr, zt.init_ptr) UP(d_zt.init_pos, zt.init_pos) UP(d_zt.init_raw, zt.init_raw)
+    UP(d_wt.order, worder) UP(d_zt.order, zorder)
+    UP(d_lsw.lvl_ptr, lsw.lvl_ptr) UP(d_lsw.lv, lsw.lv) UP(d_lsw.row, lsw.row)
+    UP(d_lsw.ptr, lsw.ptr) UP(d_lsw.col, lsw.col) UP(d_lsw.slot, lsw.slot)
+    UP(d_usw.lvl_ptr, usw.lvl_ptr) UP(d_usw.lv, usw.lv) UP(d_usw.row, usw.row)
+    UP(d_usw.ptr, usw.ptr) UP(d_usw.col, usw.col) UP(d_usw.slot, usw.slot) UP(d_usw.at, usw.at)
 #undef UP
-    if (e == cudaSuccess) e = d_y.resize(std::max<long long>(off, 1));
+    if (e == cudaSuccess) e = d_zval.resize(std::max<size_t>(zpos.size(), 1));
+    if (e == cudaSuccess)  // the padding stays zero
+      e = cudaMemsetAsync(d_zval.p, 0, std::max<size_t>(zpos.size(), 1) * sizeof(double), s);
+    if (e == cudaSuccess) e = d_gbuf.resize((size_t)products);
+    if (e == cudaSuccess) e = d_lsw.val.resize(lsw.col.size());
+    if (e == cudaSuccess) e = d_usw.val.resize(usw.col.size());
+    if (e == cudaSuccess) e = d_rec.resize(std::max(nm, 1));
+    if (e == cudaSuccess && !gk::bbd_shared_fits(max_block))
+      e = d_scratch.resize((size_t)gk::bbd_scratch_warps() * ((max_block + 2) & ~1));
     if (e == cudaSuccess) e = d_S.resize(std::max<size_t>((size_t)bs * bs, 1));
     if (e == cudaSuccess) e = d_xT.resize(std::max(bs, 1));
     if (e == cudaSuccess) e = d_z.resize(std::max(nm, 1));
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(GPUKLU_CUDA_ERROR, cuda_msg(e, "bbd tiles"));
     gk::BbdArgs& a = args;
-    a.ntiles = ntiles;
     a.bs = bs;
     a.border_start = d.border_start;
-    a.tile_pos0 = d_tile_pos0.p;
-    a.tile_size = d_tile_size.p;
-    a.tile_off = d_tile_off.p;
-    a.tile_blk = d_tile_blk.p;
-    a.init_ptr = d_init_ptr.p;
-    a.init_code = d_init_code.p;
-    a.init_raw = d_init_raw.p;
+    a.max_block = max_block;
+    auto tasks = [](const TaskDev& t, int count) {
+      return gk::BbdTasks{count, t.blk.p, t.ptr.p, t.reach.p, t.init_ptr.p, t.init_pos.p, t.init_raw.p,
+                          t.order.p};
+    };
+    a.w = tasks(d_wt, (int)wt.blk.size());
+    a.z = tasks(d_zt, (int)zt.blk.size());
+    a.grp_ptr = d_grp_ptr.p;
+    a.grp_len = d_grp_len.p;
+    a.grp_base = d_grp_base.p;
+    a.zout = d_zout.p;
+    a.zpos = d_zpos.p;
+    a.row_ptr = d_row_ptr.p;
+    a.row = d_row.p;
+    a.goff = d_goff.p;
+    a.wref_ptr = d_wref_ptr.p;
     a.bt_ptr = d_bt_ptr.p;
     a.bt_row = d_bt_row.p;
+    a.bt_ent = d_bt_ent.p;
     a.bt_raw = d_bt_raw.p;
-    a.yref_ptr = d_yref_ptr.p;
-    a.yref = d_yref.p;
-    a.c_ptr = d_c_ptr.p;
-    a.c_row = d_c_row.p;
-    a.c_pos = d_c_pos.p;
-    a.c_raw = d_c_raw.p;
     a.crow_ptr = d_crow_ptr.p;
     a.crow_col = d_crow_col.p;
     a.crow_raw = d_crow_raw.p;
     a.rrow_ptr = d_rrow_ptr.p;
     a.rrow_col = d_rrow_col.p;
     a.rrow_raw = d_rrow_raw.p;
+    a.zval = d_zval.p;
+    a.gbuf = d_gbuf.p;
+    auto sweep = [](const SweepDev& w, size_t nnz) {
+      return gk::BbdSweep{w.lvl_ptr.p, w.lv.p, w.row.p, w.ptr.p, w.col.p, w.slot.p, w.at.p, w.val.p, (int)nnz};
+    };
+    a.l = sweep(d_lsw, lsw.col.size());
+    a.u = sweep(d_usw, usw.col.size());
+    a.rec = d_rec.p;
+    a.scratch = d_scratch.p;
     a.perm = d_perm.p;
     a.bperm = d_bperm.p;
     tiles_ready = true;
@@ -4188,8 +4416,10 @@ struct gpuklu_bbd {
       st = build_tiles();
       if (st) return st;
     }
-    gk::launch_bbd_ysolve(M->pd.dp, M->d_lu.p, d_ax.p, args, d_y.p, s);
-    gk::launch_bbd_schur(d_ax.p, args, d_y.p, d_S.p, s);
+    gk::launch_bbd_z(M->pd.dp, M->d_lu.p, d_ax.p, args, s);
+    for (size_t i = 0; i + 1 < cuts.size(); ++i)
+      gk::launch_bbd_schur(M->pd.dp, M->d_lu.p, d_ax.p, args, cuts[i].first, cuts[i + 1].first,
+                           cuts[i].second, cuts[i + 1].second, d_S.p, s);
     cudaError_t e = cudaSuccess;
     if (schur_lu == 0) {
       gk::launch_dense_lu(d_S.p, d.border_size, s);
@@ -4209,6 +4439,21 @@ struct gpuklu_bbd {
     return GPUKLU_OK;
   }
 
+  // out = M^-1 M->d_rhs, M's order. Blocks whose vector and lists one thread block
+  // does not hold in shared memory (11.5 k rows) take M's own solve.
+  int solve_blocks(double* out) {
+    if (gk::bbd_solve_fits(args.max_block)) {
+      gk::launch_bbd_solve(M->pd.dp, args, M->d_rhs.p, out, stream());
+      return GPUKLU_OK;
+    }
+    const int st = M->solve_on_device(false, false);
+    if (st) return fail(st, M->err);
+    if (out != M->d_out.p)
+      cudaMemcpyAsync(out, M->d_out.p, (size_t)d.border_start * 8, cudaMemcpyDeviceToDevice,
+                      stream());
+    return GPUKLU_OK;
+  }
+
   // x = A^-1 rhs, both full-length device arrays (original order).
   int solve_device(const double* rhs, double* x) {
     cudaStream_t s = stream();
@@ -4223,14 +4468,13 @@ struct gpuklu_bbd {
     }
     const int nm = d.border_start;
     gk::launch_gather(M->d_rhs.p, rhs, d_perm.p, nm, s);  // block rows
-    int st = M->solve_on_device(false, false);
-    if (st) return fail(st, M->err);
-    cudaMemcpyAsync(d_z.p, M->d_out.p, (size_t)nm * 8, cudaMemcpyDeviceToDevice, s);
+    int st = solve_blocks(d_z.p);
+    if (st) return st;
     gk::launch_bbd_border_rhs(d_ax.p, rhs, d_z.p, args, d_xT.p, s);
     gk::launch_dense_lu_solve(d_S.p, d.border_size, d_xT.p, s);
     gk::launch_bbd_rmatvec(d_ax.p, d_xT.p, args, M->d_rhs.p, s);
-    st = M->solve_on_device(false, false);
-    if (st) return fail(st, M->err);
+    st = solve_blocks(M->d_out.p);
+    if (st) return st;
     gk::launch_bbd_combine(d_z.p, M->d_out.p, d_xT.p, args, x, s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(GPUKLU_CUDA_ERROR, cuda_msg(e, "bbd solve"));

@@ -36,6 +36,7 @@ inline size_t solve_steps_bytes(int n, int chunk) {
 struct DPlan {
   int n, nslots, nblocks, ntask;
   int max_col;  // slots of the longest column
+  const int* order;  // columns by the length of the chain that waits for them
   const int *col_ptr, *dslot, *slot_row, *upd_ptr, *upd_dst, *col_single;
   const int *amap_ptr, *amap_idx;
   const int *offd_ptr, *offd_col, *offd_raw;
@@ -78,6 +79,9 @@ struct NewtonCfg {
 struct NewtonState {
   double damping, prev_dx_norm, last_norm;
   int converged, iter;
+  unsigned ticket = 0;  // k_newton_norm: blocks done, their sums and tests
+  int pflag[32];
+  double part[32];
 };
 
 // Batched program of one group: circuits whose device lists, analysis and
@@ -228,21 +232,46 @@ struct AtranArgs {
 };
 
 // Bordered-block-diagonal solver: the index lists its kernels read.
+// The sparse triangular solves around the border: task t is one border column
+// (W = L^-1 R) or row (Z = U^-T C^T) of one block. Its solution is non-zero on
+// the plan positions reach[ptr[t] .. ptr[t + 1]), ascending.
+struct BbdTasks {
+  int n;
+  const int* blk;                              // the task's plan block
+  const long long* ptr;
+  const int *reach, *init_ptr, *init_pos, *init_raw;  // right-hand side: position in the block, raw
+  const int* order;                            // tasks as they start, the longest first
+};
+// A triangular factor by rows, the rows of a block by level: rows lv[q] to
+// lv[q + 1] for q from lvl_ptr[block] on need only rows before them. Row i is
+// position row[i] of its block and has entries [ptr[i], ptr[i + 1]).
+struct BbdSweep {
+  const int *lvl_ptr, *lv, *row, *ptr, *col, *slot;
+  const int* at;                               // a plan position's row (U only)
+  double* val;
+  int nnz;
+};
 struct BbdArgs {
-  int ntiles, bs, border_start;
-  const int* tile_pos0;        // first plan position of the tile's block
-  const int* tile_size;        // block size
-  const long long* tile_off;   // offset of the tile's [size][32] array
-  const int* tile_blk;         // plan block of the tile
-  const int *init_ptr, *init_code, *init_raw;  // R entries: (row offset * 32 + lane, raw)
+  int bs, border_start, max_block;
   // border indices below are Schur positions (the elimination order of S)
-  const int *bt_ptr, *bt_row, *bt_raw;         // B_T by Schur column
-  const int *yref_ptr, *yref;                  // per border column: (tile << 5 | lane)
-  const int *c_ptr, *c_row, *c_pos, *c_raw;    // C by plan block: (border row, row offset of Y, raw)
+  BbdTasks w, z;                               // w: by border column, its blocks ascending
+  // Z by block in groups of 32 border rows, one row per lane: entry k of lane l
+  // at grp_base + 32 k + l, zpos its position in the block (padding: the size).
+  const int *grp_ptr, *grp_len;                // groups of a block; entries of a group
+  const long long *grp_base, *zout;            // a group's first entry; a Z task's
+  const int* zpos;
+  const int *row_ptr, *row;                    // border rows of a block
+  const long long* goff;                       // a W task's products Z^T W in gbuf
+  const int* wref_ptr;                         // W tasks by border column
+  const int *bt_ptr, *bt_row, *bt_ent, *bt_raw;  // B_T by Schur column: rows, their entries
   const int *crow_ptr, *crow_col, *crow_raw;   // C by border row: (block column, raw)
   const int *rrow_ptr, *rrow_col, *rrow_raw;   // R by block row: (border column, raw)
   const int* perm;                             // bordered order -> original index
   const int* bperm;                            // Schur position -> original index
+  double *zval, *gbuf;                         // Z, Z^T W
+  BbdSweep l, u;
+  double* rec;                                 // the pivots' reciprocals
+  double* scratch;                             // vectors of blocks too large for shared memory
 };
 
 // AC sweep: the dense cells of Y(w) = G + jwC and the per-frequency solve.
@@ -342,10 +371,18 @@ void launch_batch_lanes(const BatchArgs& a, int grid, int warps_per_block, cudaS
 void lanes_kernel_info(int warps_per_block, int* regs, int* blocks_per_sm);
 
 // Bordered-block-diagonal solver pieces.
-void launch_bbd_ysolve(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B,
-                       double* ybuf, cudaStream_t s);
-void launch_bbd_schur(const double* ax, const BbdArgs& B, const double* ybuf, double* S,
+bool bbd_shared_fits(int max_block);
+int bbd_scratch_warps();  // vectors of `scratch` when it does not
+// Z and what it needs, then for border columns [j0, j1) their W tasks [t0, t1)
+// with the products and the columns of S.
+void launch_bbd_z(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B,
+                  cudaStream_t s);
+// out = M^-1 rhs (M's order), every block's vector and lists in shared memory.
+bool bbd_solve_fits(int max_block);
+void launch_bbd_solve(const DPlan& P, const BbdArgs& B, const double* rhs, double* out,
                       cudaStream_t s);
+void launch_bbd_schur(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B, int j0,
+                      int j1, int t0, int t1, double* S, cudaStream_t s);
 void launch_dense_lu(double* S, int bs, cudaStream_t s);
 // The same factorization as one cooperative launch (schur.cu): FP64 FMA
 // updates (mma = false) or DMMA updates; both agree with launch_dense_lu's
