@@ -543,6 +543,31 @@ std::vector<i32> column_order(const gk::Plan& p) {
   return out;
 }
 
+// What a handle's Newton loop reads back: the heads of two iterations' states, in
+// pinned memory, and the events behind them.
+struct NewtonLoop {
+  static constexpr size_t kHead = offsetof(gk::NewtonState, ticket);
+  unsigned char* host = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  NewtonLoop() = default;
+  NewtonLoop(const NewtonLoop&) = delete;
+  NewtonLoop& operator=(const NewtonLoop&) = delete;
+  ~NewtonLoop() {
+    if (host) cudaFreeHost(host);
+    for (cudaEvent_t ev : done)
+      if (ev) cudaEventDestroy(ev);
+  }
+  cudaError_t open() {
+    cudaError_t e = cudaSuccess;
+    if (!host) e = cudaHostAlloc((void**)&host, 256, cudaHostAllocDefault);
+    for (cudaEvent_t& ev : done)
+      if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    return e;
+  }
+  void* slot(int64_t k) { return host + 128 * (k & 1); }
+};
+static_assert(NewtonLoop::kHead <= 128, "a state's head fits its slot");
+
 // Device copy of a SolveProgram.
 struct SolveDev {
   DBuf<int4> ops, chunks, chains;
@@ -907,6 +932,7 @@ struct gpuklu_handle {
   DBuf<double> d_big;  // columns too long for shared memory while they are updated
   DBuf<int> d_rperm, d_rinv, d_status;
   DBuf<gk::NewtonState> d_nstate;
+  NewtonLoop loop;
   unsigned sepoch = 0;
   int64_t factor_count = 0, refactor_count = 0;
   bool cta_ref = false, cta_sol = false;  // one-block refactor / solve for this plan
@@ -1805,6 +1831,11 @@ int dc_newton_run(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_confi
   nc_.gmin = cfg->gmin;
   nc_.damping = cfg->damping;
   nc_.damping_min = cfg->damping_min;
+  nc_.stop_nonfinite = h->stop_nonfinite;
+  NewtonLoop& loop = h->loop;
+  e = loop.open();
+  if (e != cudaSuccess) return h->cuda_fail(e, "newton loop");
+  const int* const skip_flag = (const int*)((const char*)h->d_nstate.p + offsetof(gk::NewtonState, stop));
   const double gstart = std::max(cfg->gmin * 1e3, 1e-6);
   int64_t total = 0, last_iters = 0;
   int rsn = 1, ret = GPUKLU_OK;
@@ -1819,13 +1850,32 @@ int dc_newton_run(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_confi
       gk::NewtonState ns{cfg->damping, DBL_MAX, 0.0, 0, 0};
       e = cudaMemcpyAsync(h->d_nstate.p, &ns, sizeof(ns), cudaMemcpyHostToDevice, h->stream);
       if (e != cudaSuccess) return h->cuda_fail(e, "newton state");
-      int64_t it = 0;
+      int64_t it = 0, launched = 0;
       rsn = 1;
-      for (; it < cfg->max_iters; ++it) {
-        gk::launch_stamp(c->dc, h->d_newx.p, nc, gmin, scale, 0.0, nullptr, -1.0, h->d_ax.p,
+      // Iteration k: stamp, factor, solve, update, the state's head into slot k & 1.
+      auto launch = [&](int64_t k, const int* skip) -> int {
+        gk::DCircuit dc = c->dc;
+        dc.skip = skip;
+        gk::launch_stamp(dc, h->d_newx.p, nc, gmin, scale, 0.0, nullptr, -1.0, h->d_ax.p,
                          h->d_rhs_c.p, h->d_rhs.p, h->stream);
-        st = h->factor_on_device(h->state != gpuklu_handle::FACTORED);
-        if (st == GPUKLU_OK) st = h->solve_on_device(false, false);
+        h->pd.dp.skip = skip;
+        int s = h->factor_on_device(h->state != gpuklu_handle::FACTORED);
+        if (s == GPUKLU_OK) s = h->solve_on_device(false, false);
+        h->pd.dp.skip = nullptr;
+        if (s != GPUKLU_OK) return s;
+        gk::launch_newton_update(m, n, h->d_newx.p, h->d_out.p, h->d_nstate.p, nc_,
+                                 h->d_status.p, h->stream);
+        cudaMemcpyAsync(loop.slot(k), h->d_nstate.p, NewtonLoop::kHead, cudaMemcpyDeviceToHost,
+                        h->stream);
+        cudaEventRecord(loop.done[k & 1], h->stream);
+        return GPUKLU_OK;
+      };
+      for (; it < cfg->max_iters; ++it) {
+        st = GPUKLU_OK;
+        if (launched == it) {
+          st = launch(it, nullptr);
+          ++launched;
+        }
         if (st != GPUKLU_OK) {
           if (st == GPUKLU_DEVICE_TIMEOUT) ret = st;
           rsn = 2;
@@ -1833,17 +1883,24 @@ int dc_newton_run(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_confi
           ++it;
           break;
         }
-        gk::launch_newton_update(m, n, h->d_newx.p, h->d_out.p, h->d_nstate.p, nc_,
-                                 h->d_status.p, h->stream);
-        gk::NewtonState hs;
-        int dst = 0;
-        e = cudaMemcpyAsync(&hs, h->d_nstate.p, sizeof(hs), cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(&dst, h->d_status.p, sizeof(int), cudaMemcpyDeviceToHost,
-                              h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        // The next iteration is launched while this one runs; its kernels do
+        // nothing when this one ends the loop (NewtonState::stop). Factorizations
+        // that read back on their own take their turn instead.
+        const bool ahead = it + 1 < cfg->max_iters && h->kind != GPUKLU_KIND_DENSE && !h->repivot &&
+                           h->state == gpuklu_handle::FACTORED;
+        if (ahead) {
+          const int s = launch(it + 1, skip_flag);
+          ++launched;
+          if (s != GPUKLU_OK) return s;  // (nothing that reads back: a launch does not fail)
+        }
+        e = cudaEventSynchronize(loop.done[it & 1]);
+        if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return h->cuda_fail(e, "newton step");
-        if (dst == GPUKLU_DEVICE_TIMEOUT) {
+        gk::NewtonState hs;
+        memcpy(&hs, loop.slot(it), NewtonLoop::kHead);
+        if (hs.stop && ahead && launched > it + 1) --h->refactor_count;  // it did not run
+        if (hs.status == GPUKLU_DEVICE_TIMEOUT) {
+          cudaStreamSynchronize(h->stream);
           cudaMemset(h->d_status.p, 0, sizeof(int));
           h->err = "device dependency wait timed out";
           ret = GPUKLU_DEVICE_TIMEOUT;
@@ -1852,8 +1909,7 @@ int dc_newton_run(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_confi
           ++it;
           break;
         }
-        if (dst) cudaMemset(h->d_status.p, 0, sizeof(int));
-        if (dst == GPUKLU_NONFINITE && h->stop_nonfinite) {
+        if (hs.nonfinite && h->stop_nonfinite) {
           h->err = "non-finite Newton iterate at iteration " + std::to_string(it + 1);
           ret = GPUKLU_NONFINITE;
           rsn = 2;

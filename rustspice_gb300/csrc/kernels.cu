@@ -820,9 +820,17 @@ __device__ __forceinline__ bool grid_updates(const DPlan& P, double* C, const do
   }
 }
 
+__global__ void k_preset(double* lu, long long n, const int* skip) {
+  if (__ldcg(skip) != 0) return;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
+    lu[i] = __longlong_as_double(-1ll);
+}
+
 __global__ void __launch_bounds__(64 * kPairs) k_refactor(DPlan P, const double* __restrict__ ax,
                                                           double* lu, double* big, int colcap,
                                                           int* status, PivotCheck pc) {
+  if (P.skip != nullptr && __ldcg(P.skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bars[kPairs][2 * kGridRing];
   __shared__ int dead_flag[kPairs];
@@ -921,6 +929,7 @@ __global__ void k_solve(DPlan P, const double* __restrict__ rhs, const double* _
                         const double* __restrict__ lu, double* z, double* x, double* out,
                         unsigned* zflag, unsigned* xflag, unsigned epoch, unsigned* counter,
                         int* status) {
+  if (P.skip != nullptr && __ldcg(P.skip) != 0) return;
   const int lane = threadIdx.x & 31;
   while (true) {
     int t = 0;
@@ -1030,6 +1039,7 @@ __global__ void k_tsolve(DPlan P, const double* __restrict__ g, const double* __
 __global__ void __launch_bounds__(1024) k_refactor_cta(DPlan P, const double* __restrict__ ax,
                                                        double* lu_out, int* status,
                                                        PivotCheck pc) {
+  if (P.skip != nullptr && __ldcg(P.skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* const lu = reinterpret_cast<double*>(smem_raw);
   unsigned char* const rings = smem_raw + (((size_t)8 * P.nslots + 15) & ~(size_t)15);
@@ -1096,6 +1106,7 @@ __global__ void __launch_bounds__(256) k_solve_cta(DPlan P, const double* __rest
                                                    const double* __restrict__ ax,
                                                    const double* __restrict__ lu, double* out,
                                                    int chunk, int grouped) {
+  if (P.skip != nullptr && __ldcg(P.skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31;
   int r0 = 0, r1 = P.n, c0 = 0, c1 = P.cs_nchunk;
@@ -1276,7 +1287,8 @@ __global__ void __launch_bounds__(kSolveStepsThreads)
     k_solve_steps(SolveSched S, int n, const int* __restrict__ in, const int* __restrict__ outp,
                   const int* __restrict__ dslot, const double* __restrict__ rhs,
                   const double* __restrict__ ax, const double* __restrict__ lu, double* rec,
-                  double* out) {
+                  double* out, const int* skip) {
+  if (skip != nullptr && __ldcg(skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* const T = reinterpret_cast<double*>(smem_raw);  // the solution, a spare entry at n
   double2* const svc = reinterpret_cast<double2*>(T + ((n + 2) & ~1));  // (v, c) of every slot
@@ -1626,6 +1638,7 @@ __device__ __forceinline__ int eval_device(int type, const int* nd, const double
 __global__ void k_stamp(DCircuit C, const double* __restrict__ x, int xlen, double gmin,
                         double scale, double dt, const double* __restrict__ cap_v,
                         double be_sign, double* ax, double* rhs_c, double gdev) {
+  if (C.skip != nullptr && __ldcg(C.skip) != 0) return;
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d == 0 && C.pin_raw >= 0) ax[C.pin_raw] = 1.0;
   if (d >= C.ndev) return;
@@ -1721,6 +1734,7 @@ __global__ void k_param_grad(DCircuit C, const double* __restrict__ x, int xlen,
 }
 
 __global__ void k_rhs_sum(DCircuit C, const double* __restrict__ rhs_c, double* rhs) {
+  if (C.skip != nullptr && __ldcg(C.skip) != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= C.n) return;
   double v = 0.0;
@@ -1751,22 +1765,26 @@ __device__ __forceinline__ void newton_reduce(double& acc, int& conv, int& fin) 
 }
 // The state after an update of norm sqrt(acc).
 __device__ __forceinline__ void newton_step(NewtonState* st, const NewtonCfg& cfg, double acc,
-                                            int conv, int fin, int* status) {
+                                            int conv, int fin, const int* status) {
   const double dxn = sqrt(acc);
   st->iter += 1;
   st->converged = conv;
-  if (!fin) atomicCAS(status, DS_OK, DS_NONFINITE);
   if (!conv) {
     if (dxn > st->prev_dx_norm && st->damping > cfg.damping_min)
       st->damping = fmax(st->damping * 0.5, cfg.damping_min);
     st->prev_dx_norm = dxn;
   }
+  const int code = *(volatile const int*)status;
+  st->nonfinite = !fin;
+  st->status = code;
+  st->stop = conv || code != DS_OK || (!fin && cfg.stop_nonfinite);
 }
 
 __global__ void __launch_bounds__(1024) k_newton_update(int m, int n, double* x,
                                                         const double* __restrict__ xn,
                                                         NewtonState* st, NewtonCfg cfg,
-                                                        int* status) {
+                                                        const int* status) {
+  if (st->stop) return;  // launched before the last iteration was known to be that
   __shared__ double ssum[32];
   __shared__ int sconv[32], sfin[32];
   const int tid = threadIdx.x;
@@ -1807,8 +1825,12 @@ __global__ void __launch_bounds__(1024) k_newton_update(int m, int n, double* x,
 // 47 us and 13 us.
 __global__ void __launch_bounds__(32) k_newton_norm(int m, const double* x,
                                                     const double* __restrict__ xn, NewtonState* st,
-                                                    NewtonCfg cfg, int* status) {
+                                                    NewtonCfg cfg, const int* status) {
   const int lane = threadIdx.x;
+  if (__ldcg(&st->stop)) {
+    if (blockIdx.x == 0 && lane == 0) st->apply = 0;
+    return;
+  }
   double acc;
   int conv, fin;
   newton_part(m, x, xn, cfg, blockIdx.x * 32 + lane, acc, conv, fin);
@@ -1829,12 +1851,14 @@ __global__ void __launch_bounds__(32) k_newton_norm(int m, const double* x,
   newton_reduce(acc, conv, fin);
   if (lane == 0) {
     newton_step(st, cfg, acc, conv, fin, status);
+    st->apply = 1;
     st->ticket = 0;
   }
 }
 __global__ void k_newton_apply(int m, int n, double* x, const double* __restrict__ xn,
                                const NewtonState* st) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (!st->apply) return;
   if (st->converged) {
     if (i < n) x[i] = xn[i];
   } else if (i < m) {
@@ -2131,7 +2155,11 @@ void launch_first_factor(const DPlan& P, int maxblk, const double* ax, double* l
 
 void launch_refactor(const DPlan& P, const double* ax, double* lu, double* big, int* status,
                      int grid, cudaStream_t s, const PivotCheck& pc) {
-  cudaMemsetAsync(lu, 0xff, ((size_t)P.nslots + kLuPad) * sizeof(double), s);
+  const long long words = (long long)P.nslots + kLuPad;
+  if (P.skip != nullptr)
+    k_preset<<<(int)std::min<long long>((words + 1023) / 1024, 4096), 256, 0, s>>>(lu, words, P.skip);
+  else
+    cudaMemsetAsync(lu, 0xff, (size_t)words * sizeof(double), s);
   const int colcap = std::min((P.max_col + 1) & ~1, kColCap);
   const int bytes = kPairs * (kGridRing * kGridStage + 8 * colcap);
   cudaFuncSetAttribute(k_refactor, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -2195,7 +2223,7 @@ void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const
     cudaFuncSetAttribute(k_solve_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   k_solve_steps<<<1, kSolveStepsThreads, bytes, s>>>(
       P.ss, P.n, transpose ? P.out_col : P.in_row, transpose ? P.in_row : P.out_col, P.dslot, rhs,
-      ax, lu, rec, out);
+      ax, lu, rec, out, P.skip);
 }
 
 bool solve_groups_fit(const DPlan& P) {

@@ -57,6 +57,10 @@ struct DPlan {
   // Polls of a dependency flag before a waiting warp gives up and reports
   // DS_TIMEOUT (kSpinLimit unless the handle sets another).
   unsigned spin_limit;
+  // When set, the refactorization and solve kernels do nothing while *skip is not
+  // zero (a Newton iteration launched before the one ahead of it was known to end
+  // the loop).
+  const int* skip;
 };
 
 // Device form of a compiled circuit (device list + stamp-to-slot map).
@@ -68,17 +72,21 @@ struct DCircuit {
   const int* raw;       // [ndev*8] raw CSC index of each matrix insert, -1 none
   const int* rhs_slot;  // [ndev*2] index into the rhs contribution buffer, -1 none
   const int *rhs_ptr, *rhs_src;  // per row: contributions in stamping order
+  const int* skip;      // as DPlan::skip, for the stamping
 };
 
 struct NewtonCfg {
   int max_iters, gmin_steps;
   double abs_tol, rel_tol, gmin, damping, damping_min;
+  int stop_nonfinite;  // a non-finite iterate ends the loop (NewtonState::stop)
 };
 
 // Per-handle Newton state kept on the device between iterations.
 struct NewtonState {
   double damping, prev_dx_norm, last_norm;
   int converged, iter;
+  int stop, nonfinite, status;  // the loop is over; the iterate; the status word
+  int apply;                    // k_newton_norm ran: k_newton_apply does
   unsigned ticket = 0;  // k_newton_norm: blocks done, their sums and tests
   int pflag[32];
   double part[32];
