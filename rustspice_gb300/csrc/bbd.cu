@@ -120,19 +120,99 @@ __device__ __forceinline__ void sweep_block(const BbdSweep& S, int blk, int sz, 
   }
 }
 
-// A thread block per block of M: forward and backward substitution by levels.
-// Bounded by the levels' latency (about 150 levels of 50 x 50 meshes each way:
-// the entries' products, the sum across the warp and a barrier). Measured, 64
-// meshes of 30-50 a side: 0.61 ms against 1.43 ms for a warp per block that
-// takes the columns one after another.
-__global__ void __launch_bounds__(kSweepThreads) k_bbd_solve(DPlan P, BbdArgs B,
-                                                    const double* __restrict__ rhs, double* out) {
+// A thread block per block of M. With W and Z of the factorization at hand a solve
+// takes each triangle once: forward y = L^-1 P b and Z^T y = C M^-1 b, and when the
+// border's solution x is known, backward U^-1 (y - W x). Bounded by the levels'
+// latency (the entries' products, the sum across the warp and a barrier). Measured,
+// 64 meshes of 30-50 a side: 0.34 and 0.39 ms against 0.61 ms for both triangles at once,
+// twice per solve, and 1.43 ms for a warp per block that takes the columns one after
+// another, twice.
+__global__ void __launch_bounds__(kSweepThreads) k_bbd_forward(DPlan P, BbdArgs B,
+                                                               const double* __restrict__ rhs) {
   extern __shared__ double v[];
   const int blk = blockIdx.x, p0 = P.block_ptr[blk], sz = P.block_ptr[blk + 1] - p0;
-  for (int i = threadIdx.x; i < sz; i += blockDim.x) v[i] = rhs[P.in_row[p0 + i]];
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < sz; i += blockDim.x) v[i] = rhs[B.perm[P.in_row[p0 + i]]];
   sweep_block(B.l, blk, sz, nullptr, v);
+  __syncthreads();
+  for (int i = tid; i < sz; i += blockDim.x) B.y[p0 + i] = v[i];
+  const int r0 = B.row_ptr[blk], nrow = B.row_ptr[blk + 1] - r0;
+  const int g0 = B.grp_ptr[blk], g1 = B.grp_ptr[blk + 1];
+  for (int g = g0 + (tid >> 5); g < g1; g += blockDim.x >> 5) {
+    const int* const zi = B.zpos + B.grp_base[g] + lane;
+    const double* const zv = B.zval + B.grp_base[g] + lane;
+    double acc = 0.0;
+    for (int k = 0; k < B.grp_len[g]; k += 8) {  // a multiple of 8
+      int ix[8];
+      double zz[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        ix[u] = zi[(k + u) * 32];
+        zz[u] = zv[(k + u) * 32];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (ix[u] < sz) acc = fma(zz[u], v[ix[u]], acc);  // (the padding's position is sz)
+    }
+    const int r = (g - g0) * 32 + lane;
+    if (r < nrow) B.zdot[r0 + r] = acc;
+  }
+}
+
+// bb[j] = rhs[border row j] - the blocks' parts of C M^-1 b, in block order.
+__global__ void k_bbd_border(BbdArgs B, const double* __restrict__ rhs, double* bb) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= B.bs) return;
+  double v = rhs[B.bperm[j]];
+  for (int e = B.zref_ptr[j]; e < B.zref_ptr[j + 1]; ++e) v -= B.zdot[B.zref[e]];
+  bb[j] = v;
+}
+
+__global__ void __launch_bounds__(kSweepThreads) k_bbd_backward(DPlan P, BbdArgs B,
+                                                                const double* __restrict__ xT,
+                                                                double* x) {
+  extern __shared__ double v[];
+  const int blk = blockIdx.x, p0 = P.block_ptr[blk], sz = P.block_ptr[blk + 1] - p0;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < sz; i += blockDim.x) v[i] = B.y[p0 + i];
+  __syncthreads();
+  // v -= W x, a border column after the other; the next one's first entries are
+  // read while this one is subtracted
+  const int q1 = B.bw_ptr[blk + 1];
+  int nc = -1;
+  double nw = 0.0, nx = 0.0;
+  long long na = 0;
+  int nlen = 0;
+  auto ahead = [&](int q) {
+    nc = -1;
+    if (q >= q1) return;
+    const int t = B.bw[q];
+    na = B.w.ptr[t];
+    nlen = (int)(B.w.ptr[t + 1] - na);
+    nx = xT[B.wcol[t]];
+    if (tid < nlen) {
+      nc = B.w.reach[na + tid] - p0;
+      nw = B.wval[na + tid];
+    }
+  };
+  ahead(B.bw_ptr[blk]);
+  for (int q = B.bw_ptr[blk]; q < q1; ++q) {
+    const int c = nc, len = nlen;
+    const double w = nw, xj = nx;
+    const long long a = na;
+    ahead(q + 1);
+    if (c >= 0) v[c] = fma(-w, xj, v[c]);
+    for (int i = tid + blockDim.x; i < len; i += blockDim.x) {
+      const int r = B.w.reach[a + i] - p0;
+      v[r] = fma(-B.wval[a + i], xj, v[r]);
+    }
+    __syncthreads();
+  }
   sweep_block(B.u, blk, sz, B.rec + p0, v);
-  for (int i = threadIdx.x; i < sz; i += blockDim.x) out[P.out_col[p0 + i]] = v[i];
+  __syncthreads();
+  for (int i = tid; i < sz; i += blockDim.x) x[B.perm[P.out_col[p0 + i]]] = v[i];
+  for (int i = blk * blockDim.x + tid; i < B.bs; i += gridDim.x * blockDim.x)
+    x[B.bperm[i]] = xT[i];
 }
 
 // kRows: Z, by rows of U; else W, by columns of L, and its products with Z.
@@ -162,7 +242,7 @@ __global__ void k_bbd_reach(DPlan P, const double* __restrict__ lu,
     __syncwarp();
     const int* const reach = T.reach + T.ptr[t];
     const int len = (int)(T.ptr[t + 1] - T.ptr[t]);
-    double* const out = kRows ? B.zval + B.zout[t] : nullptr;
+    double* const out = kRows ? B.zval + B.zout[t] : B.wval + T.ptr[t];
     for (int c0 = 0; c0 < len; c0 += 32) {  // the ranges of 32 steps, one per lane
       int c = 0, qa = 0, qb = 0;
       double rc = 1.0;
@@ -197,7 +277,7 @@ __global__ void k_bbd_reach(DPlan P, const double* __restrict__ lu,
         if (i + 1 < cnt) fetch(i + 1);
         double x = v[__shfl_sync(FULL, c, i) - p0];
         if (kRows) x *= __shfl_sync(FULL, rc, i);
-        if (kRows && lane == 0) out[(long long)(c0 + i) * 32] = x;
+        if (lane == 0) out[(long long)(c0 + i) * (kRows ? 32 : 1)] = x;
         if (a + lane < b) v[i0] = fma(-l0, x, v[i0]);
         if (a + 32 + lane < b) v[i1] = fma(-l1, x, v[i1]);
         for (int q = a + 64 + lane; q < b; q += 32) {
@@ -538,11 +618,19 @@ void launch_bbd_z(const DPlan& P, const double* lu, const double* ax, const BbdA
   launch_reach<true>(P, lu, ax, B, 0, B.z.n, s);
 }
 
-void launch_bbd_solve(const DPlan& P, const BbdArgs& B, const double* rhs, double* out,
-                      cudaStream_t s) {
+void launch_bbd_forward(const DPlan& P, const BbdArgs& B, const double* rhs, double* bb,
+                        cudaStream_t s) {
   const int bytes = (int)bbd_solve_bytes(B.max_block);
-  cudaFuncSetAttribute(k_bbd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  k_bbd_solve<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, rhs, out);
+  cudaFuncSetAttribute(k_bbd_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_bbd_forward<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, rhs);
+  k_bbd_border<<<cdiv(B.bs, 128), 128, 0, s>>>(B, rhs, bb);
+}
+
+void launch_bbd_backward(const DPlan& P, const BbdArgs& B, const double* xT, double* x,
+                         cudaStream_t s) {
+  const int bytes = (int)bbd_solve_bytes(B.max_block);
+  cudaFuncSetAttribute(k_bbd_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_bbd_backward<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, xT, x);
 }
 
 void launch_bbd_schur(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B, int j0,

@@ -4004,7 +4004,7 @@ struct gpuklu_bbd {
   std::vector<i32> perm32;
   DBuf<i32> d_m_raw, d_perm, d_bt_ptr, d_bt_row, d_bt_ent, d_bt_raw, d_crow_ptr, d_crow_col, d_crow_raw,
       d_rrow_ptr, d_rrow_col, d_rrow_raw, d_bperm, d_grp_ptr, d_grp_len, d_zpos, d_row_ptr, d_row,
-      d_wref_ptr;
+      d_wref_ptr, d_zref_ptr, d_zref, d_bw_ptr, d_bw, d_wcol;
   DBuf<long long> d_grp_base, d_zout, d_goff;
   struct TaskDev {
     DBuf<i32> blk, reach, init_ptr, init_pos, init_raw, order;
@@ -4015,7 +4015,7 @@ struct gpuklu_bbd {
     DBuf<double> val;
   } d_lsw, d_usw;
   DBuf<double> d_ax, d_rhs, d_rhs_c, d_x, d_newx, d_S, d_xT, d_z;
-  DBuf<double> d_zval, d_gbuf, d_rec, d_scratch;
+  DBuf<double> d_zval, d_wval, d_gbuf, d_rec, d_scratch, d_zdot;
   // border columns [cut[i].first, cut[i + 1].first) share gbuf, cut[i].second
   // their first W task
   std::vector<std::pair<int, int>> cuts;
@@ -4296,6 +4296,19 @@ struct gpuklu_bbd {
       }
     }
     cuts.push_back({bs, (int)wt.blk.size()});
+    // border rows' places in `row`; W tasks by block and their border columns
+    std::vector<i32> zref_ptr(bs + 1, 0), zref(row.size()), bw_ptr(nb + 1, 0), bw(wt.blk.size()), wcol;
+    for (i32 r : row) ++zref_ptr[r + 1];
+    for (int r = 0; r < bs; ++r) zref_ptr[r + 1] += zref_ptr[r];
+    for (i32 b : wt.blk) ++bw_ptr[b + 1];
+    for (int b = 0; b < nb; ++b) bw_ptr[b + 1] += bw_ptr[b];
+    {
+      std::vector<i32> at(zref_ptr.begin(), zref_ptr.end());
+      for (size_t i = 0; i < row.size(); ++i) zref[at[row[i]]++] = (i32)i;
+      at.assign(bw_ptr.begin(), bw_ptr.end());
+      for (size_t t = 0; t < wt.blk.size(); ++t) bw[at[wt.blk[t]]++] = (i32)t;
+      for (int j = 0; j < bs; ++j) wcol.insert(wcol.end(), wref_ptr[j + 1] - wref_ptr[j], j);
+    }
     long long products = 1;
     for (size_t i = 0; i + 1 < cuts.size(); ++i)
       products = std::max(products, goff[cuts[i + 1].second] - goff[cuts[i].second]);
@@ -4384,7 +4397,8 @@ struct gpuklu_bbd {
     UP(d_rrow_ptr, rrow_ptr) UP(d_rrow_col, rrow_col) UP(d_rrow_raw, rrow_raw) UP(d_bperm, bperm)
     UP(d_grp_ptr, grp_ptr) UP(d_grp_len, grp_len) UP(d_grp_base, grp_base) UP(d_zout, zout)
     UP(d_zpos, zpos) UP(d_row_ptr, row_ptr) UP(d_row, row) UP(d_goff, goff)
-    UP(d_wref_ptr, wref_ptr)
+    UP(d_wref_ptr, wref_ptr) UP(d_zref_ptr, zref_ptr) UP(d_zref, zref) UP(d_bw_ptr, bw_ptr)
+    UP(d_bw, bw) UP(d_wcol, wcol)
     UP(d_wt.blk, wt.blk) UP(d_wt.ptr, wt.ptr) UP(d_wt.reach, wt.reach)
     UP(d_wt.init_ptr, wt.init_ptr) UP(d_wt.init_pos, wt.init_pos) UP(d_wt.init_raw, wt.init_raw)
     UP(d_zt.blk, zt.blk) UP(d_zt.ptr, zt.ptr) UP(d_zt.reach, zt.reach)
@@ -4399,6 +4413,8 @@ struct gpuklu_bbd {
     if (e == cudaSuccess)  // the padding stays zero
       e = cudaMemsetAsync(d_zval.p, 0, std::max<size_t>(zpos.size(), 1) * sizeof(double), s);
     if (e == cudaSuccess) e = d_gbuf.resize((size_t)products);
+    if (e == cudaSuccess) e = d_wval.resize(wt.reach.size());
+    if (e == cudaSuccess) e = d_zdot.resize(row.size());
     if (e == cudaSuccess) e = d_lsw.val.resize(lsw.col.size());
     if (e == cudaSuccess) e = d_usw.val.resize(usw.col.size());
     if (e == cudaSuccess) e = d_rec.resize(std::max(nm, 1));
@@ -4439,6 +4455,14 @@ struct gpuklu_bbd {
     a.rrow_col = d_rrow_col.p;
     a.rrow_raw = d_rrow_raw.p;
     a.zval = d_zval.p;
+    a.wval = d_wval.p;
+    a.y = d_z.p;
+    a.zdot = d_zdot.p;
+    a.zref_ptr = d_zref_ptr.p;
+    a.zref = d_zref.p;
+    a.bw_ptr = d_bw_ptr.p;
+    a.bw = d_bw.p;
+    a.wcol = d_wcol.p;
     a.gbuf = d_gbuf.p;
     auto sweep = [](const SweepDev& w, size_t nnz) {
       return gk::BbdSweep{w.lvl_ptr.p, w.lv.p, w.row.p, w.ptr.p, w.col.p, w.slot.p, w.at.p, w.val.p, (int)nnz};
@@ -4495,21 +4519,6 @@ struct gpuklu_bbd {
     return GPUKLU_OK;
   }
 
-  // out = M^-1 M->d_rhs, M's order. Blocks whose vector and lists one thread block
-  // does not hold in shared memory (11.5 k rows) take M's own solve.
-  int solve_blocks(double* out) {
-    if (gk::bbd_solve_fits(args.max_block)) {
-      gk::launch_bbd_solve(M->pd.dp, args, M->d_rhs.p, out, stream());
-      return GPUKLU_OK;
-    }
-    const int st = M->solve_on_device(false, false);
-    if (st) return fail(st, M->err);
-    if (out != M->d_out.p)
-      cudaMemcpyAsync(out, M->d_out.p, (size_t)d.border_start * 8, cudaMemcpyDeviceToDevice,
-                      stream());
-    return GPUKLU_OK;
-  }
-
   // x = A^-1 rhs, both full-length device arrays (original order).
   int solve_device(const double* rhs, double* x) {
     cudaStream_t s = stream();
@@ -4523,15 +4532,22 @@ struct gpuklu_bbd {
       return GPUKLU_OK;
     }
     const int nm = d.border_start;
-    gk::launch_gather(M->d_rhs.p, rhs, d_perm.p, nm, s);  // block rows
-    int st = solve_blocks(d_z.p);
-    if (st) return st;
-    gk::launch_bbd_border_rhs(d_ax.p, rhs, d_z.p, args, d_xT.p, s);
-    gk::launch_dense_lu_solve(d_S.p, d.border_size, d_xT.p, s);
-    gk::launch_bbd_rmatvec(d_ax.p, d_xT.p, args, M->d_rhs.p, s);
-    st = solve_blocks(M->d_out.p);
-    if (st) return st;
-    gk::launch_bbd_combine(d_z.p, M->d_out.p, d_xT.p, args, x, s);
+    if (gk::bbd_solve_fits(args.max_block)) {
+      gk::launch_bbd_forward(M->pd.dp, args, rhs, d_xT.p, s);
+      gk::launch_dense_lu_solve(d_S.p, d.border_size, d_xT.p, s);
+      gk::launch_bbd_backward(M->pd.dp, args, d_xT.p, x, s);
+    } else {  // blocks one thread block does not hold (11.5 k rows): M's own solve, twice
+      gk::launch_gather(M->d_rhs.p, rhs, d_perm.p, nm, s);  // block rows
+      int st = M->solve_on_device(false, false);
+      if (st) return fail(st, M->err);
+      cudaMemcpyAsync(d_z.p, M->d_out.p, (size_t)nm * 8, cudaMemcpyDeviceToDevice, s);
+      gk::launch_bbd_border_rhs(d_ax.p, rhs, d_z.p, args, d_xT.p, s);
+      gk::launch_dense_lu_solve(d_S.p, d.border_size, d_xT.p, s);
+      gk::launch_bbd_rmatvec(d_ax.p, d_xT.p, args, M->d_rhs.p, s);
+      st = M->solve_on_device(false, false);
+      if (st) return fail(st, M->err);
+      gk::launch_bbd_combine(d_z.p, M->d_out.p, d_xT.p, args, x, s);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(GPUKLU_CUDA_ERROR, cuda_msg(e, "bbd solve"));
     return GPUKLU_OK;

@@ -276,7 +276,10 @@ struct BbdArgs {
   const int *rrow_ptr, *rrow_col, *rrow_raw;   // R by block row: (border column, raw)
   const int* perm;                             // bordered order -> original index
   const int* bperm;                            // Schur position -> original index
-  double *zval, *gbuf;                         // Z, Z^T W
+  const int *zref_ptr, *zref;                  // per border row: its places in `row`
+  const int *bw_ptr, *bw, *wcol;               // W tasks by block; a task's border column
+  double *zval, *wval, *gbuf;                  // Z, W (by its reach), Z^T W
+  double *y, *zdot;                            // L^-1 P b by position; Z^T y by place in `row`
   BbdSweep l, u;
   double* rec;                                 // the pivots' reciprocals
   double* scratch;                             // vectors of blocks too large for shared memory
@@ -385,10 +388,13 @@ int bbd_scratch_warps();  // vectors of `scratch` when it does not
 // with the products and the columns of S.
 void launch_bbd_z(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B,
                   cudaStream_t s);
-// out = M^-1 rhs (M's order), every block's vector and lists in shared memory.
+// The solve with every block's vector and lists in shared memory: y = L^-1 P b and
+// the border's right-hand side, then from the border's solution xT the rest of x.
 bool bbd_solve_fits(int max_block);
-void launch_bbd_solve(const DPlan& P, const BbdArgs& B, const double* rhs, double* out,
-                      cudaStream_t s);
+void launch_bbd_forward(const DPlan& P, const BbdArgs& B, const double* rhs, double* bb,
+                        cudaStream_t s);
+void launch_bbd_backward(const DPlan& P, const BbdArgs& B, const double* xT, double* x,
+                         cudaStream_t s);
 void launch_bbd_schur(const DPlan& P, const double* lu, const double* ax, const BbdArgs& B, int j0,
                       int j1, int t0, int t1, double* S, cudaStream_t s);
 void launch_dense_lu(double* S, int bs, cudaStream_t s);
