@@ -950,9 +950,18 @@ struct gpuklu_handle {
   // buffers, the pass limit before the sequential kernel takes over, and the
   // passes the last first factorization ran (0: the sequential kernel).
   static constexpr int kMaxPivotPasses = 8;
-  // Below this many rows the sequential pass costs about as much as one
-  // refactorization plus its host round trip, so it runs directly.
-  static constexpr int64_t kPivotPassMinN = 512;
+  // Below this many rows the sequential pass costs about as much as two
+  // refactorizations with their host round trips, so it runs directly. One Newton
+  // iteration, us, sequential against refactorizations, a handle's first / later
+  // calls: 14 rows 585 / 168 and 623 / 132, 21 rows 669 / 201 and 659 / 133, 66 rows
+  // 972 / 413 and 849 / 176, 258 rows 2984 / 1553 and 1838 / 270 (most patterns take
+  // two or three passes at first, one later).
+  static constexpr int64_t kPivotPassMinN = 16;
+  // Small systems give up sooner: a pass costs what the sequential kernel takes for
+  // about a dozen rows.
+  int pivot_pass_limit(bool forced) const {
+    return forced ? kMaxPivotPasses : (int)std::min<int64_t>(kMaxPivotPasses, 3 + n / 32);
+  }
   DBuf<int> d_cand, d_want, d_pamap_ptr, d_pamap_idx;
   int64_t pivot_passes = 0;
   // The candidate the last settled pass ended with (per column an L slot or
@@ -1121,8 +1130,8 @@ struct gpuklu_handle {
   // depend only on earlier columns), so each pass settles at least one more
   // column, and a pass that agrees everywhere has computed exactly what the
   // sequential pass computes: its pivots, and its factor in d_lu. settled
-  // stays false when kMaxPivotPasses were not enough.
-  int pivot_pass(std::vector<i32>& rperm, bool& settled) {
+  // stays false when `limit` passes were not enough.
+  int pivot_pass(std::vector<i32>& rperm, bool& settled, int limit) {
     settled = false;
     const gk::Plan& P = sym_plan;
     const int nn = P.n;
@@ -1148,7 +1157,7 @@ struct gpuklu_handle {
     pc.cand = d_cand.p;
     pc.want = d_want.p;
     pc.tol = swap_off() ? 0.0 : 0.001;
-    for (int pass = 0; pass < kMaxPivotPasses; ++pass) {
+    for (int pass = 0; pass < limit; ++pass) {
       gk::pivot_pass_amap(P, cand_row, aptr, aidx, rperm);
       e = d_pamap_ptr.upload(aptr, stream);
       if (e == cudaSuccess) e = d_pamap_idx.upload(aidx, stream);
@@ -1202,7 +1211,7 @@ struct gpuklu_handle {
     const bool seq = pp && std::strcmp(pp, "sequential") == 0;
     const bool ref = pp && std::strcmp(pp, "refactor") == 0;
     if (!seq && (ref || n >= kPivotPassMinN)) {
-      const int st = pivot_pass(rperm, settled);
+      const int st = pivot_pass(rperm, settled, pivot_pass_limit(ref));
       if (st) return st;
     }
     if (!settled) {

@@ -10,7 +10,9 @@ import pytest
 import scipy.sparse as sp
 
 from oracle import pyoracle as po
+from rustspice_gb300 import circuits as cz
 from rustspice_gb300 import native as N
+from rustspice_gb300 import workloads as wl
 from rustspice_gb300.solver import GpuKluSolver
 
 pytestmark = pytest.mark.gpu
@@ -83,3 +85,28 @@ def test_refactor_edges(kind, size, one_block, monkeypatch):
         x = b.copy()
         g.solve(x)
         assert np.array_equal(x, o.solve(b)[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("stages", [3, 9, 10, 11, 12, 30, 61])
+@pytest.mark.parametrize("mode", ["nativeklu", "nativeklu_exact"])
+def test_pivot_pass_rule(stages, mode, monkeypatch):
+    """Pivots found as refactorizations (from 16 rows on) and by the sequential
+    kernel: the same factors, the oracle's."""
+    c = cz.inverter_chain(stages, 0.55)
+    n, ap, ai, ax, rhs = po.mna(c, wl.chain_nodeset(stages, 0.55))
+    o = po.Solver(mode, n)
+    o.prepare(n)
+    o.analyze(ap, ai)
+    o.factor(ap, ai, ax)
+    want = o.solve(rhs)[1]
+    for env in ("", "sequential"):
+        if env:
+            monkeypatch.setenv("GPUKLU_PIVOT_PASS", env)
+        g = GpuKluSolver(n, pivot_mode=N.PIVOT_EXACT if mode.endswith("exact")
+                         else N.PIVOT_REFERENCE)
+        g.factor(ap, ai, ax)
+        x = rhs.copy()
+        g.solve(x)
+        assert np.array_equal(x, want)
+        if env or n < 16:
+            assert g.pivot_passes() == 0
