@@ -1635,13 +1635,10 @@ __device__ __forceinline__ int eval_device(int type, const int* nd, const double
   return 0;
 }
 
-__global__ void k_stamp(DCircuit C, const double* __restrict__ x, int xlen, double gmin,
-                        double scale, double dt, const double* __restrict__ cap_v,
-                        double be_sign, double* ax, double* rhs_c, double gdev) {
-  if (C.skip != nullptr && __ldcg(C.skip) != 0) return;
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d == 0 && C.pin_raw >= 0) ax[C.pin_raw] = 1.0;
-  if (d >= C.ndev) return;
+__device__ __forceinline__ void stamp_device(const DCircuit& C, int d, const double* x, int xlen,
+                                             double gmin, double scale, double dt,
+                                             const double* cap_v, double be_sign, double* ax,
+                                             double* rhs_c, double gdev) {
   const int* nd = C.nodes + 4 * d;
   auto xg = [&](int i) { return (i >= 0 && i < xlen) ? x[i] : 0.0; };
   double m[8], r[2];
@@ -1655,6 +1652,37 @@ __global__ void k_stamp(DCircuit C, const double* __restrict__ x, int xlen, doub
   const int* rs = C.rhs_slot + 2 * d;
   for (int e = 0; e < nr; ++e)
     if (rs[e] >= 0) rhs_c[rs[e]] = r[e];
+}
+
+__global__ void k_stamp(DCircuit C, const double* __restrict__ x, int xlen, double gmin,
+                        double scale, double dt, const double* __restrict__ cap_v,
+                        double be_sign, double* ax, double* rhs_c, double gdev) {
+  if (C.skip != nullptr && __ldcg(C.skip) != 0) return;
+  const int d = blockIdx.x * blockDim.x + threadIdx.x;
+  if (d == 0 && C.pin_raw >= 0) ax[C.pin_raw] = 1.0;
+  if (d >= C.ndev) return;
+  stamp_device(C, d, x, xlen, gmin, scale, dt, cap_v, be_sign, ax, rhs_c, gdev);
+}
+
+// k_stamp and k_rhs_sum in one block, for circuits of up to kStampBlock devices: one
+// launch instead of two. Measured, both kernels against this one: 33 devices 6.6 and
+// 5.2 us, 530 devices 7.0 and 6.1 us, and a gap between launches less.
+__global__ void __launch_bounds__(512) k_stamp_block(DCircuit C, const double* __restrict__ x,
+                                                     int xlen, double gmin, double scale,
+                                                     double dt, const double* __restrict__ cap_v,
+                                                     double be_sign, double* ax, double* rhs_c,
+                                                     double* rhs, double gdev) {
+  if (C.skip != nullptr && __ldcg(C.skip) != 0) return;
+  const int tid = threadIdx.x;
+  if (tid == 0 && C.pin_raw >= 0) ax[C.pin_raw] = 1.0;
+  for (int d = tid; d < C.ndev; d += blockDim.x)
+    stamp_device(C, d, x, xlen, gmin, scale, dt, cap_v, be_sign, ax, rhs_c, gdev);
+  __syncthreads();
+  for (int i = tid; i < C.n; i += blockDim.x) {
+    double v = 0.0;
+    for (int t = C.rhs_ptr[i]; t < C.rhs_ptr[i + 1]; ++t) v += rhs_c[C.rhs_src[t]];
+    rhs[i] = v;
+  }
 }
 
 // dL/dp of every device at a DC solution x, given the adjoint lambda
@@ -2252,9 +2280,16 @@ void launch_solve(const DPlan& P, const double* rhs, const double* ax, const dou
                                  status);
 }
 
+// Devices and rows of a circuit stamped in one block (two passes of its threads).
+constexpr int kStampBlock = 1024;
 void launch_stamp(const DCircuit& C, const double* x, int xlen, double gmin, double scale,
                   double dt, const double* cap_v, double be_sign, double* ax, double* rhs_c,
                   double* rhs, cudaStream_t s, double gdev) {
+  if (C.ndev <= kStampBlock && C.n <= kStampBlock) {
+    k_stamp_block<<<1, 512, 0, s>>>(C, x, xlen, gmin, scale, dt, cap_v, be_sign, ax, rhs_c, rhs,
+                                    gdev);
+    return;
+  }
   const int nb = (C.ndev + 255) / 256;
   k_stamp<<<nb > 0 ? nb : 1, 256, 0, s>>>(C, x, xlen, gmin, scale, dt, cap_v, be_sign, ax,
                                           rhs_c, gdev);

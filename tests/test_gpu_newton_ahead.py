@@ -64,3 +64,15 @@ def test_a_non_finite_stop_leaves_the_iterate(side):
     (xa, sta, ita, ra), (xb, stb, itb, rb) = run(1), run(50)
     assert sta == stb == N.NONFINITE and ita == itb == 1 and ra == rb
     assert np.array_equal(xa, xb, equal_nan=True)
+
+
+@pytest.mark.parametrize("diodes", [1, 9, 10, 11, 60])
+def test_stamping_in_one_block(diodes):
+    """Circuits of 1015 to 1074 devices, on both sides of the 1024 that one block
+    stamps: the oracle's iterations and its solution at the DC bar (1e-10)."""
+    c = cz.mesh_dc(23, diodes, seed=3)
+    r, _ = _run(c, 100, 0)
+    reason, its, x = po.dc_op(c, "nativeklu", **{k: wl.TIGHT[k] for k in (
+        "max_iters", "abs_tol", "rel_tol", "gmin", "gmin_steps")})
+    assert (r.reason, r.iterations) == (reason, its)
+    assert np.max(np.abs(r.x - x)) <= 1e-10 * np.max(np.abs(x))
