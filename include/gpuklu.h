@@ -152,7 +152,7 @@ const char* gpuklu_last_error(const gpuklu_handle* h);
 /* Refactorizations the last first factorization ran to find the pivot
  * sequence of native_klu.rs:1194-1382 (the pivot pass restated as
  * refactorizations that check the threshold rule on every column); 0 when
- * the sequential one-warp pivot pass ran instead (below 512 rows, more than 8
+ * the sequential one-warp pivot pass ran instead (below 16 rows, more than 8
  * passes needed, or GPUKLU_PIVOT_PASS=sequential; GPUKLU_PIVOT_PASS=refactor
  * takes the refactorizations at every size). Both give the same pivots and
  * factor. */

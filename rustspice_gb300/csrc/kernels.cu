@@ -6,7 +6,7 @@
 //                    discovers the pivot sequence. k_first_factor_s keeps the
 //                    working column and each column's update operands in
 //                    shared memory; k_first_factor is the fallback for blocks
-//                    too large for that. From 512 rows on the host runs the
+//                    too large for that. From 16 rows on the host runs the
 //                    same pass as refactorizations in their pivot-pass mode
 //                    (PivotCheck) instead, and these kernels only when that
 //                    does not settle.
@@ -18,10 +18,11 @@
 //                    memory while it is updated. k_refactor_cta is the same
 //                    in one block, for small plans.
 //  * solve         - the forward (L) and backward (U) substitutions and the
-//                    BTF block coupling. k_solve_cta sweeps the columns in one
-//                    block (solution vector in shared memory); k_solve runs
-//                    one warp per row task driven by per-row flags (large
-//                    plans); k_tsolve solves A^T y = g for the adjoint.
+//                    BTF block coupling, and A^T y = g for the adjoint.
+//                    k_solve_steps runs them as a step program in one block
+//                    (solution vector in shared memory), k_solve_cta sweeps
+//                    the columns in one block; k_solve and k_tsolve run one
+//                    warp per row task driven by per-row flags (large plans).
 //  * stamp         - one thread per device instance writes its conductances
 //                    into the raw CSC slots given by the stamp-to-slot map and
 //                    its currents into per-contribution slots; a second pass
@@ -30,9 +31,9 @@
 //                    crates/sim-core/src/newton.rs:93-107, 187-201.
 //  * batch_newton  - batched Newton over many circuit instances, one warp per
 //                    instance (or 2, 4 per warp for small programs) with the
-//                    instance's whole state in shared memory; behind the lane
-//                    kernel (lanes.cu) it finishes the instances still
-//                    iterating.
+//                    instance's whole state in shared memory; in use when the
+//                    warp-per-instance kernel (cont.cu) is off, behind the
+//                    lane kernel (lanes.cu) or alone.
 //
 // All floating-point work of the single-circuit kernels is FP64 and compiled
 // without multiply-add contraction, so every product is rounded before it is
