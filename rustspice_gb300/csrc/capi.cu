@@ -572,14 +572,21 @@ static_assert(NewtonLoop::kHead <= 128, "a state's head fits its slot");
 struct SolveDev {
   DBuf<int4> ops, chunks, chains;
   DBuf<int2> segs, terms;
+  DBuf<double2> vc;
+  DBuf<uint2> ad;
   cudaError_t upload(const SolveProgram& sp, cudaStream_t s, gk::SolveSched& d) {
     cudaError_t e = ops.upload(sp.ops, s);
     if (e == cudaSuccess) e = chunks.upload(sp.chunks, s);
     if (e == cudaSuccess) e = segs.upload(sp.segs, s);
     if (e == cudaSuccess) e = chains.upload(sp.chains, s);
     if (e == cudaSuccess) e = terms.upload(sp.terms, s);
-    d = gk::SolveSched{(int)sp.chunks.size(), sp.chunk, sp.width, ops.p,
-                       chunks.p, chains.p, segs.p, terms.p};
+    const char* es = getenv("GPUKLU_SOLVE_STAGED");  // slots from which they are laid out ahead
+    const bool staged = (int64_t)sp.ops.size() >= (es ? atoll(es) : gk::kSolveStaged);
+    if (e == cudaSuccess && staged) e = vc.resize(sp.ops.size());
+    if (e == cudaSuccess && staged) e = ad.resize(sp.ops.size());
+    d = gk::SolveSched{(int)sp.chunks.size(), sp.chunk, sp.width, ops.p, chunks.p, chains.p,
+                       segs.p, terms.p, (int)sp.ops.size(), staged ? vc.p : nullptr,
+                       staged ? ad.p : nullptr};
     return e;
   }
 };
@@ -1340,7 +1347,7 @@ struct gpuklu_handle {
         if (e != cudaSuccess) return cuda_fail(e, "transpose solve program");
       }
       gk::launch_solve_steps(transpose ? pd.dpt : pd.dp, transpose, d_rhs.p, d_ax.p, d_lu.p,
-                             d_rec.p, d_out.p, stream);
+                             d_rec.p, d_out.p, d_status.p, stream);
       if (!sync) return GPUKLU_OK;
       return check_status("solve");
     }

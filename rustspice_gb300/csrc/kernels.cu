@@ -1284,11 +1284,45 @@ __device__ __forceinline__ unsigned exponent_of(double a) {
   return (unsigned)(__double2hiint(a) >> 20) & 0x7ffu;
 }
 
-__global__ void __launch_bounds__(kSolveStepsThreads)
+// The slots of a large program as the rows read them (values and factor; the
+// addresses, from the solution's base, of destination and source with their
+// flags), laid out by the whole grid ahead of the solve.
+__global__ void k_solve_slots(SolveSched S, int n, const double* __restrict__ ax,
+                              const double* __restrict__ lu, const int* skip) {
+  if (skip != nullptr && __ldcg(skip) != 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= S.nslots) return;
+  const int4 o = __ldg(S.ops + i);
+  const int kind = o.w & 3;
+  const bool div = kind == 1, none = kind == 3;
+  const double m = none ? 0.0 : (kind == 2 ? ax : lu)[o.z], y = div ? 1.0 / m : 0.0;
+  const bool slow = div && (exponent_of(m) - 64u > 1919u || exponent_of(y) - 64u > 1919u);
+  S.vc[i] = make_double2(div ? y : m, div ? -m : (none ? 0.0 : -1.0));
+  S.ad[i] =
+      make_uint2(8u * (unsigned)(none ? n : o.x) | (unsigned)(o.w >> 2) | (div ? kSlotDiv : 0u),
+                 8u * (unsigned)(none ? n : o.y) | (slow ? kSlotSlow : 0u));
+}
+
+// n bytes (a multiple of 16) from memory to shared memory, counted by barrier b.
+__device__ __forceinline__ void bulk_copy(unsigned d, const void* g, unsigned n, unsigned b) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          d),
+      "l"(g), "r"(n), "r"(b)
+      : "memory");
+}
+
+// kStaged (programs of kSolveStaged slots or more): the slots come ready from
+// k_solve_slots, a chunk in two bulk copies by one warp, and the loads of eight
+// loader warps no longer share the SM's load unit with the rows. Measured, 801 k
+// slots (15,403 rows): 1.69 -> 1.45 ms with the layout's 11 us; 96 k slots 234 -> 229
+// us, 42 k slots 112 -> 114 us, 122 slots 7.3 -> 9.3 us.
+template <bool kStaged>
+__global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
     k_solve_steps(SolveSched S, int n, const int* __restrict__ in, const int* __restrict__ outp,
                   const int* __restrict__ dslot, const double* __restrict__ rhs,
                   const double* __restrict__ ax, const double* __restrict__ lu, double* rec,
-                  double* out, const int* skip) {
+                  double* out, const int* skip, int* status) {
   if (skip != nullptr && __ldcg(skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* const T = reinterpret_cast<double*>(smem_raw);  // the solution, a spare entry at n
@@ -1297,11 +1331,23 @@ __global__ void __launch_bounds__(kSolveStepsThreads)
   int2* const sseg = reinterpret_cast<int2*>(sad + 2 * S.chunk);   // segments, an end mark
   const unsigned T0 = (unsigned)__cvta_generic_to_shared(T);
   const int tid = threadIdx.x, lane = tid & 31;
+  __shared__ __align__(8) unsigned long long bars[4];  // a half is full, 2: is free
+  __shared__ int dead_flag;
+  volatile int* const dead = &dead_flag;
+  const unsigned bar0 = (unsigned)__cvta_generic_to_shared(bars);
+  const unsigned A0 = kStaged ? T0 : 0u;  // what the slots' addresses count from
   for (int i = tid; i < n; i += blockDim.x) {
     T[i] = rhs[in[i]];
-    rec[i] = 1.0 / lu[dslot[i]];
+    if (!kStaged) rec[i] = 1.0 / lu[dslot[i]];
   }
-  if (tid == 0) T[n] = 0.0;
+  if (tid == 0) {
+    T[n] = 0.0;
+    if (kStaged) {
+      for (int i = 0; i < 4; ++i) bar_init(bar0 + 8 * i, i < 2 ? 1 : kSolveRow / 32);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      *dead = 0;
+    }
+  }
   __syncthreads();
   // chunk c into its half of the buffer, by the threads from tid0 on:
   // kLoadBatch operations' loads in flight together, then their values'
@@ -1366,8 +1412,8 @@ __global__ void __launch_bounds__(kSolveStepsThreads)
   };
   // one slot's operation
   auto exec = [&](uint2 a, double2 vc) {
-    const unsigned da = a.x & ~7u;
-    const double td = lds_f64(da), ts = lds_f64(a.y & ~7u);
+    const unsigned da = A0 + (a.x & ~7u);
+    const double td = lds_f64(da), ts = lds_f64(A0 + (a.y & ~7u));
     const double p = vc.x * ts;
     double r = fma(vc.y, p, td);
     if (a.x & kSlotDivRow) {
@@ -1381,10 +1427,45 @@ __global__ void __launch_bounds__(kSolveStepsThreads)
     }
     sts_f64(da, r);
   };
-  if (S.nchunks > 0) load(0, 0);
+  if (!kStaged && S.nchunks > 0) load(0, 0);
   __syncthreads();
+  if (kStaged && tid >= kSolveRow) {  // the copying warp
+    const int2 end = make_int2(3, -1);
+    for (int c = 0; c < S.nchunks; ++c) {
+      const int h = c & 1;
+      const int4 C = __ldg(S.chunks + c);
+      const int2 s0 = lane < C.w ? __ldg(S.segs + C.z + lane) : end;
+      const int2 s1 = lane + 32 < C.w ? __ldg(S.segs + C.z + lane + 32) : end;
+      if (!bar_wait(bar0 + 8 * (2 + h), (c >> 1 & 1) ^ 1u, dead)) break;
+      int2* const sg = sseg + h * (kSolveSegs + 1);
+      sg[lane] = s0;
+      sg[lane + 32] = s1;
+      if (lane == 0) sg[64] = end;
+      __syncwarp();
+      if (lane == 0) {
+        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(bar0 + 8 * h),
+                     "r"(24 * C.y)
+                     : "memory");
+        if (C.y > 0) {
+          bulk_copy((unsigned)__cvta_generic_to_shared(svc + h * S.chunk), S.vc + C.x, 16 * C.y,
+                    bar0 + 8 * h);
+          bulk_copy((unsigned)__cvta_generic_to_shared(sad + h * S.chunk), S.ad + C.x, 8 * C.y,
+                    bar0 + 8 * h);
+        }
+      }
+      __syncwarp();
+    }
+  }
   for (int c = 0; c < S.nchunks; ++c) {
-    if (tid >= kSolveRow) {
+    if (kStaged) {
+      if (tid >= kSolveRow) break;
+      if (!bar_wait(bar0 + 8 * (c & 1), c >> 1 & 1, dead)) {
+        *dead = 1;
+        atomicCAS(status, DS_OK, DS_TIMEOUT);
+        break;
+      }
+    }
+    if (!kStaged && tid >= kSolveRow) {
       if (c + 1 < S.nchunks) load(c + 1, kSolveRow);
     } else {
       const int2* seg = sseg + (c & 1) * (kSolveSegs + 1);
@@ -1445,8 +1526,14 @@ __global__ void __launch_bounds__(kSolveStepsThreads)
         }
       }
     }
-    __syncthreads();
+    if (kStaged) {  // the half is free (the rows ordered themselves where it matters)
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar0 + 8 * (2 + (c & 1)));
+    } else {
+      __syncthreads();
+    }
   }
+  if (kStaged) __syncthreads();
   for (int i = tid; i < n; i += blockDim.x) out[outp[i]] = T[i];
 }
 
@@ -2246,13 +2333,17 @@ bool solve_steps_fits(const DPlan& P) {
 }
 
 void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,
-                        const double* lu, double* rec, double* out, cudaStream_t s) {
+                        const double* lu, double* rec, double* out, int* status, cudaStream_t s) {
   const size_t bytes = solve_steps_bytes(P.n, P.ss.chunk);
+  const bool staged = P.ss.vc != nullptr;
+  const auto kernel = staged ? k_solve_steps<true> : k_solve_steps<false>;
   if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(k_solve_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  k_solve_steps<<<1, kSolveStepsThreads, bytes, s>>>(
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (staged)
+    k_solve_slots<<<(P.ss.nslots + 255) / 256, 256, 0, s>>>(P.ss, P.n, ax, lu, P.skip);
+  kernel<<<1, staged ? kSolveRow + 32 : kSolveStepsThreads, bytes, s>>>(
       P.ss, P.n, transpose ? P.out_col : P.in_row, transpose ? P.in_row : P.out_col, P.dslot, rhs,
-      ax, lu, rec, out, P.skip);
+      ax, lu, rec, out, P.skip, status);
 }
 
 bool solve_groups_fit(const DPlan& P) {

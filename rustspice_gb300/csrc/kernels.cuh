@@ -19,12 +19,18 @@ constexpr unsigned kSpinLimit = 1u << 22;
 // terms; a term: source row, lu value or ~ax value), and those into chunks
 // (first slot, slots, first segment, segments). 0 chunks: none.
 constexpr int kSolveRow = 128;   // compute threads
+constexpr int kSolveStaged = 1 << 18;  // slots of a program laid out ahead
 constexpr int kSolveSegs = 64;   // segments of a chunk, at most
 enum { kSolveSegSolo = 0, kSolveSegWide = 1, kSolveSegChain = 2 };
 struct SolveSched {
   int nchunks, chunk, width;
   const int4 *ops, *chunks, *chains;
   const int2 *segs, *terms;
+  // Programs of kSolveStaged slots or more: the slots as the rows read them, laid
+  // out ahead of every solve (else null).
+  int nslots;
+  double2* vc;
+  uint2* ad;
 };
 // Shared memory of k_solve_steps: the solution and a spare entry, then twice
 // a chunk's slots (two doubles, two words) and segments.
@@ -341,7 +347,7 @@ bool solve_steps_fits(const DPlan& P);
 // rec: n doubles of scratch (the pivots' reciprocals); transpose: P.ss is
 // the transpose solve's program
 void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,
-                        const double* lu, double* rec, double* out, cudaStream_t s);
+                        const double* lu, double* rec, double* out, int* status, cudaStream_t s);
 // One block per group of uncoupled BTF blocks (cs_grp); fits when the
 // largest group's rows fit one block's shared memory.
 bool solve_groups_fit(const DPlan& P);

@@ -74,3 +74,13 @@ def test_step_program_edges(kind, size, band):
             ref = sla.spsolve((A * scale).T.tocsc(), b)
             assert np.max(np.abs(y - ref)) <= 1e-12 * np.max(np.abs(ref))
     g.close()
+
+
+@pytest.mark.parametrize("kind,size,band", [("arrow", 2, 0), ("arrow", 300, 2), ("pairs", 33, 0),
+                                            ("pairs", 700, 0), ("ladder", 22000, 0),
+                                            ("ladder", 28600, 0)])
+def test_slots_laid_out_ahead(kind, size, band, monkeypatch):
+    """The form of large programs (slots laid out by the grid, copied in bulk) at
+    every chunk size: the same bits."""
+    monkeypatch.setenv("GPUKLU_SOLVE_STAGED", "0")
+    test_step_program_edges(kind, size, band)
