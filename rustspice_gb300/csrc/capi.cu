@@ -3159,8 +3159,8 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
       const char* eck = getenv("GPUKLU_CONT_KERNEL");
       // Instances per warp: one. GPUKLU_CONT_M=2 puts two of a program in a
       // warp (16 lanes each, a row's FP64 instruction serving both; the same
-      // results bit for bit): 976 instances take 10.3 ms against 7.6 ms, 249,856
-      // 70.3 ms against 69.2 ms, because an instance that runs to the
+      // results bit for bit): 976 instances take 10.0 ms against 7.2 ms, 249,856
+      // 64.7 ms against 65.2 ms, because an instance that runs to the
       // iteration cap keeps its warp long after the other half has run out.
       const char* ecm = getenv("GPUKLU_CONT_M");
       const int cm = ecm && ecm[0] == '2' ? 2 : 1;

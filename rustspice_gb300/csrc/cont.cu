@@ -13,8 +13,8 @@
 // sub-partition whatever its active lanes, and for the instances that run to
 // the iteration cap the latency of their rows. Measured against the lane
 // kernel's six iterations and a kernel that loads its steps from global
-// memory behind it: 976 instances (16 chains of 8-256 stages) 32.6 -> 7.6 ms,
-// 249,856 instances 71.7 -> 66.8 ms.
+// memory behind it: 976 instances (16 chains of 8-256 stages) 32.6 -> 7.2 ms,
+// 249,856 instances 71.7 -> 65.2 ms.
 #include <cfloat>
 
 #include "batch_common.cuh"

@@ -379,9 +379,11 @@ void launch_batch_newton(const BatchArgs& a, int m, int grid, int warps_per_bloc
                          cudaStream_t s, bool shared = false);
 // Registers per thread and resident blocks per SM of the batched kernel.
 // Lane-per-instance batched Newton (phase 1 of gpuklu_batch_run).
-// Continuation kernel: one warp per block, m instances per warp; kContWarps
-// blocks fit an SM's registers.
-constexpr int kContWarps = 12;
+// Warp-per-instance kernel: one warp per block, m instances per warp; kContWarps
+// blocks at least fit an SM's registers. With 8 the compiler keeps 222 registers
+// and spills none, and 9 warps share an SM; measured, 249,856 / 976 instances, ms:
+// 8 65.1 / 7.2, 10 66.2 / 7.6, 12 66.9 / 7.5, 16 68.5 / 8.2, 20 73.4 / 8.9.
+constexpr int kContWarps = 8;
 void launch_batch_cont(const BatchArgs& a, int m, int grid, cudaStream_t s);
 void cont_kernel_info(int m, int slice, int* regs, int* blocks_per_sm);
 void launch_batch_lanes(const BatchArgs& a, int grid, int warps_per_block, cudaStream_t s);
