@@ -333,6 +333,7 @@ void atran_kernel_info(int region, int prog_ints, int* regs, int* blocks_per_sm)
   const size_t sm = (size_t)prog_ints * 4 + (size_t)region * 8;
   cudaFuncSetAttribute(k_atran, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_atran, 32, sm);
+  cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm
 }
 
 }  // namespace gk

@@ -22,7 +22,11 @@ using gk::i64;
 
 namespace {
 
+// The text of an error that a call returns. The runtime keeps it as the
+// thread's last error as well: taken back here, or the next call that checks
+// its launches would report it again.
 std::string cuda_msg(cudaError_t e, const char* what) {
+  cudaGetLastError();
   return std::string(what) + ": " + cudaGetErrorString(e);
 }
 
@@ -1107,13 +1111,18 @@ struct gpuklu_handle {
     return GPUKLU_OK;
   }
 
+  // What the call's launches came to: a kernel that was refused at its launch
+  // leaves the status word as it was and shows as the thread's last error
+  // alone; one that gave up has set the word.
   int check_status(const char* what) {
     int st = 0;
+    const cudaError_t launched = cudaGetLastError();
     cudaError_t e = cudaMemcpyAsync(&st, d_status.p, sizeof(int), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (st != 0) cudaMemsetAsync(d_status.p, 0, sizeof(int), stream);
+    if (e == cudaSuccess) e = launched;
     if (e != cudaSuccess) return cuda_fail(e, what);
     if (st != 0) {
-      cudaMemsetAsync(d_status.p, 0, sizeof(int), stream);
       return fail(st, std::string(what) + ": device status " + std::to_string(st));
     }
     return GPUKLU_OK;
@@ -1543,8 +1552,11 @@ int gpuklu_get_stats(gpuklu_handle* h, gpuklu_stats* out) {
       h->kind != GPUKLU_KIND_DENSE) {
     gk::launch_rcond(h->pd.dp, h->d_lu.p, h->d_rc.p, h->stream);
     double mm[2];
-    cudaMemcpyAsync(mm, h->d_rc.p, sizeof(mm), cudaMemcpyDeviceToHost, h->stream);
-    cudaStreamSynchronize(h->stream);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(mm, h->d_rc.p, sizeof(mm), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return h->cuda_fail(e, "stats");
     h->rcond = mm[1] > 0.0 ? mm[0] / mm[1] : 0.0;
     h->rcond_valid = true;
   }
@@ -1585,7 +1597,7 @@ gpuklu_circuit* gpuklu_compile_devices(int64_t node_count, int64_t ndev, const i
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
   cudaError_t e = upload_circuit(*c);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_compile_devices: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_compile_devices").c_str());
     cudaStreamDestroy(c->stream);
     return nullptr;
   }
@@ -1641,8 +1653,10 @@ int gpuklu_stamp(gpuklu_handle* h, gpuklu_circuit* c, const double* x, int64_t x
   if (e != cudaSuccess) return h->cuda_fail(e, "stamp upload");
   gk::launch_stamp(c->dc, dx.p, (int)xlen, gmin, source_scale, dt, cap_v ? dcap.p : nullptr,
                    be_sign, dax.p, drc.p, drhs.p, h->stream);
-  e = cudaMemcpyAsync(ax_out, dax.p, c->ai.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                      h->stream);
+  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(ax_out, dax.p, c->ai.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                        h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(rhs_out, drhs.p, c->n * sizeof(double), cudaMemcpyDeviceToHost,
                         h->stream);
@@ -3268,7 +3282,7 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
   if (e == cudaSuccess) e = cudaMemsetAsync(B->d_status.p, 0, sizeof(int), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_batch_create: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_batch_create").c_str());
     return nullptr;
   }
   gk::BatchArgs a{};
@@ -3427,7 +3441,7 @@ gpuklu_batch* gpuklu_tran_create(int64_t ncirc, const int64_t* dev_off,
   if (e == cudaSuccess) e = B->d_tcounter.resize(1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_tran_create: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_tran_create").c_str());
     return nullptr;
   }
   int regs = 0, bf = 0, bb = 0;
@@ -3541,7 +3555,7 @@ gpuklu_batch* gpuklu_atran_create(int64_t ncirc, const int64_t* dev_off,
   if (e == cudaSuccess) e = B->d_tcounter.resize(1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_atran_create: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_atran_create").c_str());
     return nullptr;
   }
   int regs = 0, bps = 0;
@@ -4639,7 +4653,7 @@ gpuklu_bbd* gpuklu_bbd_create(int64_t n, const int64_t* ap, int64_t ap_len, cons
   if (e == cudaSuccess) e = cudaMemsetAsync(B->d_status.p, 0, sizeof(int), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_bbd_create: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_bbd_create").c_str());
     return nullptr;
   }
   return B.release();
@@ -4892,7 +4906,7 @@ int gpuklu_dense_lu_nopivot(double* a, int64_t n, int variant, double* ms_out) {
   if (e1) cudaEventDestroy(e1);
   if (s) cudaStreamDestroy(s);
   if (e != cudaSuccess) {
-    fprintf(stderr, "gpuklu_dense_lu_nopivot: %s\n", cudaGetErrorString(e));
+    fprintf(stderr, "%s\n", cuda_msg(e, "gpuklu_dense_lu_nopivot").c_str());
     return GPUKLU_CUDA_ERROR;
   }
   return st == 0 ? GPUKLU_OK : st;

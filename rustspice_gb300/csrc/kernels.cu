@@ -2505,6 +2505,7 @@ static void info_m(int warps_per_block, int region, int prog_ints, int* regs,
   raise_smem_limit<M, SHARED>(sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_batch_newton<M, SHARED>,
                                                 32 * warps_per_block, sm);
+  cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm
 }
 
 void batch_kernel_info(int m, int warps_per_block, int region, int prog_ints, int* regs,

@@ -280,6 +280,7 @@ void tran_kernel_info(bool backward, int warps_per_block, int region, int prog_i
   const size_t sm = (size_t)warps_per_block * ((size_t)prog_ints * 4 + (size_t)region * 8);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, 32 * warps_per_block, sm);
+  cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm
 }
 
 }  // namespace gk
