@@ -489,7 +489,7 @@ AcShape ac_shape(int n, int nf, int sms) {
 }
 
 void launch_ac_sparse(const AcArgs& a, int nf, const AcShape& s, cudaStream_t st) {
-  cudaFuncSetAttribute(k_ac_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  raise_smem_limit<k_ac_sparse>(s.smem);
   k_ac_sparse<<<s.blocks, 32 * s.warps, s.smem, st>>>(a, nf, s.masks_shared ? 1 : 0);
 }
 

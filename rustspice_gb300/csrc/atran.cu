@@ -331,7 +331,7 @@ void atran_kernel_info(int region, int prog_ints, int* regs, int* blocks_per_sm)
   cudaFuncGetAttributes(&fa, k_atran);
   *regs = fa.numRegs;
   const size_t sm = (size_t)prog_ints * 4 + (size_t)region * 8;
-  cudaFuncSetAttribute(k_atran, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  raise_smem_limit<k_atran>(sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_atran, 32, sm);
   cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm
 }

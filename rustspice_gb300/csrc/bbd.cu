@@ -591,8 +591,7 @@ void launch_reach(const DPlan& P, const double* lu, const double* ax, const BbdA
   const int stride = (B.max_block + 2) & ~1, wpb = reach_warps(B.max_block);
   if (wpb > 0) {
     const int bytes = wpb * stride * 8;
-    cudaFuncSetAttribute(k_bbd_reach<kRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
+    raise_smem_limit<k_bbd_reach<kRows, true>>(bytes);
     k_bbd_reach<kRows, true>
         <<<cdiv(t1 - t0, wpb), 32 * wpb, bytes, s>>>(P, lu, ax, B, stride, t0, t1);
   } else {
@@ -621,7 +620,7 @@ void launch_bbd_z(const DPlan& P, const double* lu, const double* ax, const BbdA
 void launch_bbd_forward(const DPlan& P, const BbdArgs& B, const double* rhs, double* bb,
                         cudaStream_t s) {
   const int bytes = (int)bbd_solve_bytes(B.max_block);
-  cudaFuncSetAttribute(k_bbd_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  raise_smem_limit<k_bbd_forward>(bytes);
   k_bbd_forward<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, rhs);
   k_bbd_border<<<cdiv(B.bs, 128), 128, 0, s>>>(B, rhs, bb);
 }
@@ -629,7 +628,7 @@ void launch_bbd_forward(const DPlan& P, const BbdArgs& B, const double* rhs, dou
 void launch_bbd_backward(const DPlan& P, const BbdArgs& B, const double* xT, double* x,
                          cudaStream_t s) {
   const int bytes = (int)bbd_solve_bytes(B.max_block);
-  cudaFuncSetAttribute(k_bbd_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  raise_smem_limit<k_bbd_backward>(bytes);
   k_bbd_backward<<<P.nblocks, kSweepThreads, bytes, s>>>(P, B, xT, x);
 }
 
@@ -639,7 +638,7 @@ void launch_bbd_schur(const DPlan& P, const double* lu, const double* ax, const 
   int nw = 8;  // warps, a column of S each
   while (nw > 1 && nw * B.bs * 8 > 100 * 1024) nw >>= 1;
   const int bytes = nw * B.bs * 8;
-  cudaFuncSetAttribute(k_bbd_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  raise_smem_limit<k_bbd_schur>(bytes);
   k_bbd_schur<<<j1 - j0, 32 * nw, bytes, s>>>(ax, B, j0, S);
 }
 
@@ -658,7 +657,7 @@ void launch_dense_lu(double* S, int bs, cudaStream_t s) {
 }
 
 void launch_dense_lu_solve(const double* S, int bs, double* x, cudaStream_t s) {
-  cudaFuncSetAttribute(k_dlu_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, bs * 8);
+  raise_smem_limit<k_dlu_solve>((size_t)bs * 8);
   k_dlu_solve<<<1, kDluThreads, bs * 8, s>>>(S, bs, x);
 }
 

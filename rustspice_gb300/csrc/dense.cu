@@ -132,8 +132,7 @@ void launch_dense_solve(int n, const double* A, const int* piv, const double* rh
                         int* status, cudaStream_t s) {
   if (n <= 0) return;
   const size_t bytes = (size_t)n * sizeof(double);
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(k_dense_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem_limit<k_dense_solve>(bytes);
   k_dense_solve<<<1, 32, bytes, s>>>(n, A, piv, rhs, out, status);
 }
 

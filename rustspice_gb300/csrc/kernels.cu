@@ -43,7 +43,6 @@
 // the Newton tolerance.
 #include <algorithm>
 #include <cstdio>
-#include <mutex>
 
 #include "batch_common.cuh"
 #include "device.cuh"
@@ -2261,8 +2260,7 @@ void launch_first_factor(const DPlan& P, int maxblk, const double* ax, double* l
   while (cap > 256 && fixed + (size_t)12 * cap > (size_t)optin) cap >>= 1;
   const size_t bytes = fixed + (size_t)12 * cap;
   if (maxblk > 0 && bytes <= (size_t)optin) {
-    cudaFuncSetAttribute(k_first_factor_s, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)bytes);
+    raise_smem_limit<k_first_factor_s>(bytes);
     k_first_factor_s<<<1, 32, bytes, s>>>(P, ax, lu, rperm, rinv, tol, maxblk, cap);
     return;
   }
@@ -2278,7 +2276,7 @@ void launch_refactor(const DPlan& P, const double* ax, double* lu, double* big, 
     cudaMemsetAsync(lu, 0xff, (size_t)words * sizeof(double), s);
   const int colcap = std::min((P.max_col + 1) & ~1, kColCap);
   const int bytes = kPairs * (kGridRing * kGridStage + 8 * colcap);
-  cudaFuncSetAttribute(k_refactor, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  raise_smem_limit<k_refactor>(bytes);
   k_refactor<<<grid, 64 * kPairs, bytes, s>>>(P, ax, lu, big, colcap, status, pc);
 }
 bool refactor_needs_big(const DPlan& P) { return P.max_col > kColCap; }
@@ -2303,7 +2301,7 @@ bool refactor_cta_fits(const DPlan& P) {
 void launch_refactor_cta(const DPlan& P, const double* ax, double* lu, int* status,
                          cudaStream_t s, const PivotCheck& pc) {
   const size_t bytes = refactor_cta_bytes(P);
-  cudaFuncSetAttribute(k_refactor_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem_limit<k_refactor_cta>(bytes);
   k_refactor_cta<<<1, 1024, bytes, s>>>(P, ax, lu, status, pc);
 }
 
@@ -2322,8 +2320,7 @@ bool solve_cta_fits(const DPlan& P) {
 void launch_solve_cta(const DPlan& P, const double* rhs, const double* ax, const double* lu,
                       double* out, cudaStream_t s) {
   const size_t bytes = solve_cta_bytes(P);
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(k_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem_limit<k_solve_cta>(bytes);
   k_solve_cta<<<1, 256, bytes, s>>>(P, rhs, ax, lu, out, kSolveChunk, 0);
 }
 
@@ -2337,8 +2334,10 @@ void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const
   const size_t bytes = solve_steps_bytes(P.n, P.ss.chunk);
   const bool staged = P.ss.vc != nullptr;
   const auto kernel = staged ? k_solve_steps<true> : k_solve_steps<false>;
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (staged)
+    raise_smem_limit<k_solve_steps<true>>(bytes);
+  else
+    raise_smem_limit<k_solve_steps<false>>(bytes);
   if (staged)
     k_solve_slots<<<(P.ss.nslots + 255) / 256, 256, 0, s>>>(P.ss, P.n, ax, lu, P.skip);
   kernel<<<1, staged ? kSolveRow + 32 : kSolveStepsThreads, bytes, s>>>(
@@ -2354,8 +2353,7 @@ bool solve_groups_fit(const DPlan& P) {
 void launch_solve_groups(const DPlan& P, const double* rhs, const double* ax, const double* lu,
                          double* out, cudaStream_t s) {
   const size_t bytes = solve_cta_bytes(P, P.cs_grp_rows);
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(k_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem_limit<k_solve_cta>(bytes);
   k_solve_cta<<<P.cs_ngrp, 256, bytes, s>>>(P, rhs, ax, lu, out, kSolveChunk, 1);
 }
 
@@ -2450,25 +2448,10 @@ static size_t smem_bytes(const BatchArgs& a, int warps_per_block) {
   return ((size_t)a.prog_ints * 4 + (size_t)a.region * M * sizeof(double)) * warps_per_block;
 }
 
-// The dynamic shared-memory limit of an instantiation is one attribute for
-// every launch of it; launches of different sizes (the batch's classes)
-// raise it to the largest size any of them needs.
-template <int M, bool SHARED>
-static void raise_smem_limit(size_t bytes) {
-  static std::mutex mu;
-  static size_t set = 0;
-  std::lock_guard<std::mutex> lock(mu);
-  if (bytes > set) {
-    cudaFuncSetAttribute(k_batch_newton<M, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)bytes);
-    set = bytes;
-  }
-}
-
 template <int M, bool SHARED>
 static void launch_m(const BatchArgs& a, int grid, int warps_per_block, cudaStream_t s) {
   const size_t sm = smem_bytes<M, SHARED>(a, warps_per_block);
-  raise_smem_limit<M, SHARED>(sm);
+  raise_smem_limit<k_batch_newton<M, SHARED>>(sm);
   k_batch_newton<M, SHARED><<<grid, 32 * warps_per_block, sm, s>>>(a);
 }
 
@@ -2502,7 +2485,7 @@ static void info_m(int warps_per_block, int region, int prog_ints, int* regs,
   *regs = fa.numRegs;
   const size_t per = (size_t)region * M * sizeof(double);
   const size_t sm = SHARED ? shared_bytes : ((size_t)prog_ints * 4 + per) * warps_per_block;
-  raise_smem_limit<M, SHARED>(sm);
+  raise_smem_limit<k_batch_newton<M, SHARED>>(sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_batch_newton<M, SHARED>,
                                                 32 * warps_per_block, sm);
   cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm

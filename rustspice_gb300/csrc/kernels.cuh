@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <mutex>
 
 namespace gk {
 
@@ -309,6 +310,29 @@ struct AcArgs {
 };
 
 // --------------------------------------------------------------- launches
+// Raises a kernel's dynamic shared-memory limit to `bytes` where it is lower.
+// The limit belongs to the kernel on a device, not to a handle or a launch:
+// set to one plan's size before its launch, another thread's smaller plan
+// could lower it in between, and an older batch would find a newer one's. So
+// it only ever goes up, under a lock. A size the device refuses is not kept,
+// and the launch reports it.
+template <auto Kernel>
+inline cudaError_t raise_smem_limit(size_t bytes) {
+  constexpr int kDevices = 64;
+  static std::mutex mu;
+  static size_t limit[kDevices] = {};
+  if (bytes <= 48 * 1024) return cudaSuccess;  // every kernel's own limit
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= kDevices) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (bytes <= limit[dev]) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit[dev] = bytes;
+  return e;
+}
+
 // maxblk: the largest diagonal block; blocks up to about 14k rows run with the
 // working column in shared memory.
 void launch_first_factor(const DPlan& P, int maxblk, const double* ax, double* lu,

@@ -278,7 +278,10 @@ void tran_kernel_info(bool backward, int warps_per_block, int region, int prog_i
   cudaFuncGetAttributes(&fa, fn);
   *regs = fa.numRegs;
   const size_t sm = (size_t)warps_per_block * ((size_t)prog_ints * 4 + (size_t)region * 8);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (backward)
+    raise_smem_limit<k_tran_bwd>(sm);
+  else
+    raise_smem_limit<k_tran_fwd>(sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, 32 * warps_per_block, sm);
   cudaGetLastError();  // more than a block may have: answered by *blocks_per_sm
 }
