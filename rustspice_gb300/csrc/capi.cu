@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -1003,7 +1004,14 @@ struct gpuklu_handle {
   bool stop_nonfinite = false;
 
   void apply_spin_limit() {
-    for (PlanDev* p : {&pd, &pd_sym}) p->dp.spin_limit = p->dpt.spin_limit = spin_limit;
+    // GPUKLU_PAIR_POLLS: a short limit on the waits within a pair of warps
+    const char* ep = getenv("GPUKLU_PAIR_POLLS");
+    const uint64_t pair =
+        ep ? strtoull(ep, nullptr, 10) : 8 * (uint64_t)std::max(spin_limit, gk::kSpinLimit);
+    for (PlanDev* p : {&pd, &pd_sym}) {
+      p->dp.spin_limit = p->dpt.spin_limit = spin_limit;
+      p->dp.pair_limit = p->dpt.pair_limit = (unsigned)std::min<uint64_t>(pair, UINT32_MAX);
+    }
   }
 
   int fail(int code, const std::string& m) {

@@ -685,8 +685,10 @@ __device__ __forceinline__ void bar_arrive(unsigned b) {
 __device__ __forceinline__ void bar_arrive_copies(unsigned b) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(b) : "memory");
 }
-// Waits for the end of a barrier's phase; false when the pair has given up.
-__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile int* dead) {
+// Waits for the end of a barrier's phase; false when the pair has given up or
+// the wait runs out.
+__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile int* dead,
+                                         unsigned limit) {
   for (unsigned spins = 0;; ++spins) {
     unsigned done;
     asm volatile(
@@ -697,8 +699,15 @@ __device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile i
         : "r"(b), "r"(parity)
         : "memory");
     if (__all_sync(FULL, done)) return true;
-    if (__any_sync(FULL, *dead != 0 || spins > 8 * kSpinLimit)) return false;
+    if (__any_sync(FULL, *dead != 0 || spins >= limit)) return false;
     if (spins > 256) __nanosleep(100);
+  }
+}
+// Ends the pair, and through the status the pairs that wait for its column.
+__device__ __forceinline__ void give_up(volatile int* dead, int* status) {
+  if ((threadIdx.x & 31) == 0) {
+    *dead = 1;
+    atomicCAS(status, DS_OK, DS_TIMEOUT);
   }
 }
 
@@ -718,7 +727,8 @@ struct Stages {
   }
 };
 
-__device__ __forceinline__ void load_columns(const DPlan& P, const double* lu, unsigned* counter,
+// Returns false when a wait gave up.
+__device__ __forceinline__ bool load_columns(const DPlan& P, const double* lu, unsigned* counter,
                                              Stages S, volatile int* dead) {
   const int lane = threadIdx.x & 31;
   auto publish = [&](int4 h) {  // after the stage's copies
@@ -730,10 +740,10 @@ __device__ __forceinline__ void load_columns(const DPlan& P, const double* lu, u
     int k = 0;
     if (lane == 0) k = (int)(atomicAdd(counter, 1u) + 1u);
     k = __shfl_sync(FULL, k, 0);
-    if (!bar_wait(S.empty(), S.ph ^ 1u, dead)) return;
+    if (!bar_wait(S.empty(), S.ph ^ 1u, dead, P.pair_limit)) return false;
     if (k >= P.n) {
       publish(make_int4(0, 0, kEnd, 0));
-      return;
+      return true;
     }
     k = P.order[k];
     const int s0 = P.col_ptr[k], ds = P.dslot[k], s1 = P.col_ptr[k + 1];
@@ -744,7 +754,7 @@ __device__ __forceinline__ void load_columns(const DPlan& P, const double* lu, u
     Pieces todo(P, s0, ds);
     bool more = todo.more();
     do {
-      if (!bar_wait(S.empty(), S.ph ^ 1u, dead)) return;
+      if (!bar_wait(S.empty(), S.ph ^ 1u, dead, P.pair_limit)) return false;
       int4 h = make_int4(0, 0, kNone, 0);
       if (more) {
         h = todo.next(S.at(), lu);
@@ -753,7 +763,7 @@ __device__ __forceinline__ void load_columns(const DPlan& P, const double* lu, u
         if (!more) h.z |= kLast;
       }
       publish(h);
-      if (!more && !bar_wait(S.empty(), S.ph, dead)) return;
+      if (!more && !bar_wait(S.empty(), S.ph, dead, P.pair_limit)) return false;
       S.advance();
     } while (more);
   }
@@ -768,7 +778,7 @@ __device__ __forceinline__ bool grid_updates(const DPlan& P, double* C, const do
   auto at = [&](int s) { return kStaged ? C[s] : ld_cg(&C[s]); };
   Piece nx;
   auto read = [&]() {
-    if (!bar_wait(S.full(), S.ph, dead)) return false;
+    if (!bar_wait(S.full(), S.ph, dead, P.pair_limit)) return false;
     nx.read(S.at(), true);
     __syncwarp();
     if ((nx.h.z & kLast) == 0) {
@@ -851,12 +861,16 @@ __global__ void __launch_bounds__(64 * kPairs) k_refactor(DPlan P, const double*
   }
   __syncthreads();
   if (loader) {
-    load_columns(P, lu, reinterpret_cast<unsigned*>(lu + P.nslots + 2), S, dead);
+    if (!load_columns(P, lu, reinterpret_cast<unsigned*>(lu + P.nslots + 2), S, dead))
+      give_up(dead, status);
     asm volatile("cp.async.wait_all;" ::: "memory");
     return;
   }
   while (true) {
-    if (!bar_wait(S.full(), S.ph, dead)) return;
+    if (!bar_wait(S.full(), S.ph, dead, P.pair_limit)) {
+      give_up(dead, status);
+      return;
+    }
     const int4 h = *reinterpret_cast<const int4*>(S.at());
     if (h.z == kEnd) return;
     const int4 h1 = *reinterpret_cast<const int4*>(S.at() + 16);
@@ -875,10 +889,7 @@ __global__ void __launch_bounds__(64 * kPairs) k_refactor(DPlan P, const double*
     __syncwarp();
     if (!(staged ? grid_updates<true>(P, cbuf - s0, lu, S, status, dead)
                  : grid_updates<false>(P, big, lu, S, status, dead))) {
-      if (lane == 0) {
-        *dead = 1;
-        atomicCAS(status, DS_OK, DS_TIMEOUT);
-      }
+      give_up(dead, status);
       return;
     }
     if (pc.want != nullptr)
@@ -1435,7 +1446,7 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
       const int4 C = __ldg(S.chunks + c);
       const int2 s0 = lane < C.w ? __ldg(S.segs + C.z + lane) : end;
       const int2 s1 = lane + 32 < C.w ? __ldg(S.segs + C.z + lane + 32) : end;
-      if (!bar_wait(bar0 + 8 * (2 + h), (c >> 1 & 1) ^ 1u, dead)) break;
+      if (!bar_wait(bar0 + 8 * (2 + h), (c >> 1 & 1) ^ 1u, dead, 8 * kSpinLimit)) break;
       int2* const sg = sseg + h * (kSolveSegs + 1);
       sg[lane] = s0;
       sg[lane + 32] = s1;
@@ -1458,7 +1469,7 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
   for (int c = 0; c < S.nchunks; ++c) {
     if (kStaged) {
       if (tid >= kSolveRow) break;
-      if (!bar_wait(bar0 + 8 * (c & 1), c >> 1 & 1, dead)) {
+      if (!bar_wait(bar0 + 8 * (c & 1), c >> 1 & 1, dead, 8 * kSpinLimit)) {
         *dead = 1;
         atomicCAS(status, DS_OK, DS_TIMEOUT);
         break;
