@@ -685,8 +685,8 @@ __device__ __forceinline__ void bar_arrive(unsigned b) {
 __device__ __forceinline__ void bar_arrive_copies(unsigned b) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(b) : "memory");
 }
-// Waits for the end of a barrier's phase; false when the pair has given up or
-// the wait runs out.
+// Waits for the end of a barrier's phase; false when the pair has given up
+// (dead, where there is one) or the wait runs out.
 __device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile int* dead,
                                          unsigned limit) {
   for (unsigned spins = 0;; ++spins) {
@@ -699,7 +699,7 @@ __device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, volatile i
         : "r"(b), "r"(parity)
         : "memory");
     if (__all_sync(FULL, done)) return true;
-    if (__any_sync(FULL, *dead != 0 || spins >= limit)) return false;
+    if (__any_sync(FULL, (dead != nullptr && *dead != 0) || spins >= limit)) return false;
     if (spins > 256) __nanosleep(100);
   }
 }
@@ -1322,9 +1322,26 @@ __device__ __forceinline__ void bulk_copy(unsigned d, const void* g, unsigned n,
       : "memory");
 }
 
+// Whether `ok` holds in all four compute warps (their barrier, as bar.sync 1).
+__device__ __forceinline__ bool all_rows(bool ok) {
+  unsigned r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
 // kStaged (programs of kSolveStaged slots or more): the slots come ready from
 // k_solve_slots, a chunk in two bulk copies by one warp, and the loads of eight
-// loader warps no longer share the SM's load unit with the rows. Measured, 801 k
+// loader warps no longer share the SM's load unit with the rows. A wait for a
+// chunk that runs out ends the solve (DS_TIMEOUT): the compute warps agree on it,
+// as one that left alone would be missing at the others' barriers, and the
+// copying warp stays until its last copies have landed. Measured, 801 k
 // slots (15,403 rows): 1.69 -> 1.45 ms with the layout's 11 us; 96 k slots 234 -> 229
 // us, 42 k slots 112 -> 114 us, 122 slots 7.3 -> 9.3 us.
 template <bool kStaged>
@@ -1332,7 +1349,7 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
     k_solve_steps(SolveSched S, int n, const int* __restrict__ in, const int* __restrict__ outp,
                   const int* __restrict__ dslot, const double* __restrict__ rhs,
                   const double* __restrict__ ax, const double* __restrict__ lu, double* rec,
-                  double* out, const int* skip, int* status) {
+                  double* out, const int* skip, int* status, unsigned pair_limit) {
   if (skip != nullptr && __ldcg(skip) != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* const T = reinterpret_cast<double*>(smem_raw);  // the solution, a spare entry at n
@@ -1441,12 +1458,16 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
   __syncthreads();
   if (kStaged && tid >= kSolveRow) {  // the copying warp
     const int2 end = make_int2(3, -1);
-    for (int c = 0; c < S.nchunks; ++c) {
+    int c = 0;  // chunks issued
+    for (; c < S.nchunks; ++c) {
       const int h = c & 1;
       const int4 C = __ldg(S.chunks + c);
       const int2 s0 = lane < C.w ? __ldg(S.segs + C.z + lane) : end;
       const int2 s1 = lane + 32 < C.w ? __ldg(S.segs + C.z + lane + 32) : end;
-      if (!bar_wait(bar0 + 8 * (2 + h), (c >> 1 & 1) ^ 1u, dead, 8 * kSpinLimit)) break;
+      if (!bar_wait(bar0 + 8 * (2 + h), (c >> 1 & 1) ^ 1u, dead, pair_limit)) {
+        give_up(dead, status);
+        break;
+      }
       int2* const sg = sseg + h * (kSolveSegs + 1);
       sg[lane] = s0;
       sg[lane + 32] = s1;
@@ -1465,13 +1486,14 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
       }
       __syncwarp();
     }
+    for (int q = max(c - 2, 0); q < c; ++q)  // the last copy into either half
+      bar_wait(bar0 + 8 * (q & 1), q >> 1 & 1, nullptr, 8 * kSpinLimit);
   }
   for (int c = 0; c < S.nchunks; ++c) {
     if (kStaged) {
       if (tid >= kSolveRow) break;
-      if (!bar_wait(bar0 + 8 * (c & 1), c >> 1 & 1, dead, 8 * kSpinLimit)) {
-        *dead = 1;
-        atomicCAS(status, DS_OK, DS_TIMEOUT);
+      if (!all_rows(bar_wait(bar0 + 8 * (c & 1), c >> 1 & 1, dead, pair_limit))) {
+        give_up(dead, status);
         break;
       }
     }
@@ -2353,7 +2375,7 @@ void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const
     k_solve_slots<<<(P.ss.nslots + 255) / 256, 256, 0, s>>>(P.ss, P.n, ax, lu, P.skip);
   kernel<<<1, staged ? kSolveRow + 32 : kSolveStepsThreads, bytes, s>>>(
       P.ss, P.n, transpose ? P.out_col : P.in_row, transpose ? P.in_row : P.out_col, P.dslot, rhs,
-      ax, lu, rec, out, P.skip, status);
+      ax, lu, rec, out, P.skip, status, P.pair_limit);
 }
 
 bool solve_groups_fit(const DPlan& P) {

@@ -64,8 +64,9 @@ struct DPlan {
   // Polls of a dependency flag before a waiting warp gives up and reports
   // DS_TIMEOUT (kSpinLimit unless the handle sets another).
   unsigned spin_limit;
-  // Polls of a barrier that another warp of the block arrives at (k_refactor's
-  // pairs): above every wait the other warp can be in.
+  // Polls of a barrier that another warp of the block or its copies arrive at
+  // (k_refactor's pairs, k_solve_steps): above every wait the other warp can be
+  // in.
   unsigned pair_limit;
   // When set, the refactorization and solve kernels do nothing while *skip is not
   // zero (a Newton iteration launched before the one ahead of it was known to end

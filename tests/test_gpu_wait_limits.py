@@ -1,6 +1,7 @@
 """Waits of a block's warps on one another that run out (the refactorization's
-loader and computing warps): the call reports DEVICE_TIMEOUT, never a factor
-that was not finished, and the kernel ends. A short limit of polls makes the
+loader and computing warps, the step-program solve's copying and compute
+warps): the call reports DEVICE_TIMEOUT, never a result that was not finished,
+and the kernel ends. A short limit of polls makes the
 waits run out; with the default limit the same handle factors as before."""
 import numpy as np
 import pytest
@@ -74,3 +75,38 @@ def test_the_newton_loop_ends_on_it(monkeypatch):
     g.set_spin_limit(0)
     again = newton_dc(g, dc, cfg)
     assert again.iterations == ok.iterations and np.array_equal(again.x, ok.x)
+
+
+@pytest.mark.parametrize("polls", [1, 4, 64, 4096])
+def test_a_staged_solve_that_gives_up_is_reported(polls, monkeypatch):
+    """The step program with its slots copied in bulk: the compute warps wait
+    for a chunk, the copying warp for a free half."""
+    monkeypatch.setenv("GPUKLU_SOLVE_STAGED", "0")
+    n, ap, ai, ax, rhs = _system("mesh")
+    g = GpuKluSolver(n, pivot_mode=N.PIVOT_EXACT)
+    g.factor(ap, ai, ax)
+    want = {}
+    for t in (False, True):
+        want[t] = rhs.copy()
+        (g.tsolve if t else g.solve)(want[t])
+    monkeypatch.setenv("GPUKLU_PAIR_POLLS", str(polls))
+    g.set_spin_limit(0)
+    gave_up = 0
+    for k in range(12):
+        x = rhs.copy()
+        try:
+            (g.tsolve if k % 2 else g.solve)(x)
+        except SolverError as e:
+            assert e.status == N.DEVICE_TIMEOUT, e
+            gave_up += 1
+            continue
+        assert np.array_equal(x, want[bool(k % 2)])
+    if polls == 1:
+        assert gave_up > 0, "no wait ran out at one poll"
+    monkeypatch.delenv("GPUKLU_PAIR_POLLS")
+    g.set_spin_limit(0)
+    for t in (False, True):
+        x = rhs.copy()
+        (g.tsolve if t else g.solve)(x)
+        assert np.array_equal(x, want[t])
+    g.close()
