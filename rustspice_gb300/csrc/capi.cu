@@ -249,7 +249,7 @@ void solve_op_list(const gk::Plan& p, std::vector<int4>& ops, bool transpose) {
 // beside the solution vector of n rows in one block's shared memory, or 0.
 int solve_chunk(int n) {
   for (int ch = 1024; ch >= 32 && n > 0; ch /= 2)
-    if (gk::solve_steps_bytes(n, ch) <= (size_t)(227 * 1024)) return ch;
+    if (gk::solve_steps_bytes(n, ch) <= gk::kSolveSteps) return ch;
   return 0;
 }
 

@@ -2359,7 +2359,7 @@ void launch_solve_cta(const DPlan& P, const double* rhs, const double* ax, const
 
 bool solve_steps_fits(const DPlan& P) {
   return P.n > 0 && P.ss.nchunks > 0 &&
-         solve_steps_bytes(P.n, P.ss.chunk) <= (size_t)smem_optin();
+         solve_steps_bytes(P.n, P.ss.chunk) + 64 <= (size_t)smem_optin();
 }
 
 void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,

@@ -35,6 +35,9 @@ struct SolveSched {
 };
 // Shared memory of k_solve_steps: the solution and a spare entry, then twice
 // a chunk's slots (two doubles, two words) and segments.
+// Its barriers (36 bytes) come out of the same 227 KB: kSolveSteps is what they
+// leave.
+constexpr size_t kSolveSteps = 227 * 1024 - 64;
 inline size_t solve_steps_bytes(int n, int chunk) {
   return (size_t)8 * ((n + 2) & ~1) + (size_t)2 * chunk * 24 + (size_t)2 * (kSolveSegs + 1) * 8;
 }
