@@ -94,28 +94,23 @@ __global__ void __launch_bounds__(32, kContWarps) k_batch_cont(BatchArgs A) {
     // ---- the next program with instances left, and up to M of them
     // (every pass either takes instances or moves the cursor on, so the
     // loop ends)
+    // Every lane takes the same turns; lane 0 alone in the loop would leave the
+    // warp diverged, lane 0 behind the others, for all that follows (measured:
+    // an iteration of a 210-stage chain 750 k cycles instead of 190 k).
     int g = -1;
     unsigned k0 = 0, cnt = 0;
-    if (lane == 0) {
-      while (true) {
-        const unsigned c = *(volatile unsigned*)A.cont_cursor;
-        if (c >= (unsigned)A.cont_ngroups) break;
-        const int gg = A.cont_groups[c];
-        const unsigned k = atomicAdd(&A.gnext2[gg], (unsigned)M);
-        const unsigned count = (unsigned)A.groups[gg].inst_count;
-        if (k < count) {
-          g = gg;
-          k0 = k;
-          cnt = count;
-          break;
-        }
-        atomicCAS(A.cont_cursor, c, c + 1);
-      }
+    while (true) {
+      unsigned c = 0;
+      if (lane == 0) c = *(volatile unsigned*)A.cont_cursor;
+      c = __shfl_sync(kFullMask, c, 0);
+      if (c >= (unsigned)A.cont_ngroups) return;
+      g = A.cont_groups[c];
+      if (lane == 0) k0 = atomicAdd(&A.gnext2[g], (unsigned)M);
+      k0 = __shfl_sync(kFullMask, k0, 0);
+      cnt = (unsigned)A.groups[g].inst_count;
+      if (k0 < cnt) break;
+      if (lane == 0) atomicCAS(A.cont_cursor, c, c + 1);
     }
-    g = __shfl_sync(kFullMask, g, 0);
-    k0 = __shfl_sync(kFullMask, k0, 0);
-    cnt = __shfl_sync(kFullMask, cnt, 0);
-    if (g < 0) return;
     const GroupHdr G = A.groups[g];
     const bt::Prog P = bt::global_view(A, G);
     const int n = P.n, nc = P.nc;
