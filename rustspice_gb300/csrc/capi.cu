@@ -273,8 +273,9 @@ int solve_op_steps(int n, const std::vector<int4>& ops, std::vector<int>& step) 
   return nsteps;
 }
 
-// The operations by step (the plan's step program). Plans whose solution
-// vector does not fit one block's shared memory get none.
+// The operations by step: what k_solve_list runs, and what the program of
+// k_solve_steps is laid out from. Plans whose solution vector does not fit one
+// block's shared memory get none.
 void make_solve_steps(const gk::Plan& p, std::vector<int4>& out_ops, std::vector<i32>& out_ptr) {
   out_ops.clear();
   out_ptr.clear();
@@ -579,6 +580,20 @@ struct SolveDev {
   DBuf<int2> segs, terms;
   DBuf<double2> vc;
   DBuf<uint2> ad;
+  DBuf<int4> list;
+  DBuf<i32> ptr;
+  cudaError_t upload_list(const gk::Plan& p, cudaStream_t s, gk::SolveSched& d) {
+    std::vector<int4> h;
+    std::vector<i32> hp;
+    make_solve_steps(p, h, hp);
+    cudaError_t e = list.upload(h, s);
+    if (e == cudaSuccess) e = ptr.upload(hp, s);
+    d = gk::SolveSched{};
+    d.nsteps = hp.empty() ? 0 : (int)hp.size() - 1;
+    d.list = list.p;
+    d.ptr = ptr.p;
+    return e;
+  }
   cudaError_t upload(const SolveProgram& sp, cudaStream_t s, gk::SolveSched& d) {
     cudaError_t e = ops.upload(sp.ops, s);
     if (e == cudaSuccess) e = chunks.upload(sp.chunks, s);
@@ -591,7 +606,7 @@ struct SolveDev {
     if (e == cudaSuccess && staged) e = ad.resize(sp.ops.size());
     d = gk::SolveSched{(int)sp.chunks.size(), sp.chunk, sp.width, ops.p, chunks.p, chains.p,
                        segs.p, terms.p, (int)sp.ops.size(), staged ? vc.p : nullptr,
-                       staged ? ad.p : nullptr};
+                       staged ? ad.p : nullptr, 0, nullptr, nullptr};
     return e;
   }
 };
@@ -638,11 +653,13 @@ struct PlanDev {
     if (e == cudaSuccess) e = cs_gop.upload(hgo, s);
     SolveProgram sp;
     const char* ess = getenv("GPUKLU_SOLVE_STEPS");
-    if (solves && !(ess && ess[0] == '0')) make_solve_program(p, false, sp);
+    const bool steps = solves && !(ess && ess[0] == '0');
+    const bool by_list = steps && solve_chunk(p.n) < gk::kSolveMinChunk;
+    if (steps && !by_list) make_solve_program(p, false, sp);
     updates = (int64_t)p.upd_dst.size();
     if (e == cudaSuccess) e = order.upload(column_order(p), s);
     gk::DPlan d{};
-    if (e == cudaSuccess) e = ss.upload(sp, s, d.ss);
+    if (e == cudaSuccess) e = by_list ? ss.upload_list(p, s, d.ss) : ss.upload(sp, s, d.ss);
     d.n = p.n;
     d.order = order.p;
     for (int k = 0; k < p.n; ++k) d.max_col = std::max<int>(d.max_col, p.col_ptr[k + 1] - p.col_ptr[k]);
@@ -1358,11 +1375,12 @@ struct gpuklu_handle {
       if (!sync) return GPUKLU_OK;
       return check_status("dense solve");
     }
-    if (steps_sol) {
-      if (transpose && pd.dpt.ss.nchunks == 0) {
-        const cudaError_t e = pd.upload_transpose(plan, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "transpose solve program");
-      }
+    if (steps_sol && transpose && pd.dpt.ss.nchunks == 0) {
+      const cudaError_t e = pd.upload_transpose(plan, stream);
+      if (e != cudaSuccess) return cuda_fail(e, "transpose solve program");
+    }
+    // (a transpose program needs its chunks: without room for any, the grid)
+    if (steps_sol && (!transpose || pd.dpt.ss.nchunks > 0)) {
       gk::launch_solve_steps(transpose ? pd.dpt : pd.dp, transpose, d_rhs.p, d_ax.p, d_lu.p,
                              d_rec.p, d_out.p, d_status.p, stream);
       if (!sync) return GPUKLU_OK;

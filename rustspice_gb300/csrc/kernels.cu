@@ -1569,6 +1569,75 @@ __global__ void __launch_bounds__(kStaged ? kSolveRow + 32 : kSolveStepsThreads)
   for (int i = tid; i < n; i += blockDim.x) out[outp[i]] = T[i];
 }
 
+// The step program of a solution that fills the shared memory: each thread
+// reads its operation, its matrix value and (for a division) its reciprocal
+// from memory two steps ahead, none of which depends on the solution; a barrier
+// a step. The quotients are k_solve_steps' (Markstein). 430 to 620 cycles a step.
+constexpr int kSolveListThreads = 128;
+
+__device__ __forceinline__ double div_markstein(double a, double b, double y) {
+  const double q = a * y;
+  if (exponent_of(a) - 64u > 1919u || exponent_of(b) - 64u > 1919u || exponent_of(q) - 64u > 1919u)
+    return a / b;
+  const double r = fma(-b, q, a);
+  return fma(r, y, q);
+}
+
+struct ListOp {
+  int4 o;
+  double v, y;
+};
+
+__global__ void __launch_bounds__(kSolveListThreads)
+    k_solve_list(SolveSched S, int n, const int* __restrict__ in, const int* __restrict__ outp,
+                 const int* __restrict__ dslot, const double* __restrict__ rhs,
+                 const double* __restrict__ ax, const double* __restrict__ lu, double* rec,
+                 double* out, const int* skip) {
+  if (skip != nullptr && __ldcg(skip) != 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* const T = reinterpret_cast<double*>(smem_raw);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < n; i += blockDim.x) {
+    T[i] = rhs[in[i]];
+    rec[i] = 1.0 / lu[dslot[i]];
+  }
+  __syncthreads();
+  const int* const sp = S.ptr;
+  const int ns = S.nsteps, nops = sp[ns];
+  auto fetch = [&](int p) {
+    ListOp f{make_int4(0, -1, 0, 3), 0.0, 0.0};
+    if (p < nops) {
+      f.o = __ldg(S.list + p);
+      f.v = f.o.w == 2 ? __ldg(ax + f.o.z) : __ldg(lu + f.o.z);
+      if (f.o.w == 1) f.y = __ldcg(rec + f.o.x);  // written above by this block
+    }
+    return f;
+  };
+  auto exec = [&](const ListOp& f) {
+    const int d = f.o.x;
+    if (f.o.w == 1)
+      T[d] = div_markstein(T[d], f.v, f.y);
+    else if (f.o.w != 3)
+      T[d] = __dsub_rn(T[d], __dmul_rn(f.v, T[f.o.y]));
+  };
+  int s0 = sp[0], s1 = sp[min(1, ns)], s2 = sp[min(2, ns)], s3 = sp[min(3, ns)];
+  ListOp f0 = fetch(s0 + tid), f1 = fetch(s1 + tid);
+  for (int t = 0; t < ns; ++t) {
+    const ListOp f2 = fetch(s2 + tid);
+    const int s4 = sp[min(t + 4, ns)];
+    if (s0 + tid < s1) exec(f0);
+    for (int p = s0 + tid + kSolveListThreads; p < s1; p += kSolveListThreads) exec(fetch(p));
+    __syncthreads();
+    s0 = s1;
+    s1 = s2;
+    s2 = s3;
+    s3 = s4;
+    f0 = f1;
+    f1 = f2;
+  }
+  for (int i = tid; i < n; i += blockDim.x) out[outp[i]] = T[i];
+}
+
 // --------------------------------------------------------------- devices
 // Level-1 MOSFET exactly as the reference evaluates it
 // (crates/sim-devices/src/bsim/evaluate.rs:285-356 via mod.rs:440-455).
@@ -2358,12 +2427,21 @@ void launch_solve_cta(const DPlan& P, const double* rhs, const double* ax, const
 }
 
 bool solve_steps_fits(const DPlan& P) {
+  if (P.n > 0 && P.ss.nsteps > 0) return (size_t)8 * P.n + 16 <= (size_t)smem_optin();
   return P.n > 0 && P.ss.nchunks > 0 &&
          solve_steps_bytes(P.n, P.ss.chunk) + 64 <= (size_t)smem_optin();
 }
 
 void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const double* ax,
                         const double* lu, double* rec, double* out, int* status, cudaStream_t s) {
+  const int *const in = transpose ? P.out_col : P.in_row, *const outp = transpose ? P.in_row : P.out_col;
+  if (P.ss.nsteps > 0) {
+    const size_t bytes = (size_t)8 * P.n;
+    raise_smem_limit<k_solve_list>(bytes);
+    k_solve_list<<<1, kSolveListThreads, bytes, s>>>(P.ss, P.n, in, outp, P.dslot, rhs, ax, lu, rec,
+                                                     out, P.skip);
+    return;
+  }
   const size_t bytes = solve_steps_bytes(P.n, P.ss.chunk);
   const bool staged = P.ss.vc != nullptr;
   const auto kernel = staged ? k_solve_steps<true> : k_solve_steps<false>;
@@ -2374,8 +2452,7 @@ void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const
   if (staged)
     k_solve_slots<<<(P.ss.nslots + 255) / 256, 256, 0, s>>>(P.ss, P.n, ax, lu, P.skip);
   kernel<<<1, staged ? kSolveRow + 32 : kSolveStepsThreads, bytes, s>>>(
-      P.ss, P.n, transpose ? P.out_col : P.in_row, transpose ? P.in_row : P.out_col, P.dslot, rhs,
-      ax, lu, rec, out, P.skip, status, P.pair_limit);
+      P.ss, P.n, in, outp, P.dslot, rhs, ax, lu, rec, out, P.skip, status, P.pair_limit);
 }
 
 bool solve_groups_fit(const DPlan& P) {

@@ -22,6 +22,12 @@ constexpr unsigned kSpinLimit = 1u << 22;
 constexpr int kSolveRow = 128;   // compute threads
 constexpr int kSolveStaged = 1 << 18;  // slots of a program laid out ahead
 constexpr int kSolveSegs = 64;   // segments of a chunk, at most
+// Slots of a chunk, at least. Smaller ones spend the time on the barrier and
+// the loads' latency between them. Measured, forward, this program against the
+// list, ms: meshes of 167 a side (27,891 rows, chunks of 128) 6.2 / 8.2, 168 (64)
+// 11.9 / 8.7, 169 (32) 21.6 / 8.7; tridiagonal systems of 28,200 rows (64) 26.3 /
+// 27.8, 28,700 (32) 40.2 / 28.3.
+constexpr int kSolveMinChunk = 128;
 enum { kSolveSegSolo = 0, kSolveSegWide = 1, kSolveSegChain = 2 };
 struct SolveSched {
   int nchunks, chunk, width;
@@ -32,6 +38,12 @@ struct SolveSched {
   int nslots;
   double2* vc;
   uint2* ad;
+  // Solutions that leave no room for chunks of kSolveMinChunk slots: the
+  // operations by step instead (k_solve_list), list[ptr[t]] to list[ptr[t + 1]]
+  // those of step t. 0 steps: none.
+  int nsteps;
+  const int4* list;
+  const int* ptr;
 };
 // Shared memory of k_solve_steps: the solution and a spare entry, then twice
 // a chunk's slots (two doubles, two words) and segments.

@@ -1,13 +1,12 @@
 """The step-program solve at the sizes where its chunks change: the last rows
 count with chunks of 1024, 512, ... slots beside the solution in one block's 227
-KB, and the ones around it. Against the oracle bit for bit; the transpose
-against SciPy."""
+KB, and the ones around it. Against the grid solve (which other tests hold to the
+oracle) bit for bit; the transpose against SciPy."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
 import scipy.sparse.linalg as sla
 
-from oracle import pyoracle as po
 from rustspice_gb300 import native as N
 from rustspice_gb300.solver import GpuKluSolver
 
@@ -37,11 +36,13 @@ def test_sizes(n, staged, monkeypatch):
     A.sort_indices()
     ap, ai, ax = A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data.copy()
     b = rng.standard_normal(n)
-    o = po.Solver("nativeklu_exact", n)
-    o.prepare(n)
-    assert o.analyze(ap, ai) == 0 and o.factor(ap, ai, ax) == 0
-    st, want = o.solve(b)
-    assert st == 0
+    with monkeypatch.context() as m:
+        m.setenv("GPUKLU_ONE_BLOCK", "0")
+        r = GpuKluSolver(n, pivot_mode=N.PIVOT_EXACT)
+        r.factor(ap, ai, ax)
+        want = b.copy()
+        r.solve(want)
+        r.close()
     g = GpuKluSolver(n, pivot_mode=N.PIVOT_EXACT)
     g.factor(ap, ai, ax)
     x = b.copy()
