@@ -531,6 +531,22 @@ void make_solve_program(const gk::Plan& p, bool transpose, SolveProgram& out) {
   lay_out_solve(ops, best_step, best_ns, best_chain, best_chains, chunk, out);
 }
 
+// Whether a transpose solve goes over the grid although it has a step program:
+// one block takes a row's operations at the rate of one SM, the grid takes every
+// block of the matrix at once, at about 2 us a row of the largest. It wins where
+// there are many uncoupled blocks, counted as the plan's slots over the largest
+// block's, times the rows. Measured, program against grid, us (rows times blocks
+// in millions): 2000 of 8 rows 298 / 125 (32), 1000 of 8 166 / 117 (8), 300 of 60
+// 1633 / 1473 (5.4), 500 of 16 303 / 239 (4), grids of 10 x 10 200 times 691 / 660
+// (4); 300 of 30 471 / 592 (2.7), 400 of 8 90 / 92 (1.3), 100 of 100 1501 / 2332 (1).
+bool many_blocks(const gk::Plan& p) {
+  if (p.nblocks < 2 || p.noffdiag > 0) return false;
+  int most = 1;
+  for (int b = 0; b < p.nblocks; ++b)
+    most = std::max(most, p.col_ptr[p.block_ptr[b + 1]] - p.col_ptr[p.block_ptr[b]]);
+  return (double)p.n * ((double)p.nslots() / most) >= 3.6e6;
+}
+
 // The columns as the grid refactorization hands them out: by the number of
 // columns that wait for one another behind it, the longest chain first (a
 // column comes after every column it depends on).
@@ -967,6 +983,7 @@ struct gpuklu_handle {
   bool cta_ref = false, cta_sol = false;  // one-block refactor / solve for this plan
   bool cta_grp = false;  // the one-block solve over groups of uncoupled BTF blocks
   bool steps_sol = false;  // the solve as a step program (k_solve_steps)
+  bool grid_tsol = false;  // but the transpose solve over the grid all the same
   DBuf<double> d_rec;      // its scratch: the pivots' reciprocals
   // Plans with up to this many multiply-subtract pairs refactor in one block:
   // its hops through shared memory are shorter than the grid kernel's through
@@ -1068,6 +1085,7 @@ struct gpuklu_handle {
     // the step-program solve (one block) when the plan has one
     // (GPUKLU_SOLVE_STEPS=0: no step programs)
     steps_sol = allow && gk::solve_steps_fits(pd.dp);
+    grid_tsol = many_blocks(plan);
     if (steps_sol && e == cudaSuccess) e = d_rec.resize(std::max<int64_t>(n, 1));
     if (e != cudaSuccess) return cuda_fail(e, "solve scratch");
     // the solve split over groups of uncoupled BTF blocks when one block does
@@ -1375,12 +1393,13 @@ struct gpuklu_handle {
       if (!sync) return GPUKLU_OK;
       return check_status("dense solve");
     }
-    if (steps_sol && transpose && pd.dpt.ss.nchunks == 0) {
+    const bool by_steps = steps_sol && !(transpose && grid_tsol);
+    if (by_steps && transpose && pd.dpt.ss.nchunks == 0) {
       const cudaError_t e = pd.upload_transpose(plan, stream);
       if (e != cudaSuccess) return cuda_fail(e, "transpose solve program");
     }
     // (a transpose program needs its chunks: without room for any, the grid)
-    if (steps_sol && (!transpose || pd.dpt.ss.nchunks > 0)) {
+    if (by_steps && (!transpose || pd.dpt.ss.nchunks > 0)) {
       gk::launch_solve_steps(transpose ? pd.dpt : pd.dp, transpose, d_rhs.p, d_ax.p, d_lu.p,
                              d_rec.p, d_out.p, d_status.p, stream);
       if (!sync) return GPUKLU_OK;
