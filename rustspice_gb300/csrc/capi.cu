@@ -2194,6 +2194,7 @@ struct gpuklu_batch {
   struct ContClass {
     int m = 1, grid = 0, slice = 0, dvs = 0, dvx = 0, first = 0, count = 0;
     long long dv_off = 0;
+    bool lanes = false;  // the lane kernel runs its instances' first iterations
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
   };
@@ -2861,6 +2862,38 @@ gk::NewtonCfg to_newton_cfg(const gpuklu_newton_config& cfg) {
   return c;
 }
 
+// How the batch's small programs run: instances per warp, and whether the lane
+// kernel (one instance per lane) runs their first iterations. Small programs
+// leave most of a warp's lanes without work; where there are far more instances
+// than the device holds at once, two share a warp (a row's FP64 instruction then
+// serves both), and the lane kernel, all of whose lanes work, comes first: its
+// six iterations take as long as one warp's, however many there are. Diode
+// circuits run about ten iterations, chains started from their nodeset three,
+// so the line for the lane kernel is lower for them. Programs of more than
+// kSmallProgram operations an iteration fill a warp's rows, and in the lane
+// kernel they outgrow the caches. Measured, ms, one per warp / two / lanes
+// first, then two (instances, operations): chains of 2 stages (122,000, 288) 4.12
+// / 2.60 / 1.57, 8 (122,000, 1012) 5.80 / 3.73 / 2.94, 8 (30,500) 2.15 / 1.80 /
+// 2.31, 64 (30,500, 8 k) 6.79 / 6.63 / 12.4; meshes of 3 x 3 (12,200, 500) 3.22 /
+// 2.42 / 2.24, 4 x 4 (30,500, 998) 8.01 / 5.93 / 4.69, 6 x 6 (12,200, 2946) 6.93 /
+// 6.28 / 7.41; chains of 2 to 10 stages (124,928, 772, nine programs in five
+// classes) 6.21 / 4.78 / 3.33; 4 x 4, three instances of a program (6,000) 3.90 / 4.29 / 5.37;
+// 256 chains of 2 stages 1.00 / 1.03 / 1.13.
+constexpr int64_t kSmallProgram = 3500;
+// Instances per warp of a class: inst instances of count programs, flops
+// operations an iteration on average, slots instances on the device at one per
+// warp.
+int instances_per_warp(int64_t inst, int count, int64_t flops, int64_t slots) {
+  if (const char* e = getenv("GPUKLU_CONT_M")) return e[0] == '2' ? 2 : 1;
+  return flops <= kSmallProgram && inst >= 3 * slots && inst >= 8 * (int64_t)count ? 2 : 1;
+}
+// Whether the lane kernel comes first for the batch's small programs (inst
+// instances of them).
+bool lanes_first(int64_t inst, int64_t flops, bool diodes) {
+  if (const char* e = getenv("GPUKLU_LANE_PHASE")) return e[0] == '1';
+  return inst > 0 && inst >= (diodes ? 5000 + 10 * flops : 20000 + 35 * flops);
+}
+
 // Groups, programs, constants and launch classes of a batch. transient: the
 // circuits are compiled with their capacitors' backward-Euler companions
 // for step dt (pivots are chosen on the matrix with those conductances).
@@ -3200,15 +3233,16 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
     const char* etgt = getenv("GPUKLU_LANE_TARGET");
     const int target = etgt ? std::max(32, atoi(etgt)) : 32;
     long long lregion = 0;
-    for (int g : gorder) {
+    auto add_tiles = [&](int g) {
       const gk::GroupHdr& h = B->groups[g];
-      if (h.inst_count == 0) continue;
       const int nt = std::max(1, (h.inst_count + target - 1) / target);
       for (int t = 0; t < nt; ++t) B->ltiles.push_back(g);
       lregion = std::max<long long>(lregion, (long long)h.node_count + h.n + h.ndv + h.nslots +
                                                  h.noffd + 4LL * h.ndev);
-    }
-    if (B->lanes && !B->ltiles.empty()) {
+    };
+    bool any = false;
+    for (int g : gorder) any |= B->groups[g].inst_count > 0;
+    if (B->lanes && any) {
       if (e == cudaSuccess) e = B->d_gnext2.resize(std::max(ngr, 1));
       // Continuation kernel: a block (one warp) holds, per instance, T and the
       // LU values in shared memory, sized for the largest program of its
@@ -3216,13 +3250,6 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
       // its differences in a slice of global memory. A class takes the
       // programs down to 0.8 of its largest; the eighth takes the rest.
       const char* eck = getenv("GPUKLU_CONT_KERNEL");
-      // Instances per warp: one. GPUKLU_CONT_M=2 puts two of a program in a
-      // warp (16 lanes each, a row's FP64 instruction serving both; the same
-      // results bit for bit): 976 instances take 10.0 ms against 7.2 ms, 249,856
-      // 64.7 ms against 65.2 ms, because an instance that runs to the
-      // iteration cap keeps its warp long after the other half has run out.
-      const char* ecm = getenv("GPUKLU_CONT_M");
-      const int cm = ecm && ecm[0] == '2' ? 2 : 1;
       const char* ecw = getenv("GPUKLU_CONT_WARPS");  // resident warps per SM and class
       int prio_low = 0, prio_high = 0;
       if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess)
@@ -3239,6 +3266,19 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
           if (B->groups[g].nchunk == 0) ok = false;
         }
       std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return need(x) > need(y); });
+      bool lanes = false;
+      {
+        int64_t inst = 0, flops = 0;
+        bool diodes = false;
+        for (int g : by) {
+          const gk::GroupHdr& h = B->groups[g];
+          if (B->group_flops[g] > kSmallProgram) continue;
+          inst += h.inst_count;
+          flops += B->group_flops[g] * h.inst_count;
+          for (int d = 0; d < h.ndev; ++d) diodes |= dev_type[h.dev_off + d] == 3;
+        }
+        lanes = lanes_first(inst, flops / std::max<int64_t>(inst, 1), diodes);
+      }
       std::vector<i32> cg;
       long long dv = 0;
       for (size_t q = 0; ok && q < by.size();) {
@@ -3246,13 +3286,14 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
         k.slice = need(by[q]);
         k.first = (int)cg.size();
         const bool rest = B->cont.size() == 7;
-        int64_t inst = 0;
+        int64_t inst = 0, flops = 0;
         std::vector<int> in;
         for (; q < by.size() && (rest || need(by[q]) * 5 >= k.slice * 4); ++q) {
           const gk::GroupHdr& h = B->groups[by[q]];
           k.dvx = std::max(k.dvx, (h.ndv + 3) & ~3);
           k.dvs = std::max(k.dvs, h.node_count);
           inst += h.inst_count;
+          flops += B->group_flops[by[q]] * h.inst_count;
           in.push_back(by[q]);
         }
         k.dvs = (k.dvx + 2 * k.dvs + 3) & ~3;
@@ -3262,9 +3303,13 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
         cg.insert(cg.end(), in.begin(), in.end());
         k.count = (int)in.size();
         int regs = 0, per_sm = 0;
-        for (k.m = cm; k.m >= 1; --k.m) {
-          gk::cont_kernel_info(k.m, k.slice, &regs, &per_sm);
-          if (per_sm > 0) break;
+        gk::cont_kernel_info(1, k.slice, &regs, &per_sm);
+        flops /= std::max<int64_t>(inst, 1);
+        k.lanes = lanes && (flops <= kSmallProgram || getenv("GPUKLU_LANE_PHASE"));
+        if (instances_per_warp(inst, k.count, flops, (int64_t)sm_count() * per_sm) == 2) {
+          int two = 0;
+          gk::cont_kernel_info(2, k.slice, &regs, &two);
+          if (two > 0) k.m = 2, per_sm = two;
         }
         if (per_sm <= 0) {
           ok = false;
@@ -3290,7 +3335,17 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
         if (e == cudaSuccess) e = B->d_cont_cursor.resize(B->cont.size());
         if (e == cudaSuccess) e = B->d_dv.resize((size_t)dv);
       }
-      if (!B->cont_kernel) {  // the lane kernel, then the warp classes
+      // the lane kernel's groups: of the classes that start with it, or every
+      // group in front of the warp classes
+      if (B->cont_kernel) {
+        for (const auto& k : B->cont)
+          if (k.lanes)
+            for (int q = 0; q < k.count; ++q) add_tiles(cg[k.first + q]);
+      } else {
+        for (int g : gorder)
+          if (B->groups[g].inst_count > 0) add_tiles(g);
+      }
+      if (!B->ltiles.empty()) {
         int regs = 0, bps = 0;
         gk::lanes_kernel_info(B->lane_wpb, &regs, &bps);
         const long long warps_max = (long long)sm_count() * std::max(bps, 1) * B->lane_wpb;
@@ -3822,11 +3877,23 @@ int gpuklu_batch_run(gpuklu_batch* b, const gpuklu_newton_config* cfg) {
   if (b->lanes && b->cont_kernel) {  // every class at once, the largest programs first
     cudaMemsetAsync(b->d_gnext2.p, 0, b->d_gnext2.n * sizeof(unsigned), s);
     cudaMemsetAsync(b->d_cont_cursor.p, 0, b->d_cont_cursor.n * sizeof(unsigned), s);
+    cudaEventRecord(b->start_ev, s);
+    const bool lane_phase = b->lane_cap > 0 && !b->ltiles.empty();
+    if (lane_phase) {  // the classes that start with it follow it, the others run beside it
+      cudaMemsetAsync(b->d_gnext.p, 0, b->d_gnext.n * sizeof(unsigned), s);
+      cudaMemsetAsync(b->d_lcounter.p, 0, sizeof(unsigned), s);
+      cudaMemsetAsync(b->d_cont_count.p, 0, b->d_cont_count.n * sizeof(unsigned), s);
+      gk::BatchArgs la = b->args;
+      la.cfg = c;
+      gk::launch_batch_lanes(la, b->lane_grid, b->lane_wpb, s);
+    }
     cudaEventRecord(b->ph_ev[1], s);
     for (const auto& k : b->cont) {
-      cudaStreamWaitEvent(k.stream, b->ph_ev[1], 0);
+      const bool parked = lane_phase && k.lanes;
+      cudaStreamWaitEvent(k.stream, parked ? b->ph_ev[1] : b->start_ev, 0);
       gk::BatchArgs ca = b->args;
       ca.cfg = c;
+      ca.cont_parked = parked ? 1 : 0;
       ca.cont_groups = b->d_cont_groups.p + k.first;
       ca.cont_ngroups = k.count;
       ca.cont_cursor = b->d_cont_cursor.p + (&k - b->cont.data());
@@ -4033,7 +4100,7 @@ int gpuklu_batch_info(const gpuklu_batch* b, int64_t* out) {
   if (!b) return GPUKLU_INVALID_MATRIX;
   for (int q = 0; q < 8; ++q) out[q] = 0;
   out[2] = (int64_t)b->groups.size();
-  out[6] = b->lanes && b->cont_kernel ? (int64_t)b->cont.size()
+  out[6] = b->lanes && b->cont_kernel ? (int64_t)b->cont.size() + (b->ltiles.empty() ? 0 : 1)
                                        : (int64_t)b->classes.size() + (b->lanes ? 1 : 0);
   out[7] = b->lanes && b->cont_kernel ? 1 : 0;  // the continuation kernel runs
   for (auto& C : b->classes) {  // the largest class (first) describes the launch

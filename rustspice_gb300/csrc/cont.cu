@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(32, kContWarps) k_batch_cont(BatchArgs A) {
       g = A.cont_groups[c];
       if (lane == 0) k0 = atomicAdd(&A.gnext2[g], (unsigned)M);
       k0 = __shfl_sync(kFullMask, k0, 0);
-      cnt = (unsigned)A.groups[g].inst_count;
+      cnt = A.cont_parked ? A.cont_count[g] : (unsigned)A.groups[g].inst_count;
       if (k0 < cnt) break;
       if (lane == 0) atomicCAS(A.cont_cursor, c, c + 1);
     }
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(32, kContWarps) k_batch_cont(BatchArgs A) {
       V[P.nv + 1] = 0.0;
     }
     const bool lists_fit = P.nheavy > 0 && P.nheavy <= LPI;
-    const int* const list = A.order + G.inst_begin;
+    const int* const list = (A.cont_parked ? A.cont_list : A.order) + G.inst_begin;
     int inst = k0 + sub < cnt ? list[k0 + sub] : -1;
     bool exhausted = inst < 0;
     int it = 0, total = 0, gstep = 0, ov_dev = -1;
@@ -135,17 +135,29 @@ __global__ void __launch_bounds__(32, kContWarps) k_batch_cont(BatchArgs A) {
     double damp = 0.0, prev = 0.0, gmin = 0.0, ov_val = 0.0;
     bool prev_exact = true;
     const double* dparams = nullptr;
-    auto start = [&]() {
+    auto start = [&]() {  // or where the lane kernel parked it, with its own sums
       dparams = A.dparams + A.inst_p_off[inst];
       ov_dev = A.inst_ov_dev[inst];
       ov_val = A.inst_ov_val[inst];
       xo = A.inst_x_off[inst];
+      prev_exact = true;
+      if (A.cont_parked) {
+        for (int i = sl; i < nc; i += LPI) X[i] = A.x_out[xo + i];
+        it = A.cont_it[inst];
+        total = A.cont_total[inst];
+        gstep = A.cont_gstep[inst];
+        damp = A.cont_damp[inst];
+        prev = A.cont_prev[inst];
+        gmin = cfg.gmin_steps == 0
+                   ? cfg.gmin
+                   : gstart + (cfg.gmin - gstart) * ((double)gstep / (double)cfg.gmin_steps);
+        return;
+      }
       const long long x0o = A.inst_x0_off[inst];
       for (int i = sl; i < nc; i += LPI) X[i] = x0o >= 0 ? A.x0[x0o + i] : 0.0;
       it = total = gstep = 0;
       damp = cfg.damping;
       prev = DBL_MAX;
-      prev_exact = true;
       gmin = cfg.gmin_steps == 0 ? cfg.gmin : gstart;
     };
     if (inst >= 0) start();

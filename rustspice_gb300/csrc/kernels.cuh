@@ -245,6 +245,7 @@ struct BatchArgs {
   long long dv_stride;         //   its differences at dv_x (dv_stride doubles per slot)
   long long dv_x;
   int slice;                   // shared doubles per instance slot: T, the LU values, two constants
+  int cont_parked;             // 1: the instances the lane kernel parked, not every one from its start
 };
 
 // Batched adaptive transient (atran.cu): per instance its time-dependent
