@@ -465,7 +465,7 @@ size_t sparse_smem(int n, int warps, bool masks) {
 
 }  // namespace
 
-AcShape ac_shape(int n, int nf, int sms) {
+AcShape ac_shape(int n, int nf, int sms, size_t limit) {
   AcShape s;
   // One warp per frequency from eight frequencies an SM on, else as many as
   // keep eight warps an SM busy, a column's updates and the masks spread over
@@ -482,7 +482,7 @@ AcShape ac_shape(int n, int nf, int sms) {
   const size_t slot = (size_t)16 * n * n;
   s.blocks = (int)std::min<long long>(
       std::min<long long>(nf, per_sm * sms),
-      (long long)std::max<size_t>(1, ((size_t)2 << 30) / slot));
+      (long long)std::max<size_t>(1, limit / slot));
   s.scratch_bytes = slot * s.blocks;
   s.mask_words = (size_t)2 * n * ((n + 31) / 32);
   return s;

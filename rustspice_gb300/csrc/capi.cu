@@ -1032,6 +1032,7 @@ struct gpuklu_handle {
   // Workspace of the AC sweep, kept between calls up to this size (a larger
   // one is the call's own).
   static constexpr size_t kAcKeep = (size_t)512 << 20;
+  static constexpr size_t kAcScratch = (size_t)2 << 30;
   DBuf<unsigned char> d_ac;
   // End the device Newton loop at the first non-finite iterate
   // (gpuklu_set_stop_on_nonfinite; off: the reference runs on to the cap).
@@ -1786,7 +1787,6 @@ int gpuklu_ac_sweep(gpuklu_handle* h, gpuklu_circuit* c, const double* x_dc, int
   mark(0, 0);
   for (int q = 0; q < ncell; ++q) mark(crow[q], ccol[q]);
   cudaStream_t s = h->stream;
-  const gk::AcShape shape = gk::ac_shape(n, (int)nf, sm_count());
   // every array of the call in one device workspace, the inputs first and
   // uploaded in one copy
   struct Part {
@@ -1813,15 +1813,33 @@ int gpuklu_ac_sweep(gpuklu_handle* h, gpuklu_circuit* c, const double* x_dc, int
   const size_t o_st = part(&zero, sizeof(int)), upload = top;
   const size_t o_ax = part(nullptr, 8 * c->ai.size()), o_rc = part(nullptr, 8 * (size_t)c->ncontrib),
                o_r = part(nullptr, 8 * (size_t)n), o_re = part(nullptr, 8 * (size_t)nf * n),
-               o_im = part(nullptr, 8 * (size_t)nf * n), o_m = part(nullptr, shape.scratch_bytes),
-               o_mw = part(nullptr, shape.masks_shared ? 0 : 4 * shape.mask_words * shape.blocks);
+               o_im = part(nullptr, 8 * (size_t)nf * n);
   std::vector<unsigned char> blob(upload, 0);
   for (const Part& q : parts)
     if (q.src && q.bytes) std::memcpy(blob.data() + q.at, q.src, q.bytes);
-  // the workspace stays with the handle up to kAcKeep bytes
+  // The blocks' matrices last: as many as kAcScratch bytes hold, a quarter of
+  // that and again while the device has no room for them (a system of up to 118
+  // unknowns needs 0.2 MB for one block; more blocks are only faster). The
+  // workspace stays with the handle up to kAcKeep bytes.
+  const char* el = getenv("GPUKLU_AC_SCRATCH");  // bytes
+  size_t limit = el ? strtoull(el, nullptr, 10) : gpuklu_handle::kAcScratch;
+  gk::AcShape shape;
+  size_t o_m = 0, o_mw = 0;
   DBuf<unsigned char> once;
-  DBuf<unsigned char>& ws = top <= gpuklu_handle::kAcKeep ? h->d_ac : once;
-  cudaError_t e = ws.resize(top);
+  DBuf<unsigned char>* buf = nullptr;
+  cudaError_t e = cudaSuccess;
+  const size_t fixed = top;
+  for (;; limit = shape.scratch_bytes / 4) {
+    top = fixed;
+    shape = gk::ac_shape(n, (int)nf, sm_count(), limit);
+    o_m = part(nullptr, shape.scratch_bytes);
+    o_mw = part(nullptr, shape.masks_shared ? 0 : 4 * shape.mask_words * shape.blocks);
+    buf = top <= gpuklu_handle::kAcKeep ? &h->d_ac : &once;
+    if (buf == &once) h->d_ac.release();
+    e = buf->resize(top);
+    if (e != cudaErrorMemoryAllocation || shape.blocks <= 1) break;
+  }
+  DBuf<unsigned char>& ws = *buf;
   if (e == cudaSuccess) e = cudaMemcpyAsync(ws.p, blob.data(), upload, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return h->cuda_fail(e, "ac upload");
   auto dbl = [&](size_t at) { return reinterpret_cast<double*>(ws.p + at); };

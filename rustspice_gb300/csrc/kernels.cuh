@@ -482,7 +482,8 @@ struct AcShape {
   bool masks_shared;
   size_t smem, scratch_bytes, mask_words;
 };
-AcShape ac_shape(int n, int nf, int sms);
+// limit: bytes of scratch at most (one matrix at least).
+AcShape ac_shape(int n, int nf, int sms, size_t limit);
 void launch_ac_sparse(const AcArgs& a, int nf, const AcShape& s, cudaStream_t st);
 
 // Transient forward / adjoint over a batch: one warp per instance.
