@@ -469,12 +469,14 @@ AcShape ac_shape(int n, int nf, int sms, size_t limit) {
   AcShape s;
   // One warp per frequency from eight frequencies an SM on, else as many as
   // keep eight warps an SM busy, a column's updates and the masks spread over
-  // them. Measured: 326-node grid, 226 frequencies, 1 / 2 / 4 / 8 warps 5.4 /
-  // 4.0 / 3.3 / 3.1 ms; 103-node ladder, 4501 frequencies, 2.7 / 5.1 / 7.9 /
-  // 12 ms, 46 frequencies 0.72 / 0.65 / 0.64 / 0.64 ms. 16 resident warps an
-  // SM: 1351 ladder frequencies take 0.86 ms against 1.43 ms with eight.
+  // them, in small systems too (full ones have n^2 updates a column). Measured:
+  // 326-node grid, 226 frequencies, 1 / 2 / 4 / 8 warps 5.4 / 4.0 / 3.3 / 3.1 ms;
+  // 103-node ladder, 4501 frequencies, 2.7 / 5.1 / 7.9 / 12 ms, 46 frequencies
+  // 0.72 / 0.65 / 0.64 / 0.64 ms; full system of 62 unknowns, 20 frequencies, 2
+  // warps 1.46, 4 1.10, 8 0.97 ms, of 32, 1 warp 0.56, 8 0.33 ms. 16 resident warps
+  // an SM: 1351 ladder frequencies take 0.86 ms against 1.43 ms with eight.
   s.warps = 1;
-  while (s.warps < 8 && (long long)s.warps * nf < 8LL * sms && s.warps * 32 < n) s.warps *= 2;
+  while (s.warps < 8 && (long long)s.warps * nf < 8LL * sms) s.warps *= 2;
   s.masks_shared = sparse_smem(n, s.warps, true) <= 100 * 1024;
   s.smem = sparse_smem(n, s.warps, s.masks_shared);
   const long long per_sm =
