@@ -520,15 +520,33 @@ void gpuklu_plan_free(gpuklu_plan* p);
  * offsets); copies when the capacities (in int32) suffice. */
 int64_t gpuklu_plan_steps(const gpuklu_plan* p, int32_t nc, int32_t ndv, int32_t* ops,
                           int64_t ops_cap, int32_t* step_ptr, int64_t steps_cap);
-/* The single-system solve's step program (k_solve_steps) for this plan: four
- * int32 per operation (destination row, source row or -1, value index, kind:
- * 0 x[d] -= lu[v] x[s], 2 x[d] -= ax[v] x[s] (block coupling), 1 x[d] /= lu[v]
- * (the pivot)) in step order, with the rows in the plan's positions, and the
- * step pointers. Returns nops << 32 | (nsteps + 1) (0: no program, the
- * solution exceeds one block's shared memory); copies when the capacities
- * (in int32) suffice. */
+/* The single-system solve's operations by step for this plan (what
+ * k_solve_list runs; k_solve_steps runs the program laid out from them, next):
+ * four int32 per operation (destination row, source row or -1, value index,
+ * kind: 0 x[d] -= lu[v] x[s], 2 x[d] -= ax[v] x[s] (block coupling), 1 x[d] /=
+ * lu[v] (the pivot)) in step order, with the rows in the plan's positions, and
+ * the step pointers. Returns nops << 32 | (nsteps + 1) (0: none, the solution
+ * exceeds one block's shared memory); copies when the capacities (in int32)
+ * suffice. */
 int64_t gpuklu_plan_solve_steps(const gpuklu_plan* p, int32_t* ops, int64_t ops_cap,
                                 int32_t* step_ptr, int64_t steps_cap);
+/* The program k_solve_steps runs for this plan's solve (transpose 0) or for
+ * the solve with A^T (1), one array at a time by name:
+ *   "info"    slots of a chunk, slots of a wide row
+ *   "ops"     slots: destination row, source row, value index, kind (as above, a
+ *             division's source its own row; 3 nothing) | 4 when a division is
+ *             among its row's operations | 8 in the last row of its step
+ *   "segs"    kind | count << 2, first chain or -1; kinds: 0 rows of 32 slots run
+ *             by one warp, a barrier after each (the warp's own), 1 wide rows, a
+ *             barrier after the last one of a step, 2 chains
+ *   "chunks"  first slot, slots, first segment, segments
+ *   "chains"  destination row, first term, terms, 0: the terms are subtracted in
+ *             order
+ *   "terms"   source row, lu index or ~ax index
+ * Returns its int32 values (-1: no such array); copies when cap suffices. An
+ * empty "chunks": the plan's solves run without a program. */
+int64_t gpuklu_plan_solve_program(const gpuklu_plan* p, int transpose, const char* name,
+                                  int32_t* out, int64_t cap);
 /* btf_decompose (crates/sim-core/src/btf.rs:143-550) on the host: out[0] the
  * number of blocks, out[1] the largest block's size - what
  * MatrixProperties::analyze (solver.rs:276-301) reads for the solver

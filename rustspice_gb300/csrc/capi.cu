@@ -5081,6 +5081,37 @@ int64_t gpuklu_plan_solve_steps(const gpuklu_plan* p, int32_t* ops, int64_t ops_
   return (int64_t)o.size() * ((int64_t)1 << 32) + (int64_t)sp.size();
 }
 
+int64_t gpuklu_plan_solve_program(const gpuklu_plan* p, int transpose, const char* name,
+                                  int32_t* out, int64_t cap) {
+  if (!p || !name) return -1;
+  SolveProgram sp;
+  make_solve_program(p->p, transpose != 0, sp);
+  std::vector<i32> v;
+  auto four = [&](const std::vector<int4>& a) {
+    for (const int4& q : a) v.insert(v.end(), {q.x, q.y, q.z, q.w});
+  };
+  auto two = [&](const std::vector<int2>& a) {
+    for (const int2& q : a) v.insert(v.end(), {q.x, q.y});
+  };
+  const std::string k(name);
+  if (k == "info")
+    v = {sp.chunk, sp.width};
+  else if (k == "ops")
+    four(sp.ops);
+  else if (k == "chunks")
+    four(sp.chunks);
+  else if (k == "chains")
+    four(sp.chains);
+  else if (k == "segs")
+    two(sp.segs);
+  else if (k == "terms")
+    two(sp.terms);
+  else
+    return -1;
+  if (out && (int64_t)v.size() <= cap) std::copy(v.begin(), v.end(), out);
+  return (int64_t)v.size();
+}
+
 gpuklu_plan* gpuklu_plan_build(int64_t n, const int64_t* ap, const int64_t* ai, int pivot_mode,
                                int kind, const int32_t* row_perm) {
   auto P = std::make_unique<gpuklu_plan>();
