@@ -159,7 +159,7 @@ def test_the_uploaded_program(sysm, mode):
             assert np.max(np.abs(got - ref)) <= 1e-9 * np.max(np.abs(ref))
         if name == "arrow300":
             assert len(pr["chains"]) > 0
-        if name in ("upper", "lower"):
+        if mode == N.PIVOT_EXACT and name in ("upper", "lower"):
             assert P.noffdiag > 0
 
 
