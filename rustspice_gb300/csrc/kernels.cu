@@ -2451,7 +2451,11 @@ void launch_solve_steps(const DPlan& P, bool transpose, const double* rhs, const
     raise_smem_limit<k_solve_steps<false>>(bytes);
   if (staged)
     k_solve_slots<<<(P.ss.nslots + 255) / 256, 256, 0, s>>>(P.ss, P.n, ax, lu, P.skip);
-  kernel<<<1, staged ? kSolveRow + 32 : kSolveStepsThreads, bytes, s>>>(
+  // a program of one short chunk has nothing for the loader warps to fetch (two
+  // rows, a call: 29.1 us without them, 30.0 with)
+  const int loaded = P.ss.nchunks == 1 && P.ss.nslots <= kSolveRow * kLoadBatch ? kSolveRow
+                                                                                : kSolveStepsThreads;
+  kernel<<<1, staged ? kSolveRow + 32 : loaded, bytes, s>>>(
       P.ss, P.n, in, outp, P.dslot, rhs, ax, lu, rec, out, P.skip, status, P.pair_limit);
 }
 
