@@ -152,9 +152,10 @@ const char* gpuklu_last_error(const gpuklu_handle* h);
 /* Refactorizations the last first factorization ran to find the pivot
  * sequence of native_klu.rs:1194-1382 (the pivot pass restated as
  * refactorizations that check the threshold rule on every column); 0 when
- * the sequential one-warp pivot pass ran instead (below 16 rows, more than 8
- * passes needed, or GPUKLU_PIVOT_PASS=sequential; GPUKLU_PIVOT_PASS=refactor
- * takes the refactorizations at every size). Both give the same pivots and
+ * the sequential one-warp pivot pass ran instead (below 16 rows, more passes
+ * needed than the 3 + n/32, at most 8, it is given, or GPUKLU_PIVOT_PASS=
+ * sequential; GPUKLU_PIVOT_PASS=refactor takes the refactorizations at every
+ * size, up to 8). Both give the same pivots and
  * factor. */
 int64_t gpuklu_pivot_pass_count(const gpuklu_handle* h);
 /* factor/solve with values already in device memory (the device-stamp path):
@@ -314,10 +315,13 @@ gpuklu_batch* gpuklu_batch_create(int64_t ncirc, const int64_t* dev_off,
                                   const double* inst_val, const double* x0,
                                   const int64_t* x0_off, int64_t x0_len);
 void gpuklu_batch_destroy(gpuklu_batch* b);
-/* Runs every instance's Newton loop on the device: one warp per instance, the
- * programs in up to eight classes by size, all classes concurrent. With that
- * kernel switched off: a lane-per-instance kernel for the first lane_cap
- * iterations, then the warp classes for the instances still iterating. */
+/* Runs every instance's Newton loop on the device: one warp per instance (two
+ * instances a warp for many of a small program), the programs in up to eight
+ * classes by size, all classes concurrent. Where there are many instances of
+ * small programs a lane-per-instance kernel runs their first lane_cap
+ * iterations before. With the warp-per-instance kernel switched off: the lane
+ * kernel for every program, then the warp classes for the instances still
+ * iterating. */
 int gpuklu_batch_run(gpuklu_batch* b, const gpuklu_newton_config* cfg);
 /* Results: per instance iterations (final run), total iterations, exit
  * reason, and x (n of its circuit values, at x_out + x_off[i]; x_off may be
@@ -339,24 +343,24 @@ const char* gpuklu_batch_last_error(const gpuklu_batch* b);
  * block, out[2] program groups, out[3] shared-memory bytes per warp,
  * out[4] registers per thread, out[5] resident blocks per SM (out[1], out[3..5]
  * describe the largest class), out[6] kernel launches per gpuklu_batch_run
- * (the lane kernel and one per size class), out[7] reserved (0). */
+ * (one per size class, and the lane kernel where it runs), out[7] 1 when the
+ * warp-per-instance kernel runs. */
 int gpuklu_batch_info(const gpuklu_batch* b, int64_t* out);
 /* Work of one Newton iteration of every instance: FP64 operations and the
  * value bytes it moves through on-chip memory (arrays of ninst). */
 int gpuklu_batch_work(const gpuklu_batch* b, int64_t* flops, int64_t* bytes);
 void* gpuklu_batch_stream(gpuklu_batch* b);
 /* Device time of the last gpuklu_batch_run (waits for it), from CUDA events
- * on the launching streams: out[0] the lane-per-instance kernel [ms], out[1]
- * the warp kernels that finish the instances it parked [ms], out[2] the
- * iterations an instance runs in the lane kernel before it is parked (0: no
- * lane phase). */
+ * on the launching streams: out[0] until the lane-per-instance kernel has
+ * ended [ms] (only the counters' resets where it does not run), out[1] from
+ * there to the end [ms], out[2] lane_cap (below; 0: the warp classes alone). */
 int gpuklu_batch_phase_ms(gpuklu_batch* b, double* out);
 /* The batch's schedule; no counterpart in the reference. lane_cap: Newton
  * iterations an instance runs with the lane-per-instance kernel's order of
- * additions (default 6; with the warp-per-instance kernel switched off, in
- * that kernel before it is parked for the warp classes); cont_tiles: shared-program tiles per circuit program in
- * the warp classes' continuation (default 2; the warp-per-instance kernel
- * has none). Results agree across schedules to the batch's 1e-10 bar (an
+ * additions (default 6), in that kernel before it is parked where that kernel
+ * comes first; cont_tiles: shared-program tiles per circuit program in the
+ * warp classes' continuation (default 2; the warp-per-instance kernel has
+ * none). Results agree across schedules to the batch's 1e-10 bar (an
  * instance's arithmetic differs between the kernels only in rounding). */
 int gpuklu_batch_set_schedule(gpuklu_batch* b, int lane_cap, int cont_tiles);
 /* Autotuner: times one run of the batch per candidate schedule (lane_cap in

@@ -3372,6 +3372,11 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
         const long long stride = lregion * 32;
         if (e == cudaSuccess)
           e = B->d_scratch.resize((size_t)B->lane_grid * B->lane_wpb * (size_t)stride);
+        if (B->cont_kernel && e == cudaErrorMemoryAllocation) {
+          e = cudaSuccess;  // no room for its scratch: the warps run every iteration
+          B->ltiles.clear();
+          for (auto& k : B->cont) k.lanes = false;
+        }
         if (e == cudaSuccess) e = B->d_ltiles.upload(B->ltiles, s);
         if (e == cudaSuccess) e = B->d_lcounter.resize(1);
         if (e == cudaSuccess) e = B->d_cont_list.resize(std::max<int64_t>(ninst, 1));
@@ -3963,7 +3968,8 @@ int gpuklu_batch_run(gpuklu_batch* b, const gpuklu_newton_config* cfg) {
 
 int gpuklu_batch_set_schedule(gpuklu_batch* b, int lane_cap, int cont_tiles) {
   if (!b) return GPUKLU_INVALID_MATRIX;
-  // lane cap 0: no lane phase, the continuation kernel starts every instance
+  // lane cap 0: no lane phase, and no iteration with the lane kernel's order of
+  // additions
   const int cap_lo = b->cont_kernel ? 0 : 1;
   if (cont_tiles < 1 || cont_tiles > 16 ||
       (b->lanes && (lane_cap < cap_lo || lane_cap > 100))) {

@@ -1,7 +1,8 @@
 // Batched DC operating points, one instance per warp or two (16 lanes each).
 //
 // Each warp takes instances from a queue over every program (most expensive
-// programs first) and runs their Newton loops to the end: the permuted
+// programs first) and runs their Newton loops to the end, from the start or
+// from where the lane kernel (lanes.cu) parked them: the permuted
 // right-hand side and the LU values in the warp's slice of shared memory, the
 // device records and the iterate in its slice of a global scratch (written
 // and read by the warp's own lanes, L2 resident), the factorization and
@@ -13,7 +14,7 @@
 // sub-partition whatever its active lanes, and for the instances that run to
 // the iteration cap the latency of their rows. Measured against the lane
 // kernel's six iterations and a kernel that loads its steps from global
-// memory behind it: 976 instances (16 chains of 8-256 stages) 32.6 -> 7.2 ms,
+// memory behind it: 976 instances (16 chains of 8-256 stages) 38.9 -> 9.8 ms,
 // 249,856 instances 71.7 -> 65.2 ms.
 #include <cfloat>
 

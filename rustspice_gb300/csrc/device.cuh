@@ -10,7 +10,6 @@ namespace gk {
 enum DevStatus : int {
   DS_OK = 0,
   DS_TIMEOUT = 7,
-  DS_NONFINITE = 8,
 };
 
 // Arithmetic without contraction: every product is rounded before it is

@@ -20,7 +20,13 @@ constexpr unsigned kSpinLimit = 1u << 22;
 // terms; a term: source row, lu value or ~ax value), and those into chunks
 // (first slot, slots, first segment, segments). 0 chunks: none.
 constexpr int kSolveRow = 128;   // compute threads
-constexpr int kSolveStaged = 1 << 18;  // slots of a program laid out ahead
+// Slots from which a program's are laid out ahead and copied in bulk: below, the
+// layout's pass and a vote a chunk cost more than the loader warps. Measured,
+// loaded / copied, us a call, forward: 48 x 48 mesh (96 k slots) 264 / 268, 80 x 80
+// (291 k) 647 / 650, 120 x 120 with 1000 inverters (921 k) 1615 / 1663, 130 x 130
+// (875 k) 1634 / 1684, 145 x 145 (1.10 M) 2089 / 2080 (transpose 2507 / 2326), 160 x
+// 160 (chunks of 512) 3529 / 3052.
+constexpr int kSolveStaged = 1 << 20;
 constexpr int kSolveSegs = 64;   // segments of a chunk, at most
 // Slots of a chunk, at least. Smaller ones spend the time on the barrier and
 // the loads' latency between them. Measured, forward, this program against the
@@ -425,8 +431,8 @@ void launch_batch_newton(const BatchArgs& a, int m, int grid, int warps_per_bloc
 // Lane-per-instance batched Newton (phase 1 of gpuklu_batch_run).
 // Warp-per-instance kernel: one warp per block, m instances per warp; kContWarps
 // blocks at least fit an SM's registers. With 8 the compiler keeps 222 registers
-// and spills none, and 9 warps share an SM; measured, 249,856 / 976 instances, ms:
-// 8 65.1 / 7.2, 10 66.2 / 7.6, 12 66.9 / 7.5, 16 68.5 / 8.2, 20 73.4 / 8.9.
+// and spills none, and 8 warps share an SM; measured, 249,856 / 976 instances, ms:
+// 8 65.2 / 9.8, 9 68.9 / 10.6, 10 68.7 / 10.0, 12 68.7 / 9.9, 16 74.5 / 10.9.
 constexpr int kContWarps = 8;
 void launch_batch_cont(const BatchArgs& a, int m, int grid, cudaStream_t s);
 void cont_kernel_info(int m, int slice, int* regs, int* blocks_per_sm);
