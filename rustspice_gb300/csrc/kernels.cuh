@@ -340,14 +340,14 @@ struct AcArgs {
 // The limit belongs to the kernel on a device, not to a handle or a launch:
 // set to one plan's size before its launch, another thread's smaller plan
 // could lower it in between, and an older batch would find a newer one's. So
-// it only ever goes up, under a lock. A size the device refuses is not kept,
-// and the launch reports it.
+// it only ever goes up, under a lock, from the first launch on: a kernel's own
+// limit is 48 KB less what it declares (528 bytes in k_refactor). A size the
+// device refuses is not kept, and the launch reports it.
 template <auto Kernel>
 inline cudaError_t raise_smem_limit(size_t bytes) {
   constexpr int kDevices = 64;
   static std::mutex mu;
   static size_t limit[kDevices] = {};
-  if (bytes <= 48 * 1024) return cudaSuccess;  // every kernel's own limit
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

@@ -88,6 +88,43 @@ def test_a_circuit_refused_for_its_size_leaves_the_next_batch_its_memory():
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+RISING = """
+import numpy as np, scipy.sparse as sp
+from rustspice_gb300.solver import GpuKluSolver
+
+def check(a):
+    a = sp.csc_matrix(a)
+    a.sort_indices()
+    n = a.shape[0]
+    g, x = GpuKluSolver(n), np.ones(n)
+    g.factor(a.indptr.astype(np.int64), a.indices.astype(np.int64), a.data)
+    g.solve(x)
+    assert np.abs(a @ x - 1.0).max() < 1e-10, n
+
+for n in range(%d, %d):
+    if %d:  # the last column holds n values
+        a = sp.lil_matrix(sp.diags([4.0 * n], shape=(n, n)))
+        a[n - 1, :n - 1] = -1.0
+        a[:n - 1, n - 1] = -1.0
+    else:
+        a = sp.diags([-1.0, 4.0, -1.0], [-1, 0, 1], shape=(n, n))
+    check(a)
+"""
+
+
+@pytest.mark.parametrize("lo,hi,arrow", [(690, 732, 1), (16, 515, 0)])
+def test_sizes_that_rise_through_a_kernels_own_limit(lo, hi, arrow):
+    """A kernel's own limit is 48 KB less its declared shared memory. Sizes
+    that rise by a row at a time pass every one of the bytes between (columns
+    of 704 to 720 slots in the grid refactorization), each in a launch that is
+    the largest so far. Diagonally dominant systems: the residual is rounding,
+    some 1e-13 at the most."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", RISING % (lo, hi, arrow)], cwd=root,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_bordered_solvers_of_two_sizes():
     cfg = N.newton_config(**CFG)
     work = []
