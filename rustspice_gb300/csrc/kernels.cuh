@@ -20,13 +20,13 @@ constexpr unsigned kSpinLimit = 1u << 22;
 // terms; a term: source row, lu value or ~ax value), and those into chunks
 // (first slot, slots, first segment, segments). 0 chunks: none.
 constexpr int kSolveRow = 128;   // compute threads
-// Slots from which a program's are laid out ahead and copied in bulk: below, the
-// layout's pass and a vote a chunk cost more than the loader warps. Measured,
-// loaded / copied, us a call, forward: 48 x 48 mesh (96 k slots) 264 / 268, 80 x 80
-// (291 k) 647 / 650, 120 x 120 with 1000 inverters (921 k) 1615 / 1663, 130 x 130
-// (875 k) 1634 / 1684, 145 x 145 (1.10 M) 2089 / 2080 (transpose 2507 / 2326), 160 x
-// 160 (chunks of 512) 3529 / 3052.
-constexpr int kSolveStaged = 1 << 20;
+// Slots from which a program's are laid out ahead and copied in bulk. Measured,
+// loaded / copied: the operating point and adjoint of the 120 x 120 mesh with 1000
+// inverters 24.3 / 23.1 ms; single solves, us: 145 x 145 mesh (1.10 M slots) 2089 /
+// 2080 (transpose 2507 / 2326), 160 x 160 (chunks of 512) 3529 / 3052, but 80 x 80
+// (291 k) 647 / 650, 120 x 120 (719 k) 1350 / 1424, 130 x 130 (875 k) 1634 / 1684. Below
+// the line the layout's pass and a vote a chunk only cost: 48 x 48 (96 k) 264 / 268.
+constexpr int kSolveStaged = 1 << 18;
 constexpr int kSolveSegs = 64;   // segments of a chunk, at most
 // Slots of a chunk, at least. Smaller ones spend the time on the barrier and
 // the loads' latency between them. Measured, forward, this program against the
