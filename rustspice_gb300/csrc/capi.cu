@@ -2900,10 +2900,13 @@ gk::NewtonCfg to_newton_cfg(const gpuklu_newton_config& cfg) {
 constexpr int64_t kSmallProgram = 3500;
 // Instances per warp of a class: inst instances of count programs, flops
 // operations an iteration on average, slots instances on the device at one per
-// warp.
-int instances_per_warp(int64_t inst, int count, int64_t flops, int64_t slots) {
+// warp. Beside larger programs (all_small false) one: their rows fill the FP64
+// pipes, and a half whose partner runs to the iteration cap then only idles
+// (4096 chains of 8 to 256 stages, the smallest class at two a warp and at one:
+// 60.9 and 59.8 ms).
+int instances_per_warp(int64_t inst, int count, int64_t flops, int64_t slots, bool all_small) {
   if (const char* e = getenv("GPUKLU_CONT_M")) return e[0] == '2' ? 2 : 1;
-  return flops <= kSmallProgram && inst >= 3 * slots && inst >= 8 * (int64_t)count ? 2 : 1;
+  return all_small && flops <= kSmallProgram && inst >= 3 * slots && inst >= 8 * (int64_t)count ? 2 : 1;
 }
 // Whether the lane kernel comes first for the batch's small programs (inst
 // instances of them).
@@ -3284,13 +3287,16 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
           if (B->groups[g].nchunk == 0) ok = false;
         }
       std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return need(x) > need(y); });
-      bool lanes = false;
+      bool lanes = false, all_small = true;
       {
         int64_t inst = 0, flops = 0;
         bool diodes = false;
         for (int g : by) {
           const gk::GroupHdr& h = B->groups[g];
-          if (B->group_flops[g] > kSmallProgram) continue;
+          if (B->group_flops[g] > kSmallProgram) {
+            all_small = false;
+            continue;
+          }
           inst += h.inst_count;
           flops += B->group_flops[g] * h.inst_count;
           for (int d = 0; d < h.ndev; ++d) diodes |= dev_type[h.dev_off + d] == 3;
@@ -3324,7 +3330,8 @@ gpuklu_batch* batch_build(int64_t ncirc, const int64_t* dev_off, const int64_t* 
         gk::cont_kernel_info(1, k.slice, &regs, &per_sm);
         flops /= std::max<int64_t>(inst, 1);
         k.lanes = lanes && (flops <= kSmallProgram || getenv("GPUKLU_LANE_PHASE"));
-        if (instances_per_warp(inst, k.count, flops, (int64_t)sm_count() * per_sm) == 2) {
+        if (instances_per_warp(inst, k.count, flops, (int64_t)sm_count() * per_sm, all_small) ==
+            2) {
           int two = 0;
           gk::cont_kernel_info(2, k.slice, &regs, &two);
           if (two > 0) k.m = 2, per_sm = two;
