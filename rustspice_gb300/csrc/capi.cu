@@ -31,6 +31,10 @@ std::string cuda_msg(cudaError_t e, const char* what) {
   return std::string(what) + ": " + cudaGetErrorString(e);
 }
 
+// At the start of a call whose launches are checked by the thread's last error:
+// what another library, or the caller, left there is not this call's.
+void forget_errors() { cudaGetLastError(); }
+
 // Owning device allocation.
 template <class T>
 struct DBuf {
@@ -1477,6 +1481,7 @@ int gpuklu_analyze(gpuklu_handle* h, const int64_t* ap, int64_t ap_len, const in
 
 int gpuklu_factor(gpuklu_handle* h, const int64_t* ap, int64_t ap_len, const int64_t* ai,
                   int64_t ai_len, const double* ax) {
+  forget_errors();
   if (!h) return GPUKLU_INVALID_MATRIX;
   if (h->state == gpuklu_handle::EMPTY || !h->same_pattern(ap, ap_len, ai, ai_len)) {
     int st = h->do_analyze(ap, ap_len, ai, ai_len);
@@ -1489,6 +1494,7 @@ int gpuklu_factor(gpuklu_handle* h, const int64_t* ap, int64_t ap_len, const int
 }
 
 int gpuklu_factor_device(gpuklu_handle* h, const double* d_ax) {
+  forget_errors();
   if (!h || h->state == gpuklu_handle::EMPTY) return GPUKLU_FACTOR_FAILED;
   cudaError_t e = cudaMemcpyAsync(h->d_ax.p, d_ax, h->last_ai.size() * sizeof(double),
                                   cudaMemcpyDeviceToDevice, h->stream);
@@ -1497,6 +1503,7 @@ int gpuklu_factor_device(gpuklu_handle* h, const double* d_ax) {
 }
 
 int gpuklu_solve(gpuklu_handle* h, double* rhs, int64_t len) {
+  forget_errors();
   if (!h || h->state != gpuklu_handle::FACTORED) return GPUKLU_SOLVE_FAILED;
   if (len != h->n)  // DenseSolver::solve reports SolveFailed (solver.rs:689-691)
     return h->fail(h->kind == GPUKLU_KIND_DENSE ? GPUKLU_SOLVE_FAILED : GPUKLU_INVALID_MATRIX,
@@ -1513,6 +1520,7 @@ int gpuklu_solve(gpuklu_handle* h, double* rhs, int64_t len) {
 }
 
 int gpuklu_solve_device(gpuklu_handle* h, double* d_rhs) {
+  forget_errors();
   if (!h || h->state != gpuklu_handle::FACTORED) return GPUKLU_SOLVE_FAILED;
   cudaError_t e = cudaMemcpyAsync(h->d_rhs.p, d_rhs, h->n * sizeof(double),
                                   cudaMemcpyDeviceToDevice, h->stream);
@@ -1526,6 +1534,7 @@ int gpuklu_solve_device(gpuklu_handle* h, double* d_rhs) {
 }
 
 int gpuklu_tsolve(gpuklu_handle* h, double* g, int64_t len) {
+  forget_errors();
   if (!h || h->state != gpuklu_handle::FACTORED) return GPUKLU_SOLVE_FAILED;
   if (len != h->n) return h->fail(GPUKLU_INVALID_MATRIX, "RHS length mismatch");
   cudaError_t e = cudaMemcpyAsync(h->d_rhs.p, g, len * sizeof(double), cudaMemcpyHostToDevice,
@@ -1593,6 +1602,7 @@ int gpuklu_set_pivot_mode(gpuklu_handle* h, int mode) {
 }
 
 int gpuklu_get_stats(gpuklu_handle* h, gpuklu_stats* out) {
+  forget_errors();
   if (!h || !out) return GPUKLU_INVALID_MATRIX;
   if (h->state == gpuklu_handle::FACTORED && !h->rcond_valid &&
       h->kind != GPUKLU_KIND_DENSE) {
@@ -2041,6 +2051,7 @@ extern "C" {
 int gpuklu_newton_dc(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_config* cfg,
                      const double* x0, double* x_out, int64_t x_cap, int64_t* x_len,
                      int64_t* iters, int64_t* iters_total, int* reason) {
+  forget_errors();
   if (!h || !c || !cfg) return GPUKLU_INVALID_MATRIX;
   // Engine::run_dc_result: x = zeros(node_count), solver.prepare(node_count)
   // (a size other than the matrix's when there are voltage sources, so the
@@ -2059,6 +2070,7 @@ int gpuklu_dc_sweep(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_con
                     int64_t src_dev, const double* values, int64_t npts, const double* x0,
                     int64_t x0_stride, int stop_on_failure, double* x_out, int64_t x_stride,
                     int64_t* x_len, int64_t* iters, int64_t* iters_total, int* reason) {
+  forget_errors();
   if (!h || !c || !cfg || !values || npts < 0) return GPUKLU_INVALID_MATRIX;
   if (src_dev < 0 || src_dev >= c->ndev)
     return h->fail(GPUKLU_INVALID_MATRIX, "gpuklu_dc_sweep: no device " +
@@ -2108,6 +2120,7 @@ int gpuklu_dc_sweep(gpuklu_handle* h, gpuklu_circuit* c, const gpuklu_newton_con
 int gpuklu_dc_backward(gpuklu_handle* h, gpuklu_circuit* c, const double* x, int64_t xlen,
                        const double* dl_dx, double gmin, double* lambda_out,
                        double* grad_out) {
+  forget_errors();
   if (!h || !c || !x || !dl_dx) return GPUKLU_INVALID_MATRIX;
   const int n = c->n;
   gpuklu_prepare(h, n);
@@ -4824,6 +4837,7 @@ int gpuklu_bbd_perm(const gpuklu_bbd* b, int64_t* perm) {
 }
 
 int gpuklu_bbd_factor(gpuklu_bbd* b, const double* ax) {
+  forget_errors();
   if (!b || !ax) return GPUKLU_INVALID_MATRIX;
   cudaError_t e = cudaMemcpyAsync(b->d_ax.p, ax, b->ai.size() * 8, cudaMemcpyHostToDevice,
                                   b->stream());
@@ -4832,6 +4846,7 @@ int gpuklu_bbd_factor(gpuklu_bbd* b, const double* ax) {
 }
 
 int gpuklu_bbd_solve(gpuklu_bbd* b, double* rhs, int64_t len) {
+  forget_errors();
   if (!b || !rhs || len != b->n) return GPUKLU_INVALID_MATRIX;
   if (!b->fallback && !b->tiles_ready) return b->fail(GPUKLU_SOLVE_FAILED, "solve before factor");
   cudaStream_t s = b->stream();
@@ -4849,6 +4864,7 @@ int gpuklu_bbd_solve(gpuklu_bbd* b, double* rhs, int64_t len) {
 int gpuklu_bbd_newton_dc(gpuklu_bbd* b, gpuklu_circuit* c, const gpuklu_newton_config* cfg,
                          const double* x0, double* x_out, int64_t x_cap, int64_t* x_len,
                          int64_t* iters, int64_t* iters_total, int* reason) {
+  forget_errors();
   if (!b || !c || !cfg) return GPUKLU_INVALID_MATRIX;
   if (c->n != b->n || c->ap != b->ap || c->ai != b->ai)
     return b->fail(GPUKLU_INVALID_MATRIX, "the circuit's pattern differs from the solver's");
@@ -4966,6 +4982,7 @@ cudaError_t noalloc_scratch(unsigned char** out) {
 }  // namespace
 
 extern "C" int gpuklu_solve_device_noalloc(gpuklu_handle* h, const double* d_rhs, double* d_x) {
+  forget_errors();
   if (!h || h->state != gpuklu_handle::FACTORED) return GPUKLU_SOLVE_FAILED;
   if (h->kind == GPUKLU_KIND_DENSE)
     return h->fail(GPUKLU_SOLVE_FAILED, "gpuklu_solve_device_noalloc: not for the dense solver");

@@ -1,6 +1,7 @@
 """Calls of the CUDA runtime that it refuses: a call whose kernel was not
 launched reports it, and a call is not failed by what an earlier one was
 refused. Nothing here runs a kernel that faults."""
+import ctypes
 import threading
 
 import numpy as np
@@ -10,8 +11,8 @@ from oracle import pyoracle as po
 from rustspice_gb300 import circuits as cz
 from rustspice_gb300 import native as N
 from rustspice_gb300 import workloads as wl
-from rustspice_gb300.solver import (DeviceCircuit, GpuKluSolver, SolverError, TranBatch,
-                                    newton_dc)
+from rustspice_gb300.solver import (BbdSolver, DeviceCircuit, GpuKluSolver, SolverError, TranBatch,
+                                    dc_backward, newton_dc)
 
 pytestmark = pytest.mark.gpu
 
@@ -93,3 +94,35 @@ def test_a_refused_allocation_does_not_fail_the_next_call():
     assert np.array_equal(x, want)
     refused()
     assert newton_dc(h, dc, N.newton_config(**wl.TIGHT)).converged
+
+
+def test_an_error_left_by_other_code_does_not_fail_a_call():
+    """The thread's last error as another user of the CUDA runtime leaves it (a
+    device number that does not exist) before each call."""
+    rt = ctypes.CDLL("libcudart.so.13")
+    c = cz.mesh_dc(8, 8)
+    n, ap, ai, ax, rhs = po.mna(c, np.zeros(c.node_count))
+    g = GpuKluSolver(n, pivot_mode=N.PIVOT_EXACT)
+    h, dc = GpuKluSolver(1, pivot_mode=N.PIVOT_EXACT), DeviceCircuit(c)
+    cb, asg, nb = cz.bordered_meshes(3, 24, 8, 8, 4)
+    dcb = DeviceCircuit(cb)
+    b = BbdSolver(*dcb.pattern(), asg, nb)
+    cfg = N.newton_config(**wl.TIGHT)
+    out = {}
+
+    def solve(f):
+        x = rhs.copy()
+        f(x)
+        return x
+
+    calls = {"factor": lambda: g.factor(ap, ai, ax), "refactor": lambda: g.factor(ap, ai, ax),
+             "solve": lambda: solve(g.solve), "tsolve": lambda: solve(g.tsolve),
+             "newton": lambda: newton_dc(h, dc, cfg).x,
+             "adjoint": lambda: dc_backward(h, dc, out["newton"], np.ones(dc.n))[0],
+             "bordered": lambda: b.newton_dc(dcb, cfg, x0=wl.bordered_nodeset(cb)).x}
+    for name, call in calls.items():
+        assert rt.cudaSetDevice(4096) != 0 and rt.cudaPeekAtLastError() != 0
+        out[name] = call()
+        assert rt.cudaPeekAtLastError() == 0, name
+        again = call()
+        assert out[name] is None or np.array_equal(out[name], again), name
